@@ -127,7 +127,9 @@ __device__ __forceinline__ real3 operator*(real3 a, real s) { return make_real3(
 __device__ __forceinline__ real3 operator-(real3 a) { return make_real3(-a.x, -a.y, -a.z); }
 __device__ __forceinline__ void operator+=(real3& a, real3 b) { a.x += b.x; a.y += b.y; a.z += b.z; }
 __device__ __forceinline__ void operator-=(real3& a, real3 b) { a.x -= b.x; a.y -= b.y; a.z -= b.z; }
-__device__ __forceinline__ real dot3(real3 a, real3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// Fused explicitly, so that every instance of a pass rounds it the same way: of a sum of two
+// products the compiler is free to fuse either.
+__device__ __forceinline__ real dot3(real3 a, real3 b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
 
 // Exact f32 distance as the reference computes it for the in-range test:
 // (x_i - x_j).norm() < support_radius (SPH/main.py:845), no FMA contraction.
@@ -174,24 +176,25 @@ __device__ __forceinline__ real3 kernel_grad(real3 r, real rn, const SceneDev& s
 
 // The same cubic spline and gradient as kernel_w / kernel_grad, from r^2 and without
 // divisions (1/h precomputed, 1/|r| from rsqrt): used inside the neighbour loops,
-// where it agrees with the reference expressions to a few ulp.
+// where it agrees with the reference expressions to a few ulp. Multiply-adds are written
+// out, so that they round the same way wherever the expressions are inlined.
 __device__ __forceinline__ void kwg_r2(real3 r, real r2, const SceneDev& s, real& w, real3& g) {
   const real inv_rn = r2 > 0.f ? rsqrt(r2) : 0.f;
   const real rn = r2 * inv_rn;
   const real q = rn * s.inv_h;
-  const real t = 1.f - q;
+  const real t = fma(-rn, s.inv_h, real(1));
   const bool in = q <= 1.f;
   const bool inner = q <= 0.5f;
-  w = in ? (inner ? s.k_w * (6.f * q * q * (q - 1.f) + 1.f) : s.k2_w * (t * t * t)) : 0.f;
-  const real f = inner ? s.k_grad * q * (3.f * q - 2.f) : -s.k_grad * t * t;
+  w = in ? (inner ? s.k_w * fma(6.f * q * q, q - 1.f, real(1)) : s.k2_w * (t * t * t)) : 0.f;
+  const real f = inner ? s.k_grad * q * fma(real(3), q, real(-2)) : -s.k_grad * t * t;
   const real c = (rn > 1e-5f && in) ? f * inv_rn * s.inv_h : 0.f;
   g = make_real3(r.x * c, r.y * c, r.z * c);
 }
 __device__ __forceinline__ real kw_r2(real r2, const SceneDev& s) {
   const real rn = r2 > 0.f ? r2 * rsqrt(r2) : 0.f;
   const real q = rn * s.inv_h;
-  const real t = 1.f - q;
-  const real w = q <= 0.5f ? s.k_w * (6.f * q * q * (q - 1.f) + 1.f) : s.k2_w * (t * t * t);
+  const real t = fma(-rn, s.inv_h, real(1));
+  const real w = q <= 0.5f ? s.k_w * fma(6.f * q * q, q - 1.f, real(1)) : s.k2_w * (t * t * t);
   return q <= 1.f ? w : 0.f;
 }
 __device__ __forceinline__ real3 kgrad_r2(real3 r, real r2, const SceneDev& s) {
@@ -242,6 +245,64 @@ __device__ __forceinline__ void nb_batches(const int32_t* __restrict__ list, int
 #pragma unroll
     for (int u = 0; u < NB_U; ++u)
       if (k + u < c) use(j[u], g[u]);
+  }
+}
+
+// Lane split of the neighbour passes: L lanes (1, 2, 4 or 8) share a particle. A warp
+// covers 32 / L consecutive slots; lane `sub * (32 / L) + p` works on slot p of the warp
+// and takes every L-th entry of its list, so that a scene of a few thousand particles
+// still fills the chip and the chain of dependent loads and arithmetic per thread is L
+// times shorter. The trip count is uniform across the warp (warp collectives are allowed
+// in the body); `valid` is false on the lanes past the end.
+#define FOR_SPLIT(L, i, sub, valid, n)                                                                \
+  for (int _w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); _w * (32 / (L)) < (n);           \
+       _w += (int)((gridDim.x * blockDim.x) >> 5))                                                    \
+    for (int i = _w * (32 / (L)) + (int)(threadIdx.x & (32 / (L) - 1)),                               \
+             sub = (int)(threadIdx.x & 31) / (32 / (L)), _once = 1;                                   \
+         _once; _once = 0)                                                                            \
+      for (bool valid = i < (n); _once; _once = 0)
+
+// The `real`s of a struct, from lane `src` of the warp.
+template <typename T>
+__device__ __forceinline__ T shfl_reals(const T& t, int src) {
+  T r;
+  const real* a = reinterpret_cast<const real*>(&t);
+  real* b = reinterpret_cast<real*>(&r);
+#pragma unroll
+  for (int w = 0; w < (int)(sizeof(T) / sizeof(real)); ++w) b[w] = __shfl_sync(0xffffffffu, a[w], src);
+  return r;
+}
+
+// The neighbour loop of a pass: `load(j)` gathers what a neighbour contributes from,
+// `term(g)` computes its contribution (a struct of reals) and `fold(t)` adds one
+// contribution to the particle's sums. With one lane per particle these run entry by
+// entry in batches of U (nb_batches). With L lanes each computes the contributions of its
+// own entries, and every lane of the particle folds the L contributions of a trip in list
+// order (shuffles): the sums are the same operations in the same order for every L, so
+// results do not depend on it, nor on what a scene is batched with. All 32 lanes call
+// this; lanes without work pass c = 0.
+template <int U, int L, bool STREAM = false, typename Load, typename Term, typename Fold>
+__device__ __forceinline__ void nb_sum(const int32_t* __restrict__ list, int stride, int c, int self, int sub,
+                                       Load load, Term term, Fold fold) {
+  if constexpr (L == 1) {
+    if (c > 0) nb_batches<U, STREAM>(list, stride, c, self, load, [&](int, const auto& g) { fold(term(g)); });
+  } else {
+    constexpr int P = 32 / L;
+    const int p = (int)(threadIdx.x & (P - 1));
+    const int cm = __reduce_max_sync(0xffffffffu, c);
+    int q0 = sub < c ? nb_list_load<false>(list + (size_t)sub * stride) : self;
+    int q1 = sub + L < c ? nb_list_load<false>(list + (size_t)(sub + L) * stride) : self;
+    for (int k = 0; k < cm; k += L) {
+      const int j = q0, kk = k + 2 * L + sub;
+      q0 = q1;
+      q1 = kk < c ? nb_list_load<false>(list + (size_t)kk * stride) : self;
+      const auto t = term(load(j));
+#pragma unroll
+      for (int e = 0; e < L; ++e) {
+        const auto u = shfl_reals(t, e * P + p);
+        if (k + e < c) fold(u);
+      }
+    }
   }
 }
 

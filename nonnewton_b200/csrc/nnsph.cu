@@ -61,12 +61,13 @@ struct nn_ctx {
   int unroll = NN_DEFAULT_UNROLL;      // neighbour chains in flight per thread (1, 2, 4; 0: per pass)
   int cell_factor = 1;                 // cells of edge h / cell_factor
   int x_split = NN_DEFAULT_XSPLIT;     // x cells per cell edge
+  int lanes = 1;                       // lanes per particle of the neighbour passes (lanes_for)
   // state binding and scenes
   nn_state state{};
   bool bound = false;
   std::vector<nn_scene_desc> scenes;
   std::vector<SceneDev> sdev;
-  int n = 0, ncells = 0, ne = 0;
+  int n = 0, n_fluid = 0, ncells = 0, ne = 0;
   bool any_fluid = false, any_div = false, any_nonnewton = false, any_implicit = false, any_cfl = false;
   int forces_feat = 0;                 // FF_* terms of the force pass any scene needs
   bool fold_np = false;                // the step takes the fluid's non-pressure terms from the
@@ -120,7 +121,20 @@ static uint64_t feature_sig(const nn_ctx* c) {
   return (uint64_t)c->any_fluid | ((uint64_t)c->any_div << 1) | ((uint64_t)c->any_nonnewton << 2) |
          ((uint64_t)c->any_implicit << 3) | ((uint64_t)std::min(c->el_mult_max, 255) << 8) |
          ((uint64_t)(c->ne > 0) << 16) | ((uint64_t)c->block << 20) |
-         ((uint64_t)c->forces_feat << 40) | ((uint64_t)c->fold_np << 48);
+         ((uint64_t)c->forces_feat << 40) | ((uint64_t)c->fold_np << 48) | ((uint64_t)c->lanes << 52);
+}
+
+// Lanes per particle of the neighbour passes (nb_sum), by the fluid particles they walk. A
+// thread's pass over its 26-odd neighbours is one chain of dependent loads and arithmetic,
+// 10-20 us however few particles there are; splitting it over L lanes shortens it until the
+// chip is full, and past that only costs the shuffles that fold the terms in list order.
+// Step times at 8 / 4 / 2 / 1 lanes (us): 2,197 fluid 209 / 225 / 264 / 287; 8,000 279 /
+// 284 / 322 / 368; 15,625 330 / 307 / 342 / 381; 24,389 361 / 321 / 345 / 382; 39,304
+// 486 / 427 / 389 / 433; 46,656 277 / 246 / 227 / 253; 68,921 667 / 542 / 517 / 468.
+// An explicit unroll (nn_set_tuning) selects the one-lane passes it names.
+static int lanes_for(const nn_ctx* c, int n_fluid) {
+  if (c->unroll) return 1;
+  return n_fluid <= 10000 ? 8 : n_fluid <= 28000 ? 4 : n_fluid <= 56000 ? 2 : 1;
 }
 
 static thread_local char g_err[512];
@@ -188,7 +202,7 @@ static Dev make_dev(nn_ctx* c, int cur) {
 // Launch helpers: grids are a multiple of the SM count (resident blocks per SM from
 // the occupancy calculator), capped by the work; kernels grid-stride over device sizes.
 template <typename... KArgs, typename... Args>
-static int launch(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, int work, Args... args) {
+static int launch_lanes(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, int work, int lanes, Args... args) {
   auto it = c->occ.find((const void*)k);
   int per_sm;
   if (it == c->occ.end()) {
@@ -202,7 +216,7 @@ static int launch(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, int
   // A captured graph must serve any batch composition up to the capacity, so its
   // grids are sized by the capacity (kernels grid-stride over the device sizes).
   if (c->in_capture) work = std::max(work, c->cap);
-  int64_t want = ((int64_t)std::max(work, 1) + block - 1) / block;
+  int64_t want = ((int64_t)std::max(work, 1) * lanes + block - 1) / block;
   int grid = (int)std::min<int64_t>(want, (int64_t)c->sms * per_sm);
   grid = std::max(grid, 1);
   k<<<grid, block, 0, s>>>(args...);
@@ -211,6 +225,15 @@ static int launch(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, int
   if (c->in_capture) c->capture_nodes++;
   else c->launches++;
   return NN_OK;
+}
+template <typename... KArgs, typename... Args>
+static int launch(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, int work, Args... args) {
+  return launch_lanes(c, s, k, block, work, 1, args...);
+}
+// A neighbour pass: c->lanes threads per particle.
+template <typename... KArgs, typename... Args>
+static int launch_nb(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, Args... args) {
+  return launch_lanes(c, s, k, block, c->n, c->lanes, args...);
 }
 template <typename... KArgs, typename... Args>
 static int launch1(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), Args... args) {
@@ -222,7 +245,7 @@ static int launch1(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), Args... args)
   return NN_OK;
 }
 
-// Each pass's neighbour-batch depth at unroll 0, measured against the other depth on
+// Each one-lane pass's neighbour-batch depth at unroll 0, measured against the other depth on
 // the 2.4M-particle dam break (early and settled states): the update passes, with
 // little arithmetic per pair, keep 2 neighbours in flight (at 1: k_pressure_update
 // +17-31 %, k_density_adv +3 %); the passes with more arithmetic per pair gather one
@@ -235,20 +258,31 @@ enum : int {
 };
 static inline int ku(const nn_ctx* c, int pass_default) { return c->unroll ? c->unroll : pass_default; }
 // The instantiation of a neighbour kernel for the context's (or the pass's) batch depth.
-#define KU(k, def) (ku(c, def) == 4 ? &k<4> : ku(c, def) == 2 ? &k<2> : &k<1>)
-#define KU2(k, B, def) (ku(c, def) == 4 ? &k<4, B> : ku(c, def) == 2 ? &k<2, B> : &k<1, B>)
+#define KU_(k, def, ...)                                                                        \
+  (c->lanes == 8   ? &k<1, 8 __VA_ARGS__>                                                       \
+   : c->lanes == 4 ? &k<1, 4 __VA_ARGS__>                                                       \
+   : c->lanes == 2 ? &k<1, 2 __VA_ARGS__>                                                       \
+   : ku(c, def) == 4 ? &k<4, 1 __VA_ARGS__>                                                     \
+   : ku(c, def) == 2 ? &k<2, 1 __VA_ARGS__>                                                     \
+                     : &k<1, 1 __VA_ARGS__>)
+#define COMMA ,
+#define KU(k, def) KU_(k, def, )
+#define KU2(k, B, def) KU_(k, def, COMMA B)
 
 // The force pass instance for the batch's terms (c->forces_feat) and batch depth.
-template <int U, int... F>
+template <int U, int L, int... F>
 static void (*forces_pick(int feat, std::integer_sequence<int, F...>))(Dev, int) {
-  static void (*const tbl[])(Dev, int) = {forces_kernel_of<U, F>()...};
+  static void (*const tbl[])(Dev, int) = {forces_kernel_of<U, L, F>()...};
   return tbl[feat];
 }
 static void (*forces_kernel(const nn_ctx* c))(Dev, int) {
   using All = std::make_integer_sequence<int, 16>;
   const int f = c->forces_feat & 15;
   const int u = ku(c, U_FORCES);
-  return u == 4 ? forces_pick<4>(f, All{}) : u == 2 ? forces_pick<2>(f, All{}) : forces_pick<1>(f, All{});
+  if (c->lanes == 8) return forces_pick<1, 8>(f, All{});
+  if (c->lanes == 4) return forces_pick<1, 4>(f, All{});
+  if (c->lanes == 2) return forces_pick<1, 2>(f, All{});
+  return u == 4 ? forces_pick<4, 1>(f, All{}) : u == 2 ? forces_pick<2, 1>(f, All{}) : forces_pick<1, 1>(f, All{});
 }
 
 #define RC(x)                 \
@@ -366,13 +400,13 @@ static int enq_divergence(nn_ctx* c, cudaStream_t s, bool fused) {
   if (!fused) RC(launch1(c, s, k_solver_begin, d, 0));
   RC(solver_loop(c, s, false,
                  [&](cudaStream_t q) {
-                   return fused ? NN_OK : launch(c, q, KU(k_density_change, U_DENSITY_CHANGE), B, c->n, make_dev(c, c->cur), 0, 0);
+                   return fused ? NN_OK : launch_nb(c, q, KU(k_density_change, U_DENSITY_CHANGE), B, make_dev(c, c->cur), 0, 0);
                  },
                  [&](cudaStream_t q) {
                    Dev e = make_dev(c, c->cur);
-                   RC(launch(c, q, KU(k_divergence_update, U_DIVERGENCE_UPDATE), B, c->n, e));
-                   RC(launch(c, q, KU(k_density_change, U_DENSITY_CHANGE), B, c->n, e, 1, np ? 1 : 0));
-                   if (np) RC(launch(c, q, KU(k_density_change_np, U_DENSITY_CHANGE_NP), B, c->n, e, 1, 1));
+                   RC(launch_nb(c, q, KU(k_divergence_update, U_DIVERGENCE_UPDATE), B, e));
+                   RC(launch_nb(c, q, KU(k_density_change, U_DENSITY_CHANGE), B, e, 1, np ? 1 : 0));
+                   if (np) RC(launch_nb(c, q, KU(k_density_change_np, U_DENSITY_CHANGE_NP), B, e, 1, 1));
                    return launch1(c, q, k_solver_check, e, 0, np ? 1 : 0);
                  }));
   return fused ? NN_OK : launch(c, s, k_alpha_times_dt, 256, c->n, d);
@@ -387,12 +421,12 @@ static int enq_pressure(nn_ctx* c, cudaStream_t s, int init_mode, bool begun = f
   if (!begun) RC(launch1(c, s, k_solver_begin, d, 1));
   return solver_loop(c, s, false,
                      [&](cudaStream_t q) {
-                       return launch(c, q, KU(k_density_adv, U_DENSITY_ADV), B, c->n, make_dev(c, c->cur), init_mode);
+                       return launch_nb(c, q, KU(k_density_adv, U_DENSITY_ADV), B, make_dev(c, c->cur), init_mode);
                      },
                      [&](cudaStream_t q) {
                        Dev e = make_dev(c, c->cur);
-                       RC(launch(c, q, KU(k_pressure_update, U_PRESSURE_UPDATE), B, c->n, e));
-                       RC(launch(c, q, KU(k_density_adv, U_DENSITY_ADV), B, c->n, e, 1));
+                       RC(launch_nb(c, q, KU(k_pressure_update, U_PRESSURE_UPDATE), B, e));
+                       RC(launch_nb(c, q, KU(k_density_adv, U_DENSITY_ADV), B, e, 1));
                        return launch1(c, q, k_solver_check, e, 1, 0);
                      });
 }
@@ -404,13 +438,13 @@ static int enq_pressure(nn_ctx* c, cudaStream_t s, int init_mode, bool begun = f
 static int enq_nonpressure(nn_ctx* c, cudaStream_t s, int advect, int clear) {
   Dev d = make_dev(c, c->cur);
   const int B = c->block;
-  RC(launch(c, s, forces_kernel(c), B, c->n, d, clear));
+  RC(launch_nb(c, s, forces_kernel(c), B, d, clear));
   if (c->any_implicit) {
-    RC(launch(c, s, KU(k_cg_setup, U_CG_SETUP), B, c->n, d));
+    RC(launch_nb(c, s, KU(k_cg_setup, U_CG_SETUP), B, d));
     RC(solver_loop(c, s, true, [&](cudaStream_t q) { return launch1(c, q, k_cg_check0, make_dev(c, c->cur)); },
                    [&](cudaStream_t q) {
                      Dev e = make_dev(c, c->cur);
-                     RC(launch(c, q, KU(k_cg_matvec, U_CG_MATVEC), B, c->n, e));
+                     RC(launch_nb(c, q, KU(k_cg_matvec, U_CG_MATVEC), B, e));
                      RC(launch1(c, q, k_cg_alpha, e));
                      RC(launch(c, q, k_cg_update, 256, c->n, e));
                      RC(launch1(c, q, k_cg_check, e));
@@ -456,10 +490,10 @@ static int enq_substep(nn_ctx* c, cudaStream_t s, bool begun = false) {
   Dev d = make_dev(c, c->cur);
   if (c->any_div) {
     if (!begun) RC(launch1(c, s, k_solver_begin, d, 0));
-    RC(launch(c, s, KU2(k_density_factor, true, U_DENSITY_FACTOR), c->block, c->n, d, 1, 1));
+    RC(launch_nb(c, s, KU2(k_density_factor, true, U_DENSITY_FACTOR), c->block, d, 1, 1));
     RC(enq_divergence(c, s, true));
   } else {
-    RC(launch(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, c->n, d, 1, 1));
+    RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 1, 1));
   }
   RC(enq_nonpressure(c, s, 1, 1));
   return enq_pressure(c, s, 2, begun);
@@ -471,7 +505,7 @@ static int enq_step(nn_ctx* c, cudaStream_t s) {
   // start in k_clear_acc's first block: one-block kernels cost a graph node each
   RC(enq_search(c, s, true));
   Dev d = make_dev(c, c->cur);
-  RC(launch(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, c->n, d, 1));
+  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1));
   RC(launch(c, s, k_clear_acc, 256, c->n, d, c->fold_np ? 1 : 0, 1));
   RC(enq_substep(c, s, true));
   RC(enq_elastic(c, s));
@@ -767,6 +801,7 @@ int nn_set_tuning(nn_ctx* c, int32_t block, int32_t unroll, int32_t cell_factor)
   if (cell_factor != c->cell_factor) c->scenes.clear();  // cell layout changes: set the scenes again
   c->block = block;
   c->unroll = unroll;
+  c->lanes = lanes_for(c, c->n_fluid);
   c->cell_factor = cell_factor;
   c->occ.clear();
   return NN_OK;
@@ -911,6 +946,9 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
   if (cells > c->max_cells) drop_graphs(c);  // the scan grids were sized for the old table
   RC(ensure_cells(c, cells));
   c->ne = (int)el_id.size();
+  c->n_fluid = 0;
+  for (int k = 0; k < nscenes; ++k) c->n_fluid += scenes[k].n_fluid;
+  c->lanes = lanes_for(c, c->n_fluid);
   // elastic buffers are reallocated below (their pointers and stride are graph arguments)
   if (feature_sig(c) != c->graph_sig || c->ne > 0) drop_graphs(c);
   c->scenes.assign(scenes, scenes + nscenes);
@@ -1017,8 +1055,8 @@ int nn_initialize(nn_ctx* c) {
     RC(launch(c, s, k_rigid_com, 256, c->n, d, r, 1));
     RC(launch1(c, s, k_rigid_cm, d, r, 1));
   }
-  RC(launch(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, c->n, d, 0));
-  RC(launch(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, c->n, d, 1));
+  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 0));
+  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1));
   RC(enq_sync_out(c, s, SM_VOL));
   CK(cudaStreamSynchronize(s));
   c->el_stale = false;
@@ -1074,11 +1112,11 @@ int nn_run_pass(nn_ctx* c, int32_t pass) {
   RC(launch(c, s, k_sync_in, 256, c->n, d, (uint32_t)SM_ALL));
   RC(launch1(c, s, k_step_dt, d, 0));
   switch (pass) {
-    case NN_PASS_STATIC_BOUNDARY_VOLUME: RC(launch(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, c->n, d, 0)); break;
-    case NN_PASS_MOVING_BOUNDARY_VOLUME: RC(launch(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, c->n, d, 1)); break;
+    case NN_PASS_STATIC_BOUNDARY_VOLUME: RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 0)); break;
+    case NN_PASS_MOVING_BOUNDARY_VOLUME: RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1)); break;
     case NN_PASS_CLEAR_ACCELERATIONS: RC(launch(c, s, k_clear_acc, 256, c->n, d, 0, 0)); break;
-    case NN_PASS_DENSITIES: RC(launch(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, c->n, d, 1, 0)); break;
-    case NN_PASS_DFSPH_FACTOR: RC(launch(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, c->n, d, 0, 1)); break;
+    case NN_PASS_DENSITIES: RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 1, 0)); break;
+    case NN_PASS_DFSPH_FACTOR: RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 0, 1)); break;
     case NN_PASS_DIVERGENCE_SOLVE: if (c->any_div) RC(enq_divergence(c, s, false)); break;
     case NN_PASS_NON_PRESSURE_FORCES: if (c->any_fluid) RC(enq_nonpressure(c, s, 0, 0)); break;
     case NN_PASS_NON_PRESSURE_ADVECT: RC(launch(c, s, k_np_advect, 256, c->n, d)); break;
@@ -1127,18 +1165,18 @@ int nn_time_kernel(nn_ctx* c, int32_t kernel, int32_t reps, float* ms_out) {
   auto one = [&]() -> int {
     const int B = c->block;
     switch (kernel) {
-      case NN_K_PRESSURE_UPDATE: return launch(c, s, KU(k_pressure_update, U_PRESSURE_UPDATE), B, c->n, d);
-      case NN_K_DENSITY_ADV: return launch(c, s, KU(k_density_adv, U_DENSITY_ADV), B, c->n, d, 1);
-      case NN_K_DIVERGENCE_UPDATE: return launch(c, s, KU(k_divergence_update, U_DIVERGENCE_UPDATE), B, c->n, d);
-      case NN_K_DENSITY_CHANGE: return launch(c, s, KU(k_density_change, U_DENSITY_CHANGE), B, c->n, d, 1, 0);
-      case NN_K_DENSITY_CHANGE_NP: return launch(c, s, KU(k_density_change_np, U_DENSITY_CHANGE_NP), B, c->n, d, 1, 0);
+      case NN_K_PRESSURE_UPDATE: return launch_nb(c, s, KU(k_pressure_update, U_PRESSURE_UPDATE), B, d);
+      case NN_K_DENSITY_ADV: return launch_nb(c, s, KU(k_density_adv, U_DENSITY_ADV), B, d, 1);
+      case NN_K_DIVERGENCE_UPDATE: return launch_nb(c, s, KU(k_divergence_update, U_DIVERGENCE_UPDATE), B, d);
+      case NN_K_DENSITY_CHANGE: return launch_nb(c, s, KU(k_density_change, U_DENSITY_CHANGE), B, d, 1, 0);
+      case NN_K_DENSITY_CHANGE_NP: return launch_nb(c, s, KU(k_density_change_np, U_DENSITY_CHANGE_NP), B, d, 1, 0);
       case NN_K_DENSITY_FACTOR:  // the instance the step runs (with the first density change)
-        return c->any_div ? launch(c, s, KU2(k_density_factor, true, U_DENSITY_FACTOR), B, c->n, d, 1, 1)
-                          : launch(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), B, c->n, d, 1, 1);
+        return c->any_div ? launch_nb(c, s, KU2(k_density_factor, true, U_DENSITY_FACTOR), B, d, 1, 1)
+                          : launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), B, d, 1, 1);
       case NN_K_BUILD_LISTS: return launch(c, s, k_build_lists, NS_WARPS * 32, c->n, d);
-      case NN_K_CG_MATVEC: return launch(c, s, KU(k_cg_matvec, U_CG_MATVEC), B, c->n, d);
-      case NN_K_CG_SETUP: return launch(c, s, KU(k_cg_setup, U_CG_SETUP), B, c->n, d);
-      default: return launch(c, s, forces_kernel(c), B, c->n, d, 0);
+      case NN_K_CG_MATVEC: return launch_nb(c, s, KU(k_cg_matvec, U_CG_MATVEC), B, d);
+      case NN_K_CG_SETUP: return launch_nb(c, s, KU(k_cg_setup, U_CG_SETUP), B, d);
+      default: return launch_nb(c, s, forces_kernel(c), B, d, 0);
     }
   };
   RC(one());  // warm-up

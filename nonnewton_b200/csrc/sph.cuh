@@ -20,24 +20,24 @@ struct GPV { real4 p, v; };
 
 // ---------------------------------------------------------------------------
 // compute_static_boundary_volume / compute_moving_boundary_volume (SPH/main.py:1010-1035)
-template <int U>
+template <int U, int L>
 __global__ void k_boundary_volume(Dev d, int moving) {
   const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
-    const uint32_t fl = d.w.flags[i];
-    if (moving ? !cls_dyn_solid(fl) : !cls_static_solid(fl)) continue;
+  FOR_SPLIT(L, i, sub, valid, n) {
+    const uint32_t fl = valid ? d.w.flags[i] : 0u;
+    const bool work = valid && (moving ? cls_dyn_solid(fl) : cls_static_solid(fl));
+    if (!__any_sync(0xffffffffu, work)) continue;
     const SceneDev& s = d.sc[slot_scene(fl)];
-    const real3 xi = f3(d.w.pos[i]);
+    const real3 xi = work ? f3(d.w.pos[i]) : make_real3(0.f, 0.f, 0.f);
     real delta = s.W0;
     // plain loads: this pass writes pos.w of solid slots (the sign never changes)
-    nb_batches<U>(d.nbr + i, d.cap, d.nbr_cnt[i], i, [&](int j) { return d.w.pos[j]; },
-               [&](int, real4 pj) {
-                 if (!w_fluid(pj.w)) {
+    nb_sum<U, L>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, work ? i : 0, sub, [&](int j) { return d.w.pos[j]; },
+                 [&](real4 pj) {
                    const real3 r = xi - f3(pj);
-                   delta += kw_r2(dot3(r, r), s);
-                 }
-               });
-    d.w.pos[i].w = -(1.f / delta * 3.f);
+                   return w_fluid(pj.w) ? real(0) : kw_r2(dot3(r, r), s);
+                 },
+                 [&](real w) { delta += w; });
+    if (work && sub == 0) d.w.pos[i].w = -(1.f / delta * 3.f);
   }
 }
 
@@ -75,48 +75,57 @@ __global__ void k_clear_acc(Dev d, int solid_terms, int step_start) {
 // and, with CHANGE, the divergence solve's first compute_density_change and
 // alpha *= 1/dt (SPH/main.py:1686-1688): all read the same neighbours at the same
 // positions and velocities, and each only needs the particle's own factor.
-template <int U, bool CHANGE>
+struct TFactor { real V, w, gx, gy, gz, gg, dv; };  // volume, W, grad W, |V grad W|^2 (fluid), v_ij . grad W
+template <int U, int L, bool CHANGE>
 __global__ void k_density_factor(Dev d, int do_density, int do_factor) {
   const int n = d.d_n[0];
-  FOR_SLOTS_WARP(i, valid, n) {
+  FOR_SPLIT(L, i, sub, valid, n) {
     const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const bool work = valid && cls_fluid(fl);
     const int scn = slot_scene(fl);
     real rho = 0.f;
+    if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
+    const SceneDev& s = d.sc[scn];
+    const int self = work ? i : 0;
+    const real4 pi = d.w.pos[self];
+    const real3 xi = f3(pi);
+    const real3 vi = f3(d.w.vel[self]);
+    const int c = work ? d.nbr_cnt[i] : 0;
+    real den = 0.f, sum_grad = 0.f, dd = 0.f;
+    real3 gpi = make_real3(0.f, 0.f, 0.f);
+    auto term = [&](real4 pj, real4 vj) {
+      const real3 r = xi - f3(pj);
+      TFactor t;
+      real3 g;
+      kwg_r2(r, dot3(r, r), s, t.w, g);
+      t.V = fabs(pj.w);
+      const real3 gpj = g * t.V;
+      t.gg = w_fluid(pj.w) ? dot3(gpj, gpj) : real(0);
+      t.gx = g.x; t.gy = g.y; t.gz = g.z;
+      t.dv = CHANGE ? dot3(vi - f3(vj), g) : real(0);
+      return t;
+    };
+    auto fold = [&](const TFactor& t) {
+      den = fma(t.V, t.w, den);
+      sum_grad += t.gg;
+      gpi = make_real3(fma(t.gx, t.V, gpi.x), fma(t.gy, t.V, gpi.y), fma(t.gz, t.V, gpi.z));
+      if (CHANGE) dd = fma(t.V, t.dv, dd);
+    };
+    if constexpr (CHANGE) {
+      nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
+                   [&](const GPV& g) { return term(g.p, g.v); }, fold);
+    } else {
+      nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return pos_of(d, j); },
+                   [&](real4 pj) { return term(pj, pj); }, fold);
+    }
     if (work) {
-      const SceneDev& s = d.sc[scn];
-      const real4 pi = d.w.pos[i];
-      const real3 xi = f3(pi);
-      const real3 vi = f3(d.w.vel[i]);
-      const int c = d.nbr_cnt[i];
-      real den = 0.f, sum_grad = 0.f, dd = 0.f;
-      real3 gpi = make_real3(0.f, 0.f, 0.f);
-      auto body = [&](real4 pj, real4 vj) {
-        const real3 r = xi - f3(pj);
-        real w;
-        real3 g;
-        kwg_r2(r, dot3(r, r), s, w, g);
-        const real V = fabs(pj.w);
-        den += V * w;
-        const real3 gpj = g * (-V);
-        if (w_fluid(pj.w)) sum_grad += dot3(gpj, gpj);
-        gpi -= gpj;
-        if (CHANGE) dd += V * dot3(vi - f3(vj), g);
-      };
-      if constexpr (CHANGE) {
-        nb_batches<U>(d.nbr + i, d.cap, c, i, [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
-                      [&](int, const GPV& g) { body(g.p, g.v); });
-      } else {
-        nb_batches<U>(d.nbr + i, d.cap, c, i, [&](int j) { return pos_of(d, j); },
-                      [&](int, real4 pj) { body(pj, pj); });
-      }
       if (do_density) {
         rho = pi.w * s.W0;
         rho += den;
         rho = rho * s.rho0;
-        d.w.dens[i] = rho;
+        if (sub == 0) d.w.dens[i] = rho;
       }
-      if (do_factor) {
+      if (do_factor && sub == 0) {
         sum_grad += dot3(gpi, gpi);
         real alpha = sum_grad > 1e-6f ? -1.f / sum_grad : 0.f;
         if (CHANGE && d.dyn[scn].act_v) {
@@ -129,12 +138,19 @@ __global__ void k_density_factor(Dev d, int do_density, int do_factor) {
         d.alpha[i] = alpha;
       }
     }
+    }
     if (do_density) warp_max_to(&d.dyn[scn].max_density_bits, __float_as_uint((float)rho), work);
   }
 }
 
 __device__ __forceinline__ real nn_law(real g, const SceneDev& s);
 __device__ __forceinline__ real strain_rate_norm(const real (&S)[6], real rho_i, bool quirks);
+// A neighbour's symmetric velocity gradient v_ji (x) grad W + its transpose, without the
+// mass: 00 11 22 01 02 12 (calcStrainRate, SPH/main.py:461-492).
+__device__ __forceinline__ void strain_term(real3 v, real3 g, real (&e)[6]) {
+  e[0] = v.x * g.x + v.x * g.x; e[1] = v.y * g.y + v.y * g.y; e[2] = v.z * g.z + v.z * g.z;
+  e[3] = fma(v.x, g.y, v.y * g.x); e[4] = fma(v.x, g.z, v.z * g.x); e[5] = fma(v.y, g.z, v.z * g.y);
+}
 
 // compute_density_change (SPH/main.py:1610-1645). mode 0: first call of
 // divergence_solve, also applies alpha *= 1/dt (1688); mode 1: solver iteration,
@@ -153,120 +169,171 @@ __device__ __forceinline__ real strain_rate_norm(const real (&S)[6], real rho_i,
 // mode); the solids' outputs come from k_clear_acc.
 // `sel` = 1 in such a loop: the plain instance skips, and the NP instance takes, the
 // scenes whose np_body this body is; 0: every scene.
-template <int U, bool NP>
-__device__ __forceinline__ void density_change_body(Dev d, int mode, int sel) {
+struct TDiv { real V, dv; };  // volume, v_ij . grad W
+// with the non-pressure terms: surface tension (sx, sy, sz) * sw and strain rate e * m
+struct TDivNp { real V, dv, sx, sy, sz, sw, m, e[6]; };
+template <int U, int L, bool NP>
+__device__ __forceinline__ void density_change_body(const Dev& d, int mode, int sel) {
   const int n = d.d_n[0];
-  FOR_SLOTS_WARP(i, valid, n) {
+  FOR_SPLIT(L, i, sub, valid, n) {
     uint32_t fl = valid ? d.w.flags[i] : 0u;
     const int scn = slot_scene(fl);
     const SceneDyn& y = d.dyn[scn];
     const bool np_here = sel && y.it_v == y.np_body;
-    bool work = valid && cls_fluid(fl) && y.act_v && (NP ? (np_here || !sel) : !np_here);
+    const bool work = valid && cls_fluid(fl) && y.act_v && (NP ? (np_here || !sel) : !np_here);
     double err = 0.0;
-    if (work) {
+    if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
       const SceneDev& s = d.sc[scn];
-      const real3 xi = f3(d.w.pos[i]);
-      const real3 vi = f3(d.w.vel[i]);
-      const int c = d.nbr_cnt[i];
+      const int self = work ? i : 0;
+      const real3 xi = f3(d.w.pos[self]);
+      const real3 vi = f3(d.w.vel[self]);
+      const int c = work ? d.nbr_cnt[i] : 0;
       real dd = 0.f;
       if constexpr (!NP) {
-        nb_batches<U>(d.nbr + i, d.cap, c, i, [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
-                   [&](int, const GPV& g) {
-                     const real3 r = xi - f3(g.p);
-                     dd += fabs(g.p.w) * dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s));
-                   });
+        nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
+                     [&](const GPV& g) {
+                       const real3 r = xi - f3(g.p);
+                       return TDiv{fabs(g.p.w), dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s))};
+                     },
+                     [&](const TDiv& t) { dd = fma(t.V, t.dv, dd); });
       } else {
         const bool st_on = (s.flags & NN_F_SURFACE_TENSION) != 0;
         const bool sr_on = (s.flags & NN_F_NONNEWTON) != 0;
-        const real mi = d.w.mass[i];
+        const real mi = d.w.mass[self];
         real3 st = make_real3(0.f, 0.f, 0.f);
         real S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // strain-rate sum: 00 11 22 01 02 12
-        nb_batches<U>(d.nbr + i, d.cap, c, i, [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
-                   [&](int, const GPV& g) {
-                     const real3 r = xi - f3(g.p);
-                     const real r2 = dot3(r, r);
-                     real w;
-                     real3 gw;
-                     kwg_r2(r, r2, s, w, gw);
-                     dd += fabs(g.p.w) * dot3(vi - f3(g.v), gw);
-                     const real mj = g.v.w;
-                     if (st_on && w_fluid(g.p.w)) st -= (r * (s.sigma / mi * mj)) * (r2 > s.dia2 ? w : s.w_dia);
-                     if (sr_on) {
-                       const real3 vji = f3(g.v) - vi;
-                       const real t[6] = {(vji.x * gw.x + vji.x * gw.x) * mj, (vji.y * gw.y + vji.y * gw.y) * mj,
-                                           (vji.z * gw.z + vji.z * gw.z) * mj, (vji.x * gw.y + vji.y * gw.x) * mj,
-                                           (vji.x * gw.z + vji.z * gw.x) * mj, (vji.y * gw.z + vji.z * gw.y) * mj};
+        auto load = [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; };
+        auto add_st = [&](real3 b, real sw) { st = make_real3(fma(-b.x, sw, st.x), fma(-b.y, sw, st.y), fma(-b.z, sw, st.z)); };
+        auto add_sr = [&](const real (&e)[6], real m) {
 #pragma unroll
-                       for (int k = 0; k < 6; ++k) S[k] += t[k];
-                     }
-                   });
-        real4 a = make_real4(s.g[0], s.g[1], s.g[2], 0.f);
-        if (st_on) { a.x += st.x; a.y += st.y; a.z += st.z; }
-        d.acc4[i] = a;
-        const real rho_i = d.w.dens[i];
-        real mu = s.mu_newton;
-        if (sr_on) {
-          const real g = strain_rate_norm(S, rho_i, false);
-          mu = nn_law(g, s);
-          d.srn[i] = g;
-          d.mu[i] = mu;
+          for (int k = 0; k < 6; ++k) S[k] = fma(e[k], m, S[k]);
+        };
+        // a term struct with the lanes' common operands costs registers that one lane per
+        // particle does not have at its cap (40 B spilled): it adds each sum where it is made
+        if constexpr (L == 1) {
+          nb_batches<U>(d.nbr + i, d.cap, c, self, load, [&](int, const GPV& g) {
+            const real3 r = xi - f3(g.p);
+            const real r2 = dot3(r, r);
+            real w;
+            real3 gw;
+            kwg_r2(r, r2, s, w, gw);
+            dd = fma(fabs(g.p.w), dot3(vi - f3(g.v), gw), dd);
+            const real mj = g.v.w;
+            if (st_on && w_fluid(g.p.w)) add_st(r * (s.sigma / mi * mj), r2 > s.dia2 ? w : s.w_dia);
+            if (sr_on) {
+              real e[6];
+              strain_term(f3(g.v) - vi, gw, e);
+              add_sr(e, mj);
+            }
+          });
+        } else {
+          nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, load,
+                       [&](const GPV& g) {
+                         TDivNp t;
+                         const real3 r = xi - f3(g.p);
+                         const real r2 = dot3(r, r);
+                         real w;
+                         real3 gw;
+                         kwg_r2(r, r2, s, w, gw);
+                         t.V = fabs(g.p.w);
+                         t.dv = dot3(vi - f3(g.v), gw);
+                         t.m = g.v.w;
+                         const real3 b = r * (s.sigma / mi * t.m);
+                         t.sx = b.x; t.sy = b.y; t.sz = b.z;
+                         t.sw = st_on && w_fluid(g.p.w) ? (r2 > s.dia2 ? w : s.w_dia) : real(0);
+                         strain_term(f3(g.v) - vi, gw, t.e);
+                         return t;
+                       },
+                       [&](const TDivNp& t) {
+                         dd = fma(t.V, t.dv, dd);
+                         if (st_on) add_st(make_real3(t.sx, t.sy, t.sz), t.sw);
+                         if (sr_on) add_sr(t.e, t.m);
+                       });
         }
-        if (scene_implicit(s)) d.cg_aux[i] = make_real2(mu, mi / rho_i);
+        if (work && sub == 0) {
+          real4 a = make_real4(s.g[0], s.g[1], s.g[2], 0.f);
+          if (st_on) { a.x += st.x; a.y += st.y; a.z += st.z; }
+          d.acc4[i] = a;
+          const real rho_i = d.w.dens[i];
+          real mu = s.mu_newton;
+          if (sr_on) {
+            const real g = strain_rate_norm(S, rho_i, false);
+            mu = nn_law(g, s);
+            d.srn[i] = g;
+            d.mu[i] = mu;
+          }
+          if (scene_implicit(s)) d.cg_aux[i] = make_real2(mu, mi / rho_i);
+        }
       }
-      dd = fmax(dd, real(0));
-      if (c < 20) dd = 0.f;
-      d.rho_adv[i] = dd;
-      real a = d.alpha[i];
-      if (mode == 0) {
-        a = a * d.dyn[scn].inv_dt;
-        d.alpha[i] = a;
+      if (work && sub == 0) {
+        dd = fmax(dd, real(0));
+        if (c < 20) dd = 0.f;
+        d.rho_adv[i] = dd;
+        real a = d.alpha[i];
+        if (mode == 0) {
+          a = a * d.dyn[scn].inv_dt;
+          d.alpha[i] = a;
+        }
+        d.kappa[i] = dd * a;
+        err = (double)(s.rho0 * dd - 0.f);
       }
-      d.kappa[i] = dd * a;
-      err = (double)(s.rho0 * dd - 0.f);
     }
     // one reduction per warp and slot group: per-lane partial sums kept across the
     // loop (as in k_density_adv) measured 18 % slower here
-    if (mode == 1) scene_add(d.acc, ACC_ERR, 0, scn, work, err);
+    if (mode == 1) scene_add(d.acc, ACC_ERR, 0, scn, work && sub == 0, err);
   }
 }
-template <int U>
-__global__ void NN_PASS_REGS k_density_change(Dev d, int mode, int sel) { density_change_body<U, false>(d, mode, sel); }
+template <int U, int L>
+__global__ void NN_PASS_REGS k_density_change(Dev d, int mode, int sel) { density_change_body<U, L, false>(d, mode, sel); }
 // The NP instance is capped at 64 registers: uncapped it takes 79 (6 blocks of 128 per
 // SM) and ran 0.455 ms on the 2.4M scene, capped 0.428 ms (44 bytes spilled).
-template <int U>
-__global__ void NN_REGS64 k_density_change_np(Dev d, int mode, int sel) { density_change_body<U, true>(d, mode, sel); }
+template <int U, int L>
+__global__ void NN_REGS64 k_density_change_np(Dev d, int mode, int sel) { density_change_body<U, L, true>(d, mode, sel); }
 
 // divergence_solver_iteration_kernel (SPH/main.py:1721-1760). The pushes onto
 // dynamic solids (1755-1760) are omitted: clear_accelerations (1552) discards them.
+//
+// A pair moves v_i by V_j grad W * dt (k_i + k_j) where |k_i + k_j| > eps, with k_j = 0 for
+// solid j (whose k is not kept): both of the reference's branches, without a divergent one.
 struct GPK { real4 p; real k; };
-template <int U>
-__global__ void NN_PASS_REGS k_divergence_update(Dev d) {
+struct TPush { real x, y, z, c; };  // V_j grad W, dt * (k_i + k_j)
+__device__ __forceinline__ TPush push_term(real3 xi, const GPK& g, real k_i, real dt, const SceneDev& s) {
+  const real3 r = xi - f3(g.p);
+  const real ks = k_i + (w_fluid(g.p.w) ? g.k : real(0));
+  if (!(fabs(ks) > s.eps)) return TPush{0.f, 0.f, 0.f, 0.f};
+  const real3 a = kgrad_r2(r, dot3(r, r), s) * fabs(g.p.w);
+  return TPush{a.x, a.y, a.z, dt * ks};
+}
+__device__ __forceinline__ void push_fold(real3& v, const TPush& t) {
+  v = make_real3(fma(t.x, t.c, v.x), fma(t.y, t.c, v.y), fma(t.z, t.c, v.z));
+}
+template <int U, int L>
+__device__ __forceinline__ void divergence_update_body(const Dev& d) {
   const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
-    const uint32_t fl = d.w.flags[i];
-    if (!cls_fluid(fl)) continue;
+  FOR_SPLIT(L, i, sub, valid, n) {
+    const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const int scn = slot_scene(fl);
-    if (!d.dyn[scn].act_v) continue;
+    const bool work = valid && cls_fluid(fl) && d.dyn[scn].act_v;
+    if (L == 1 ? !work : !__any_sync(0xffffffffu, work)) continue;
     const SceneDev& s = d.sc[scn];
     const real dt = d.dyn[scn].dt;
-    const real3 xi = f3(d.w.pos[i]);
-    const real k_i = d.kappa[i];
+    const int self = work ? i : 0;
+    const real3 xi = f3(d.w.pos[self]);
+    const real k_i = d.kappa[self];
     real3 dv = make_real3(0.f, 0.f, 0.f);
-    nb_batches<U>(d.nbr + i, d.cap, d.nbr_cnt[i], i, [&](int j) { return GPK{pos_of(d, j), ldg(&d.kappa[j])}; },
-               [&](int, const GPK& g) {
-                 const real3 r = xi - f3(g.p);
-                 if (w_fluid(g.p.w)) {
-                   const real k_sum = k_i + g.k;
-                   if (fabs(k_sum) > s.eps) dv -= kgrad_r2(r, dot3(r, r), s) * (-g.p.w) * (dt * k_sum);
-                 } else if (fabs(k_i) > s.eps) {
-                   dv += kgrad_r2(r, dot3(r, r), s) * g.p.w * ((-dt * 1.f) * k_i);
-                 }
-               });
-    real4 v = d.w.vel[i];
-    v.x += dv.x; v.y += dv.y; v.z += dv.z;
-    d.w.vel[i] = v;
+    nb_sum<U, L>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, self, sub,
+                 [&](int j) { return GPK{pos_of(d, j), ldg(&d.kappa[j])}; },
+                 [&](const GPK& g) { return push_term(xi, g, k_i, dt, s); },
+                 [&](const TPush& t) { push_fold(dv, t); });
+    if (work && sub == 0) {
+      real4 v = d.w.vel[i];
+      v.x += dv.x; v.y += dv.y; v.z += dv.z;
+      d.w.vel[i] = v;
+    }
   }
 }
+template <int U, int L>
+__global__ void NN_PASS_REGS k_divergence_update(Dev d) { divergence_update_body<U, L>(d); }
 
 // multiply_time_step (SPH/main.py:1677-1681): alpha *= dt after the divergence loop.
 __global__ void k_alpha_times_dt(Dev d) {
@@ -286,93 +353,102 @@ __global__ void k_alpha_times_dt(Dev d) {
 // (nb_batches<U, true>) and the list build writes them streaming: -2 % here and
 // -10 % in k_pressure_update, the step 3.475 -> 3.435 ms on the 2.4M scene (the other
 // passes measured flat or slower with it).
-template <int U>
-__global__ void NN_PASS_REGS k_density_adv(Dev d, int mode) {
+template <int U, int L>
+__device__ __forceinline__ void density_adv_body(const Dev& d, int mode) {
   const int n = d.d_n[0];
   LaneSums<1> sums;
   const int q[1] = {ACC_ERR};
-  FOR_SLOTS_WARP(i, valid, n) {
+  FOR_SPLIT(L, i, sub, valid, n) {
     uint32_t fl = valid ? d.w.flags[i] : 0u;
     const int scn = slot_scene(fl);
-    bool work = valid && cls_fluid(fl) && d.dyn[scn].act_p;
+    const bool work = valid && cls_fluid(fl) && d.dyn[scn].act_p;
     double err = 0.0;
-    if (work) {
+    if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
       const SceneDev& s = d.sc[scn];
       const real dt = d.dyn[scn].dt;
-      const real3 xi = f3(d.w.pos[i]);
-      const real3 vi = f3(d.w.vel[i]);
+      const int self = work ? i : 0;
+      const real3 xi = f3(d.w.pos[self]);
+      const real3 vi = f3(d.w.vel[self]);
       real delta = 0.f;
-      nb_batches<U, true>(d.nbr + i, d.cap, d.nbr_cnt[i], i,
+      nb_sum<U, L, true>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, self, sub,
                  [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
-                 [&](int, const GPV& g) {
+                 [&](const GPV& g) {
                    const real3 r = xi - f3(g.p);
-                   delta += fabs(g.p.w) * dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s));
-                 });
-      real da = d.w.dens[i] * s.inv_rho0 + dt * delta;
-      da = fmax(da, real(1));
-      d.rho_adv[i] = da;
-      real a = d.alpha[i];
-      if (mode != 1) {
-        // mode 2 also applies the divergence solve's closing alpha *= dt (1713)
-        if (mode == 2 && d.dyn[scn].div_ran) a = a * d.dyn[scn].dt;
-        a = a * d.dyn[scn].inv_dt2;
-        d.alpha[i] = a;
+                   return TDiv{fabs(g.p.w), dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s))};
+                 },
+                 [&](const TDiv& t) { delta = fma(t.V, t.dv, delta); });
+      if (work && sub == 0) {
+        real da = d.w.dens[i] * s.inv_rho0 + dt * delta;
+        da = fmax(da, real(1));
+        d.rho_adv[i] = da;
+        real a = d.alpha[i];
+        if (mode != 1) {
+          // mode 2 also applies the divergence solve's closing alpha *= dt (1713)
+          if (mode == 2 && d.dyn[scn].div_ran) a = a * d.dyn[scn].dt;
+          a = a * d.dyn[scn].inv_dt2;
+          d.alpha[i] = a;
+        }
+        d.kappa[i] = (da - 1.f) * a;
+        err = (double)(s.rho0 * da - s.rho0);
       }
-      d.kappa[i] = (da - 1.f) * a;
-      err = (double)(s.rho0 * da - s.rho0);
     }
-    if (mode == 1) sums.add(d.acc, q, work, scn, {err});
+    if (mode == 1) sums.add(d.acc, q, work && sub == 0, scn, {err});
   }
   if (mode == 1) sums.flush(d.acc, q);
 }
+template <int U, int L>
+__global__ void NN_PASS_REGS k_density_adv(Dev d, int mode) { density_adv_body<U, L>(d, mode); }
 
 // pressure_solve_iteration_kernel (SPH/main.py:1799-1841). Fluid slots update v in
 // place per neighbour; dynamic solid slots gather the two-way coupling acceleration
 // from their fluid neighbours (the reference scatters it with atomics, 1835-1841).
-template <int U>
-__global__ void NN_PASS_REGS k_pressure_update(Dev d) {
+template <int U, int L>
+__device__ __forceinline__ void pressure_update_body(const Dev& d) {
   const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
-    const uint32_t fl = d.w.flags[i];
+  FOR_SPLIT(L, i, sub, valid, n) {
+    const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const bool fluid = cls_fluid(fl);
-    if (!fluid && !cls_dyn_solid(fl)) continue;
     const int scn = slot_scene(fl);
-    if (!d.dyn[scn].act_p) continue;
+    const bool work = valid && (fluid || cls_dyn_solid(fl)) && d.dyn[scn].act_p;
+    if (L == 1 ? !work : !__any_sync(0xffffffffu, work)) continue;
     const SceneDev& s = d.sc[scn];
     const real dt = d.dyn[scn].dt;
-    const real4 pi = d.w.pos[i];
+    const int self = work ? i : 0;
+    const real4 pi = d.w.pos[self];
     const real3 xi = f3(pi);
+    const int c = work ? d.nbr_cnt[i] : 0;
     auto load = [&](int j) { return GPK{pos_of(d, j), ldg(&d.kappa[j])}; };
-    if (fluid) {
-      const real k_i = d.kappa[i];
-      real4 v4 = d.w.vel[i];
+    if (L == 1 ? fluid : __any_sync(0xffffffffu, work && fluid)) {
+      const real k_i = d.kappa[self];
+      const real4 v4 = d.w.vel[self];
       real3 vi = f3(v4);
-      nb_batches<U, true>(d.nbr + i, d.cap, d.nbr_cnt[i], i, load, [&](int, const GPK& g) {
-        const real3 r = xi - f3(g.p);
-        if (w_fluid(g.p.w)) {
-          const real k_sum = k_i + g.k;
-          if (fabs(k_sum) > s.eps) vi -= kgrad_r2(r, dot3(r, r), s) * (-g.p.w) * (dt * k_sum);
-        } else if (fabs(k_i) > s.eps) {
-          vi += kgrad_r2(r, dot3(r, r), s) * g.p.w * ((-dt * 1.f) * k_i);
-        }
-      });
-      d.w.vel[i] = make_real4(vi.x, vi.y, vi.z, v4.w);
-    } else {
+      nb_sum<U, L, true>(d.nbr + i, d.cap, fluid ? c : 0, self, sub, load,
+                         [&](const GPK& g) { return push_term(xi, g, k_i, dt, s); },
+                         [&](const TPush& t) { push_fold(vi, t); });
+      if (work && fluid && sub == 0) d.w.vel[i] = make_real4(vi.x, vi.y, vi.z, v4.w);
+    }
+    if (L == 1 ? !fluid : __any_sync(0xffffffffu, work && !fluid)) {
       const real Vi = fabs(pi.w);
       const real inv_dt = 1.f / dt;
       real3 ai = make_real3(0.f, 0.f, 0.f);
-      nb_batches<U, true>(d.nbr + i, d.cap, d.nbr_cnt[i], i, load, [&](int, const GPK& g) {
-        if (!w_fluid(g.p.w) || !(fabs(g.k) > s.eps)) return;
-        const real3 r = f3(g.p) - xi;  // x_fluid - x_solid, as the fluid computes it
-        const real3 vc = kgrad_r2(r, dot3(r, r), s) * (-Vi) * ((-dt * 1.f) * g.k);
-        ai -= vc * inv_dt;
-      });
-      real4 a = d.acc4[i];
-      a.x += ai.x; a.y += ai.y; a.z += ai.z;
-      d.acc4[i] = a;
+      nb_sum<U, L, true>(d.nbr + i, d.cap, fluid ? 0 : c, self, sub, load,
+                         [&](const GPK& g) {
+                           const real3 r = f3(g.p) - xi;  // x_fluid - x_solid, as the fluid computes it
+                           const real3 a = kgrad_r2(r, dot3(r, r), s) * -Vi * (dt * g.k);
+                           const bool on = w_fluid(g.p.w) && fabs(g.k) > s.eps;
+                           return on ? TPush{a.x, a.y, a.z, inv_dt} : TPush{0.f, 0.f, 0.f, 0.f};
+                         },
+                         [&](const TPush& t) { push_fold(ai, t); });
+      if (work && !fluid && sub == 0) {
+        real4 a = d.acc4[i];
+        a.x += ai.x; a.y += ai.y; a.z += ai.z;
+        d.acc4[i] = a;
+      }
     }
   }
 }
+template <int U, int L>
+__global__ void NN_PASS_REGS k_pressure_update(Dev d) { pressure_update_body<U, L>(d); }
 
 // Loop control after each solver iteration: per-scene average error against eta,
 // the reference's iteration counting (SPH/main.py:1695-1703, 1778-1784), and the
@@ -564,16 +640,27 @@ struct GF { real4 p, v; real rho; int id; };  // v.w = mass
 #define FF_VI 2  // explicit viscosity (fluid and boundary) and its reaction on dynamic solids
 #define FF_SR 4  // strain rate and viscosity law
 #define FF_Q 8   // reference quirk mode
-template <int U, int FF>
-__device__ __forceinline__ void forces_body(Dev d, int clear) {
+// A neighbour's contributions, as many words as the instance's terms need: surface tension
+// (x, y, z) * w at ST, viscosity grad W * a at VI, strain rate e[6] * m at SR.
+template <int FF>
+struct TForce {
+  static constexpr int ST = 0, VI = ST + ((FF & FF_ST) ? 4 : 0), SR = VI + ((FF & FF_VI) ? 4 : 0),
+                       N = SR + ((FF & FF_SR) ? 7 : 0);
+  real w[N > 0 ? N : 1];
+};
+template <int U, int L, int FF>
+__device__ __forceinline__ void forces_body(const Dev& d, int clear) {
+  static_assert(!(FF & FF_Q) || L == 1, "quirk mode keeps one lane per particle");
   const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
-    const uint32_t fl = d.w.flags[i];
+  FOR_SPLIT(L, i, sub, valid, n) {
+    const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const bool fluid = cls_fluid(fl);
     const int scn = slot_scene(fl);
     const SceneDev& s = d.sc[scn];
-    if (s.n_fluid == 0) continue;  // the reference runs the substep only with fluid
-    if (d.dyn[scn].np_fresh) continue;  // computed by the divergence loop's last density change
+    // the reference runs the substep only with fluid; np_fresh: computed by the divergence
+    // loop's last density change
+    const bool work = valid && s.n_fluid != 0 && !d.dyn[scn].np_fresh;
+    if (L == 1 ? !work : !__any_sync(0xffffffffu, work)) continue;
     const bool implicit = scene_implicit(s);
     const bool quirks = (FF & FF_Q) && (s.flags & NN_F_QUIRKS);
     const bool st_on = (FF & FF_ST) && fluid && (s.flags & NN_F_SURFACE_TENSION);
@@ -582,60 +669,95 @@ __device__ __forceinline__ void forces_body(Dev d, int clear) {
         (FF & FF_VI) && cls_dyn_solid(fl) && !implicit && (s.flags & NN_F_VISCOSITY) && s.visc_b != 0.f;
     const bool nn_on = (FF & FF_SR) && (s.flags & NN_F_NONNEWTON);
     const bool sr_on = nn_on && (fluid || quirks);
-    const real4 pi = d.w.pos[i];
+    const bool walk = work && (st_on || vi_on || vb_on || sr_on);
+    const int self = work ? i : 0;
+    const real4 pi = d.w.pos[self];
     const real3 xi = f3(pi);
-    const real3 vi = f3(d.w.vel[i]);
+    const real3 vi = f3(d.w.vel[self]);
     real4 a;
     if (clear) a = cls_static_solid(fl) ? make_real4(0.f, 0.f, 0.f, 0.f) : make_real4(s.g[0], s.g[1], s.g[2], 0.f);
-    else a = d.acc4[i];
-    real3 st = make_real3(0.f, 0.f, 0.f), vs = make_real3(0.f, 0.f, 0.f), rf = make_real3(0.f, 0.f, 0.f);
+    else a = d.acc4[self];
+    real3 st = make_real3(0.f, 0.f, 0.f), vs = make_real3(0.f, 0.f, 0.f);
     real S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // strain-rate sum: 00 11 22 01 02 12
     int last_id = -1;                             // quirk: the last neighbour in id order survives
-    if (st_on || vi_on || vb_on || sr_on) {
-      const real mi = d.w.mass[i];
-      const real rho_i = d.w.dens[i];
+    if (L == 1 ? walk : __any_sync(0xffffffffu, walk)) {
+      using T = TForce<FF>;
+      const real mi = d.w.mass[self];
+      const real rho_i = d.w.dens[self];
       const real Vi = fabs(pi.w);
       const bool need_rho = vi_on || vb_on;  // density and id only where a term reads them
-      nb_batches<U>(d.nbr + i, d.cap, d.nbr_cnt[i], i,
-                    [&](int j) {
-                      return GF{pos_of(d, j), ldg(&d.w.vel[j]), need_rho ? ldg(&d.w.dens[j]) : 1.f,
-                                quirks ? ldg(&d.w.id[j]) : 0};
-                    },
-                    [&](int, const GF& g) {
-                      const real3 r = xi - f3(g.p);
-                      const real r2 = dot3(r, r);
-                      real w;
-                      real3 gw;
-                      kwg_r2(r, r2, s, w, gw);
-                      const bool jf = w_fluid(g.p.w);
-                      const real mj = g.v.w;
-                      if (jf && st_on) st -= (r * (s.sigma / mi * mj)) * (r2 > s.dia2 ? w : s.w_dia);
-                      if (vi_on) {
-                        const real v_xy = dot3(vi - f3(g.v), r);
-                        if (jf) vs += gw * (10.f * s.visc * (mj / g.rho) * v_xy / (r2 + s.c01h2));
-                        else if (s.visc_b != 0.f)
-                          vs += gw * (10.f * s.visc_b * (s.rho0 * fabs(g.p.w) / rho_i) * v_xy / (r2 + s.c01h2));
-                      }
-                      if (vb_on && jf) {  // reaction on a dynamic solid: the fluid's term with i <-> j
-                        const real3 rr = -r;
-                        const real v_xy = dot3(f3(g.v) - vi, rr);
-                        rf += (-gw) * (10.f * s.visc_b * (s.rho0 * Vi / g.rho) * v_xy / (r2 + s.c01h2));
-                      }
-                      if (sr_on) {
-                        const real3 vji = f3(g.v) - vi;
-                        const real t[6] = {(vji.x * gw.x + vji.x * gw.x) * mj, (vji.y * gw.y + vji.y * gw.y) * mj,
-                                            (vji.z * gw.z + vji.z * gw.z) * mj, (vji.x * gw.y + vji.y * gw.x) * mj,
-                                            (vji.x * gw.z + vji.z * gw.x) * mj, (vji.y * gw.z + vji.z * gw.y) * mj};
-                        const bool take = g.id > last_id;
-                        if (quirks && take) last_id = g.id;
+      auto load = [&](int j) {
+        return GF{pos_of(d, j), ldg(&d.w.vel[j]), need_rho ? ldg(&d.w.dens[j]) : 1.f, quirks ? ldg(&d.w.id[j]) : 0};
+      };
+      auto term = [&](const GF& g) {
+        T t;
+        const real3 r = xi - f3(g.p);
+        const real r2 = dot3(r, r);
+        real w;
+        real3 gw;
+        kwg_r2(r, r2, s, w, gw);
+        const bool jf = w_fluid(g.p.w);
+        const real mj = g.v.w;
+        if constexpr ((FF & FF_ST) != 0) {
+          const real3 b = r * (s.sigma / mi * mj);
+          t.w[T::ST] = b.x; t.w[T::ST + 1] = b.y; t.w[T::ST + 2] = b.z;
+          t.w[T::ST + 3] = jf && st_on ? (r2 > s.dia2 ? w : s.w_dia) : real(0);
+        }
+        if constexpr ((FF & FF_VI) != 0) {
+          // a dynamic solid takes the reaction of the fluid's term with i <-> j
+          const real v_xy = dot3(vi - f3(g.v), r);
+          real c = 0.f;
+          if (vi_on) {
+            if (jf) c = 10.f * s.visc * (mj / g.rho) * v_xy / (r2 + s.c01h2);
+            else if (s.visc_b != 0.f) c = 10.f * s.visc_b * (s.rho0 * fabs(g.p.w) / rho_i) * v_xy / (r2 + s.c01h2);
+          } else if (vb_on && jf) {
+            c = 10.f * s.visc_b * (s.rho0 * Vi / g.rho) * v_xy / (r2 + s.c01h2);
+          }
+          t.w[T::VI] = gw.x; t.w[T::VI + 1] = gw.y; t.w[T::VI + 2] = gw.z;
+          t.w[T::VI + 3] = c;
+        }
+        if constexpr ((FF & FF_SR) != 0) {
+          real e[6];
+          strain_term(f3(g.v) - vi, gw, e);
+          t.w[T::SR] = mj;
 #pragma unroll
-                        for (int k = 0; k < 6; ++k) S[k] = quirks ? (take ? t[k] : S[k]) : S[k] + t[k];
-                      }
-                    });
+          for (int k = 0; k < 6; ++k) t.w[T::SR + 1 + k] = e[k];
+        }
+        return t;
+      };
+      auto fold = [&](const T& t, int id) {
+        if constexpr ((FF & FF_ST) != 0) {
+          if (st_on) {
+            const real w = t.w[T::ST + 3];
+            st = make_real3(fma(-t.w[T::ST], w, st.x), fma(-t.w[T::ST + 1], w, st.y), fma(-t.w[T::ST + 2], w, st.z));
+          }
+        }
+        if constexpr ((FF & FF_VI) != 0) {
+          const real c = t.w[T::VI + 3];
+          vs = make_real3(fma(t.w[T::VI], c, vs.x), fma(t.w[T::VI + 1], c, vs.y), fma(t.w[T::VI + 2], c, vs.z));
+        }
+        if constexpr ((FF & FF_SR) != 0) {
+          if (sr_on) {
+            const real m = t.w[T::SR];
+            const bool take = id > last_id;
+            if (quirks && take) last_id = id;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+              const real e = t.w[T::SR + 1 + k];
+              S[k] = quirks ? (take ? e * m : S[k]) : fma(e, m, S[k]);
+            }
+          }
+        }
+      };
+      const int c = walk ? d.nbr_cnt[i] : 0;
+      if constexpr ((FF & FF_Q) != 0)
+        nb_batches<U>(d.nbr + i, d.cap, c, self, load, [&](int, const GF& g) { fold(term(g), g.id); });
+      else
+        nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, load, term, [&](const T& t) { fold(t, 0); });
     }
+    if (!work || sub != 0) continue;
     if (st_on) { a.x += st.x; a.y += st.y; a.z += st.z; }
-    if (vi_on) { a.x += vs.x; a.y += vs.y; a.z += vs.z; }
-    if (vb_on) { a.x -= rf.x; a.y -= rf.y; a.z -= rf.z; }
+    if (vi_on || vb_on) { a.x += vs.x; a.y += vs.y; a.z += vs.z; }
     d.acc4[i] = a;
     real mu = s.mu_newton;
     if (nn_on) {
@@ -661,14 +783,15 @@ __device__ __forceinline__ void forces_body(Dev d, int clear) {
 // 0.457 -> 0.404 ms on the 2.4M scene, -21 % on the shear-thinning drop. With it, the
 // spills cost more than the occupancy gains (+8 % on the dam break), so that instance
 // keeps the compiler's own budget (forces_kernel_of picks the wrapper).
-template <int U, int FF>
-__global__ void k_forces(Dev d, int clear) { forces_body<U, FF>(d, clear); }
-template <int U, int FF>
-__global__ void NN_REGS64 k_forces_r64(Dev d, int clear) { forces_body<U, FF>(d, clear); }
-template <int U, int FF>
+template <int U, int L, int FF>
+__global__ void k_forces(Dev d, int clear) { forces_body<U, L, FF>(d, clear); }
+template <int U, int L, int FF>
+__global__ void NN_REGS64 k_forces_r64(Dev d, int clear) { forces_body<U, L, FF>(d, clear); }
+template <int U, int L, int FF>
 constexpr void (*forces_kernel_of())(Dev, int) {
-  if constexpr ((FF & FF_VI) != 0) return &k_forces<U, FF>;
-  else return &k_forces_r64<U, FF>;
+  constexpr int LF = (FF & FF_Q) ? 1 : L;
+  if constexpr ((FF & FF_VI) != 0) return &k_forces<U, LF, FF>;
+  else return &k_forces_r64<U, LF, FF>;
 }
 
 // ---------------------------------------------------------------------------
@@ -692,108 +815,155 @@ __device__ __forceinline__ bool cg_row(const Dev& d, int i, uint32_t fl) {
 // solids, so the matvec reads the same operands in two float4 gathers (32 B per pair)
 // instead of three loads (40 B): the matvec 0.302 -> 0.265 ms on the 2.4M scene.
 struct GCG { real4 p, x; real2 a; };
-template <int U, bool SETUP>
-__device__ __forceinline__ real3 cg_apply(const Dev& d, int i, const real4* __restrict__ vec, real3 vi,
-                                           const SceneDev& s, real dt, real* D, real3* bcorr) {
-  const real3 xi = f3(d.w.pos[i]);
-  const real2 ai = d.cg_aux[i];
-  const real mi = d.w.mass[i];
-  const real rho_i = d.w.dens[i];
+struct TMatvec { real x, y, z, c; };                             // grad W, c
+struct TSetup { real x, y, z, c, b, wx, wy, wz, rx, ry, rz; };   // and b of bcorr, c w grad W, r
+template <int U, int L, bool SETUP>
+__device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool work, const real4* __restrict__ vec,
+                                           real3 vi, const SceneDev& s, real dt, real* D, real3* bcorr) {
+  const int self = work ? i : 0;
+  const real3 xi = f3(d.w.pos[self]);
+  const real2 ai = d.cg_aux[self];
+  const real mi = d.w.mass[self];
+  const real rho_i = d.w.dens[self];
   real3 acc = vi * mi;
   const real cdt = dt * 10.f;
   const real cb = cdt * s.mu_b * mi * s.rho0 / (rho_i * rho_i);
-  nb_batches<U>(d.nbr + i, d.cap, d.nbr_cnt[i], i,
-             [&](int j) {
-               GCG g;
-               if (SETUP) {
-                 g.p = pos_of(d, j);
-                 g.x = ldg(&vec[j]);
-                 g.a = ldg(&d.cg_aux[j]);
-               } else {
-                 g.p = ldg(&d.cg_pos[j]);
-                 g.x = ldg(&vec[j]);
-                 g.a = make_real2(g.x.w, g.p.w);  // fluid j: (mu_j, m_j / rho_j)
-               }
-               return g;
-             },
-             [&](int, const GCG& g) {
-               const real3 r = xi - f3(g.p);
-               const real r2 = dot3(r, r);
-               const real3 gw = kgrad_r2(r, r2, s);
-               const real w = fast_div(1.f, r2 + s.c01h2);
-               real c;
-               real3 diff;
-               if (w_fluid(g.p.w)) {
-                 c = cdt * 0.5f * (ai.x + g.a.x) * ai.y * g.a.y;
-                 diff = vi - f3(g.x);
-               } else {
-                 c = cb * fabs(g.p.w);
-                 diff = vi;
-                 if (SETUP && g.a.y > 0.f) *bcorr -= gw * (c * dot3(r, f3(g.x)) * w);  // dynamic solid
-               }
-               acc -= gw * (c * dot3(r, diff) * w);
-               if (SETUP) {
-                 const real cw = c * w;
-                 D[0] -= cw * gw.x * r.x; D[1] -= cw * gw.y * r.y; D[2] -= cw * gw.z * r.z;
-                 D[3] -= cw * gw.x * r.y; D[4] -= cw * gw.x * r.z; D[5] -= cw * gw.y * r.z;
-               }
-             });
+  const int cnt = work ? d.nbr_cnt[i] : 0;
+  auto add = [&](real3& sum, real3 g, real c) { sum = make_real3(fma(-g.x, c, sum.x), fma(-g.y, c, sum.y), fma(-g.z, c, sum.z)); };
+  if constexpr (SETUP) {
+    auto load = [&](int j) { return GCG{pos_of(d, j), ldg(&vec[j]), ldg(&d.cg_aux[j])}; };
+    auto add_diag = [&](real3 wg, real3 r) {
+      D[0] = fma(-wg.x, r.x, D[0]); D[1] = fma(-wg.y, r.y, D[1]); D[2] = fma(-wg.z, r.z, D[2]);
+      D[3] = fma(-wg.x, r.y, D[3]); D[4] = fma(-wg.x, r.z, D[4]); D[5] = fma(-wg.y, r.z, D[5]);
+    };
+    if constexpr (L == 1) {  // each sum added where its term is made, as in density_change_body
+      nb_batches<U>(d.nbr + i, d.cap, cnt, self, load, [&](int, const GCG& g) {
+        const real3 r = xi - f3(g.p);
+        const real r2 = dot3(r, r);
+        const real3 gw = kgrad_r2(r, r2, s);
+        const real w = fast_div(1.f, r2 + s.c01h2);
+        real c;
+        real3 diff;
+        if (w_fluid(g.p.w)) {
+          c = cdt * 0.5f * (ai.x + g.a.x) * ai.y * g.a.y;
+          diff = vi - f3(g.x);
+        } else {
+          c = cb * fabs(g.p.w);
+          diff = vi;
+          if (g.a.y > 0.f) add(*bcorr, gw, c * dot3(r, f3(g.x)) * w);  // dynamic solid
+        }
+        add(acc, gw, c * dot3(r, diff) * w);
+        const real cw = c * w;
+        add_diag(make_real3(cw * gw.x, cw * gw.y, cw * gw.z), r);
+      });
+    } else {
+      nb_sum<U, L>(d.nbr + i, d.cap, cnt, self, sub, load,
+                   [&](const GCG& g) {
+                     const real3 r = xi - f3(g.p);
+                     const real r2 = dot3(r, r);
+                     const real3 gw = kgrad_r2(r, r2, s);
+                     const real w = fast_div(1.f, r2 + s.c01h2);
+                     const bool jf = w_fluid(g.p.w);
+                     const real c = jf ? cdt * 0.5f * (ai.x + g.a.x) * ai.y * g.a.y : cb * fabs(g.p.w);
+                     const real3 diff = jf ? vi - f3(g.x) : vi;
+                     const real cw = c * w;
+                     TSetup t;
+                     t.x = gw.x; t.y = gw.y; t.z = gw.z;
+                     t.c = c * dot3(r, diff) * w;
+                     t.b = !jf && g.a.y > 0.f ? c * dot3(r, f3(g.x)) * w : real(0);  // dynamic solid
+                     t.wx = cw * gw.x; t.wy = cw * gw.y; t.wz = cw * gw.z;
+                     t.rx = r.x; t.ry = r.y; t.rz = r.z;
+                     return t;
+                   },
+                   [&](const TSetup& t) {
+                     const real3 gw = make_real3(t.x, t.y, t.z);
+                     add(*bcorr, gw, t.b);
+                     add(acc, gw, t.c);
+                     add_diag(make_real3(t.wx, t.wy, t.wz), make_real3(t.rx, t.ry, t.rz));
+                   });
+    }
+  } else {
+    nb_sum<U, L>(d.nbr + i, d.cap, cnt, self, sub,
+                 [&](int j) { return GPV{ldg(&d.cg_pos[j]), ldg(&vec[j])}; },
+                 [&](const GPV& g) {  // fluid j: (mu_j, m_j / rho_j) in v.w, p.w
+                   const real3 r = xi - f3(g.p);
+                   const real r2 = dot3(r, r);
+                   const real3 gw = kgrad_r2(r, r2, s);
+                   const real w = fast_div(1.f, r2 + s.c01h2);
+                   real c;
+                   real3 diff;
+                   if (w_fluid(g.p.w)) {
+                     c = cdt * 0.5f * (ai.x + g.v.w) * ai.y * g.p.w;
+                     diff = vi - f3(g.v);
+                   } else {
+                     c = cb * fabs(g.p.w);
+                     diff = vi;
+                   }
+                   return TMatvec{gw.x, gw.y, gw.z, c * dot3(r, diff) * w};
+                 },
+                 [&](const TMatvec& t) { add(acc, make_real3(t.x, t.y, t.z), t.c); });
+  }
   return acc;
 }
 
 __device__ __forceinline__ real3 sym_apply(const real* P, real3 v) {  // P: 00 11 22 01 02 12
-  return make_real3(P[0] * v.x + P[3] * v.y + P[4] * v.z, P[3] * v.x + P[1] * v.y + P[5] * v.z,
-                     P[4] * v.x + P[5] * v.y + P[2] * v.z);
+  return make_real3(fma(P[4], v.z, fma(P[3], v.y, P[0] * v.x)), fma(P[5], v.z, fma(P[1], v.y, P[3] * v.x)),
+                     fma(P[2], v.z, fma(P[5], v.y, P[4] * v.x)));
 }
 
-// 64 registers (from 72): 8 blocks of 128 per SM instead of 7
-template <int U>
-__global__ void NN_REGS64 k_cg_setup(Dev d) {
+template <int U, int L>
+__device__ __forceinline__ void cg_setup_body(const Dev& d) {
   const int n = d.d_n[0];
-  FOR_SLOTS_WARP(i, valid, n) {
+  FOR_SPLIT(L, i, sub, valid, n) {
     const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const int scn = slot_scene(fl);
     const bool work = valid && cg_row(d, i, fl);
     double rr = 0, bb = 0, rz = 0;
     // a solid neighbour's matvec operands: its pos (x, -V); its p is not read
-    if (valid && cls_solid(fl) && scene_implicit(d.sc[scn])) d.cg_pos[i] = d.w.pos[i];
-    if (work) {
+    if (valid && sub == 0 && cls_solid(fl) && scene_implicit(d.sc[scn])) d.cg_pos[i] = d.w.pos[i];
+    if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
       const SceneDev& s = d.sc[scn];
       const real dt = d.dyn[scn].dt;
-      const real mi = d.w.mass[i];
-      const real3 vi = f3(d.w.vel[i]);
+      const int self = work ? i : 0;
+      const real mi = d.w.mass[self];
+      const real3 vi = f3(d.w.vel[self]);
       real D[6] = {mi, mi, mi, 0.f, 0.f, 0.f};
       real3 bc = make_real3(0.f, 0.f, 0.f);
-      const real3 Av = cg_apply<U, true>(d, i, d.w.vel, vi, s, dt, D, &bc);
-      const real3 b = vi * mi + bc;
-      // symmetric 3x3 inverse in double
-      double a00 = D[0], a11 = D[1], a22 = D[2], a01 = D[3], a02 = D[4], a12 = D[5];
-      double c00 = a11 * a22 - a12 * a12, c01 = a02 * a12 - a01 * a22, c02 = a01 * a12 - a02 * a11;
-      double det = a00 * c00 + a01 * c01 + a02 * c02;
-      double id = 1.0 / det;
-      real P[6] = {(real)(c00 * id), (real)((a00 * a22 - a02 * a02) * id), (real)((a00 * a11 - a01 * a01) * id),
-                    (real)(c01 * id), (real)(c02 * id), (real)((a01 * a02 - a00 * a12) * id)};
+      const real3 Av = cg_apply<U, L, true>(d, i, sub, work, d.w.vel, vi, s, dt, D, &bc);
+      if (work && sub == 0) {
+        const real3 b = vi * mi + bc;
+        // symmetric 3x3 inverse in double
+        double a00 = D[0], a11 = D[1], a22 = D[2], a01 = D[3], a02 = D[4], a12 = D[5];
+        double c00 = a11 * a22 - a12 * a12, c01 = a02 * a12 - a01 * a22, c02 = a01 * a12 - a02 * a11;
+        double det = a00 * c00 + a01 * c01 + a02 * c02;
+        double id = 1.0 / det;
+        real P[6] = {(real)(c00 * id), (real)((a00 * a22 - a02 * a02) * id), (real)((a00 * a11 - a01 * a01) * id),
+                      (real)(c01 * id), (real)(c02 * id), (real)((a01 * a02 - a00 * a12) * id)};
 #pragma unroll
-      for (int k = 0; k < 6; ++k) d.cg_pinv[(size_t)k * d.cap + i] = P[k];
-      const real3 r = b - Av;
-      const real3 z = sym_apply(P, r);
-      d.cg_x[i] = make_real4(vi.x, vi.y, vi.z, 0.f);
-      d.cg_r[i] = make_real4(r.x, r.y, r.z, 0.f);
-      d.cg_z[i] = make_real4(z.x, z.y, z.z, 0.f);
-      const real2 ai = d.cg_aux[i];
-      const real3 xi = f3(d.w.pos[i]);
-      d.cg_pos[i] = make_real4(xi.x, xi.y, xi.z, ai.y);
-      d.cg_p[i] = make_real4(z.x, z.y, z.z, ai.x);
-      rr = (double)r.x * r.x + (double)r.y * r.y + (double)r.z * r.z;
-      bb = (double)b.x * b.x + (double)b.y * b.y + (double)b.z * b.z;
-      rz = (double)r.x * z.x + (double)r.y * z.y + (double)r.z * z.z;
+        for (int k = 0; k < 6; ++k) d.cg_pinv[(size_t)k * d.cap + i] = P[k];
+        const real3 r = b - Av;
+        const real3 z = sym_apply(P, r);
+        d.cg_x[i] = make_real4(vi.x, vi.y, vi.z, 0.f);
+        d.cg_r[i] = make_real4(r.x, r.y, r.z, 0.f);
+        d.cg_z[i] = make_real4(z.x, z.y, z.z, 0.f);
+        const real2 ai = d.cg_aux[i];
+        const real3 xi = f3(d.w.pos[i]);
+        d.cg_pos[i] = make_real4(xi.x, xi.y, xi.z, ai.y);
+        d.cg_p[i] = make_real4(z.x, z.y, z.z, ai.x);
+        rr = (double)r.x * r.x + (double)r.y * r.y + (double)r.z * r.z;
+        bb = (double)b.x * b.x + (double)b.y * b.y + (double)b.z * b.z;
+        rz = (double)r.x * z.x + (double)r.y * z.y + (double)r.z * z.z;
+      }
     }
     // per iteration: partial sums kept across iterations spill under the 64-register cap
-    scene_add(d.acc, ACC_RR, 0, scn, work, rr);
-    scene_add(d.acc, ACC_BB, 0, scn, work, bb);
-    scene_add(d.acc, ACC_RZ, 0, scn, work, rz);
+    scene_add(d.acc, ACC_RR, 0, scn, work && sub == 0, rr);
+    scene_add(d.acc, ACC_BB, 0, scn, work && sub == 0, bb);
+    scene_add(d.acc, ACC_RZ, 0, scn, work && sub == 0, rz);
   }
 }
+// 64 registers (from 72): 8 blocks of 128 per SM instead of 7
+template <int U, int L>
+__global__ void NN_REGS64 k_cg_setup(Dev d) { cg_setup_body<U, L>(d); }
 
 // After setup: relative residual of the initial guess decides whether to iterate.
 __global__ void k_cg_check0(Dev d) {
@@ -823,27 +993,31 @@ __global__ void k_cg_check0(Dev d) {
   }
 }
 
-template <int U>
-__global__ void k_cg_matvec(Dev d) {
+template <int U, int L>
+__device__ __forceinline__ void cg_matvec_body(const Dev& d) {
   const int n = d.d_n[0];
   LaneSums<1> sums;
   const int q[1] = {ACC_PAP};
-  FOR_SLOTS_WARP(i, valid, n) {
+  FOR_SPLIT(L, i, sub, valid, n) {
     const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const int scn = slot_scene(fl);
     const bool work = valid && cg_row(d, i, fl) && d.dyn[scn].act_cg;
     double pap = 0;
-    if (work) {
+    if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
       const SceneDev& s = d.sc[scn];
-      const real3 p = f3(d.cg_p[i]);
-      const real3 Ap = cg_apply<U, false>(d, i, d.cg_p, p, s, d.dyn[scn].dt, nullptr, nullptr);
-      d.cg_Ap[i] = make_real4(Ap.x, Ap.y, Ap.z, 0.f);
-      pap = (double)p.x * Ap.x + (double)p.y * Ap.y + (double)p.z * Ap.z;
+      const real3 p = f3(d.cg_p[work ? i : 0]);
+      const real3 Ap = cg_apply<U, L, false>(d, i, sub, work, d.cg_p, p, s, d.dyn[scn].dt, nullptr, nullptr);
+      if (work && sub == 0) {
+        d.cg_Ap[i] = make_real4(Ap.x, Ap.y, Ap.z, 0.f);
+        pap = (double)p.x * Ap.x + (double)p.y * Ap.y + (double)p.z * Ap.z;
+      }
     }
-    sums.add(d.acc, q, work, scn, {pap});
+    sums.add(d.acc, q, work && sub == 0, scn, {pap});
   }
   sums.flush(d.acc, q);
 }
+template <int U, int L>
+__global__ void NN_REGS64 k_cg_matvec(Dev d) { cg_matvec_body<U, L>(d); }
 
 __global__ void k_cg_update(Dev d) {
   const int n = d.d_n[0];

@@ -1,0 +1,55 @@
+"""The lane split of the neighbour passes (nb_sum): contexts pick 8, 4, 2 or 1 lanes per
+particle by their fluid count, and every split folds a particle's terms in list order, so
+the fields are the one-lane passes' (an explicit unroll) bit for bit: odd sizes on both
+sides of each line of the rule, and every pass (explicit and implicit viscosity, the
+folded non-pressure terms, a rigid body's coupling)."""
+import numpy as np
+import pytest
+import torch
+
+from nonnewton_b200 import scene as S
+from nonnewton_b200 import sph
+from nonnewton_b200.config import SimConfig
+
+pytestmark = pytest.mark.gpu
+FIELDS = ("x", "v", "acceleration", "density", "volume")
+CROSS = dict(extra_cfg={"useNonNewtonianModel": True},
+             fluid_cfg={"nonNewtonMethod": "CROSS_", "viscosity0": 5.0, "viscosity_inf": 0.01, "consistency_index": 1.0,
+                        "power_index": 0.7, "viscosityMethod": 13, "viscoMaxError": 1e-3, "viscosityBoundary": 0.1})
+
+
+def _run(sc, unroll):
+    m = sph.initialize(SimConfig(config=sc.config), particles=sc.particles, quirks=sc.param.quirks,
+                       tuning=dict(unroll=unroll))
+    solver = sph.build_solver()
+    solver.initialize()
+    g = torch.Generator("cuda").manual_seed(1)
+    v = torch.rand(m.pd.v.shape, generator=g, device="cuda") - 0.5
+    m.pd.v.copy_(v * m.pd.is_dynamic[:, None])
+    for _ in range(3):
+        solver.step()
+    assert solver.stats()["status"] == 0
+    nf = sc.particles.n_fluid
+    law = ("strain_rate_norm", "nonnewton_viscosity") if sc.param.use_nonnewtonian else ()  # else not written
+    out = {k: getattr(m.pd, k).clone() for k in FIELDS + law}
+    out.update({k: getattr(m.pd, k)[:nf].clone() for k in ("dfsph_factor", "density_adv")})
+    return out
+
+
+@pytest.mark.parametrize("counts,kind", [((1, 1, 1), {}), ((5, 3, 1), CROSS), ((11, 13, 9), CROSS), ((25, 20, 20), {}),
+                                         ((25, 21, 19), CROSS), ((29, 31, 31), {}), ((39, 37, 31), CROSS),
+                                         ((39, 39, 37), {})])
+def test_sums_do_not_depend_on_the_lanes(cuda_lib, counts, kind):
+    sc = S.dam_break(seed=3, n_side=counts, box=max(counts) * 0.02 + 0.1, **kind)
+    a, b = _run(sc, 0), _run(sc, 1)
+    for k in a:
+        assert np.array_equal(a[k].cpu().numpy(), b[k].cpu().numpy()), k
+
+
+def test_coupled_solids_do_not_depend_on_the_lanes(cuda_lib):
+    sc = S.rigid_drop(seed=2, coupling=2)
+    sc.particles.x[sc.particles.phase_id >= 2000, 1] -= 0.05  # into reach of the fluid
+    sc.config["Configuration"]["boundaryViscosity"] = 0.5
+    a, b = _run(sc, 0), _run(sc, 2)
+    for k in a:
+        assert np.array_equal(a[k].cpu().numpy(), b[k].cpu().numpy()), k
