@@ -367,6 +367,16 @@ static int solver_loop(nn_ctx* c, cudaStream_t s, bool check_first, Pre pre, Bod
   return NN_OK;
 }
 
+// The list build: one cell row per warp while the scene does not fill the chip, else one
+// warp for all rows of its slots (rows / whole, us: 3,933 slots 9 / 36; 23,002 13 / 35;
+// 85,147 40 / 51; 135,201 46 / 44; 900,002 265 / 200; 2,400,002 694 / 470). Both write the
+// same lists.
+#define NN_BUILD_ROWS_MAX 110000
+static int enq_build_lists(nn_ctx* c, cudaStream_t s, const Dev& d) {
+  if (c->n <= NN_BUILD_ROWS_MAX) return launch_lanes(c, s, k_build_lists_rows, NSR_WARPS * 32, c->n, NSR_WARPS, d);
+  return launch(c, s, k_build_lists, NS_WARPS * 32, c->n, d);
+}
+
 // ---- pass sequences ---------------------------------------------------------------
 // NeighborhoodSearchSparse.run_search (SPH/main.py:822-829): the new slots go into the
 // other working set; the source (caller state or previous slots) is a device flag.
@@ -384,7 +394,7 @@ static int enq_search(nn_ctx* c, cudaStream_t s, bool reset_step = false) {
   RC(launch(c, s, k_scatter, B, c->n, d));
   RC(launch(c, s, k_cell_sort, B, (int)std::min<int64_t>(cells, INT32_MAX), d));
   RC(launch(c, s, k_gather, B, c->n, d));
-  RC(launch(c, s, k_build_lists, NS_WARPS * 32, c->n, d));
+  RC(enq_build_lists(c, s, d));
   c->searched = true;
   return NN_OK;
 }
@@ -1173,7 +1183,7 @@ int nn_time_kernel(nn_ctx* c, int32_t kernel, int32_t reps, float* ms_out) {
       case NN_K_DENSITY_FACTOR:  // the instance the step runs (with the first density change)
         return c->any_div ? launch_nb(c, s, KU2(k_density_factor, true, U_DENSITY_FACTOR), B, d, 1, 1)
                           : launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), B, d, 1, 1);
-      case NN_K_BUILD_LISTS: return launch(c, s, k_build_lists, NS_WARPS * 32, c->n, d);
+      case NN_K_BUILD_LISTS: return enq_build_lists(c, s, d);
       case NN_K_CG_MATVEC: return launch_nb(c, s, KU(k_cg_matvec, U_CG_MATVEC), B, d);
       case NN_K_CG_SETUP: return launch_nb(c, s, KU(k_cg_setup, U_CG_SETUP), B, d);
       default: return launch_nb(c, s, forces_kernel(c), B, d, 0);
@@ -1484,7 +1494,7 @@ extern "C" int nn_neighbors_noalloc(const float* x, int32_t n, const double* dom
   k_scatter<<<gN, B, 0, st>>>(d);
   k_cell_sort<<<gC, B, 0, st>>>(d);
   k_na_gather<<<gN, B, 0, st>>>(d);
-  k_build_lists<<<gN, NS_WARPS * 32, 0, st>>>(d);
+  k_build_lists_rows<<<std::min((n + 31) / 32, 1024), NSR_WARPS * 32, 0, st>>>(d);
   k_export_neighbors<<<gN, B, 0, st>>>(d, num_neighbors, neighbors, width);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(c, NN_ERR_CUDA, "nn_neighbors_noalloc: %s", cudaGetErrorString(e));

@@ -53,3 +53,40 @@ def test_coupled_solids_do_not_depend_on_the_lanes(cuda_lib):
     a, b = _run(sc, 0), _run(sc, 2)
     for k in a:
         assert np.array_equal(a[k].cpu().numpy(), b[k].cpu().numpy()), k
+
+
+@pytest.mark.parametrize("seed,counts,max_nb", [(1, (1, 1, 1), 64), (2, (3, 5, 7), 64), (3, (13, 13, 13), 64),
+                                                (4, (17, 9, 31), 40)])
+@pytest.mark.parametrize("cell_factor", [1, 2])
+def test_list_build_per_row(cuda_lib, seed, counts, max_nb, cell_factor):
+    """Small scenes build their lists one cell row per warp: against brute force, in a
+    scene with ragged warps and a crowded cell (windows past the hit mask), under both
+    stencils; a too small capacity reports the overflow with the true count."""
+    from nonnewton_b200 import _abi
+
+    sc = S.dam_break(seed=seed, n_side=counts, box=max(counts) * 0.02 + 0.04)
+    x = sc.particles.x
+    crowd = min(90, len(x) // 8)
+    x[:crowd] = x[0] + np.random.default_rng(seed).uniform(0, 0.015, (crowd, 3)).astype(np.float32)
+    m = sph.initialize(SimConfig(config=sc.config), particles=sc.particles, max_neighbors=256,
+                       tuning=dict(cell_factor=cell_factor))
+    m.ns.run_search()
+    width = 200
+    num, lists = m.engine.neighbors(len(x), width)
+    xt = m.pd.x
+    r = xt[:, None] - xt[None]
+    d = (r[..., 0] * r[..., 0] + r[..., 1] * r[..., 1] + r[..., 2] * r[..., 2]).sqrt()
+    near = (d < torch.tensor(sc.param.support_radius, dtype=torch.float32, device="cuda"))
+    near.fill_diagonal_(False)
+    want = torch.full((len(x), width), -1, dtype=torch.int32, device="cuda")
+    i, j = near.nonzero(as_tuple=True)
+    want[i, torch.arange(len(i), device="cuda") - (near.sum(1).cumsum(0) - near.sum(1))[i]] = j.int()
+    assert torch.equal(num, near.sum(1).int()) and torch.equal(lists, want)
+    # narrower rows keep the smallest ids
+    _, cut = m.engine.neighbors(len(x), 7)
+    assert torch.equal(cut, want[:, :7])
+    if int(num.max()) > max_nb:
+        m.engine.set_neighbor_cap(max_nb)
+        m.engine.run_pass(_abi.NN_PASS_SEARCH)
+        st = m.engine.stats(0)
+        assert st["status"] == _abi.NN_ERR_NEIGHBOR_OVERFLOW and st["max_neighbors_seen"] == int(num.max())
