@@ -1210,7 +1210,7 @@ int nn_get_neighbors(nn_ctx* c, int32_t* num, int32_t* lists, int32_t width) {
   if (!num || !lists || width <= 0) return fail(c, NN_ERR_INVALID_ARG, "nn_get_neighbors: bad arguments");
   if (!c->searched) return fail(c, NN_ERR_STATE, "run the neighbour search first");
   cudaStream_t s = run_stream(c);
-  RC(launch(c, s, k_export_neighbors, 256, c->n, make_dev(c, c->cur), num, lists, width));
+  RC(launch_lanes(c, s, k_export_neighbors, NS_EXPORT_WARPS * 32, c->n, 32, make_dev(c, c->cur), num, lists, width));
   CK(cudaStreamSynchronize(s));
   return NN_OK;
 }
@@ -1495,7 +1495,8 @@ extern "C" int nn_neighbors_noalloc(const float* x, int32_t n, const double* dom
   k_cell_sort<<<gC, B, 0, st>>>(d);
   k_na_gather<<<gN, B, 0, st>>>(d);
   k_build_lists_rows<<<std::min((n + 31) / 32, 1024), NSR_WARPS * 32, 0, st>>>(d);
-  k_export_neighbors<<<gN, B, 0, st>>>(d, num_neighbors, neighbors, width);
+  const int gE = std::min((n + NS_EXPORT_WARPS - 1) / NS_EXPORT_WARPS, 1024);
+  k_export_neighbors<<<gE, NS_EXPORT_WARPS * 32, 0, st>>>(d, num_neighbors, neighbors, width);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(c, NN_ERR_CUDA, "nn_neighbors_noalloc: %s", cudaGetErrorString(e));
   return NN_OK;

@@ -620,31 +620,36 @@ __global__ void __launch_bounds__(NSR_WARPS * 32) k_build_lists_rows(Dev d) {
 
 // meta.ns.num_neighbors / neighbors in particle-id space, rows sorted by id
 // (materialised on demand for parity checks and the elastic rest state). `num` gets
-// the stored count, or the full count where the search kept it (nbr_raw).
-__global__ void k_export_neighbors(Dev d, int32_t* num, int32_t* lists, int width) {
+// the stored count, or the full count where the search kept it (nbr_raw); of more than
+// `width` neighbours the smallest ids are kept.
+//
+// One warp per slot: the ids of the list go to shared memory 32 at a time, every lane
+// ranks its own by counting the smaller ones (ids are distinct) and writes them in place,
+// so that a row leaves in one or two coalesced stores. One thread per slot with an
+// insertion sort in the output row took 148 us on 135,201 particles (a dependent global
+// load and store per move).
+#define NS_EXPORT_WARPS 8
+#define NS_EXPORT_MAX 1024  // the largest neighbour capacity (nn_ctx_create, nn_set_neighbor_cap)
+__global__ void __launch_bounds__(NS_EXPORT_WARPS * 32) k_export_neighbors(Dev d, int32_t* num, int32_t* lists, int width) {
+  __shared__ int32_t ids_all[NS_EXPORT_WARPS][NS_EXPORT_MAX];
+  int32_t* ids = ids_all[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
     const int id = d.w.id[i];
-    const int c = d.nbr_cnt[i];
+    const int c = min(d.nbr_cnt[i], NS_EXPORT_MAX);
     int32_t* row = lists + (size_t)id * width;
-    int w = min(c, width);
-    // insertion sort of the neighbour ids into the output row
-    for (int k = 0; k < w; ++k) {
-      int v = d.w.id[d.nbr[(size_t)k * d.cap + i]];
-      int p = k;
-      while (p > 0 && row[p - 1] > v) { row[p] = row[p - 1]; --p; }
-      row[p] = v;
+    for (int k = lane; k < c; k += 32) ids[k] = d.w.id[d.nbr[(size_t)k * d.cap + i]];
+    __syncwarp();
+    for (int k = lane; k < c; k += 32) {
+      const int v = ids[k];
+      int rank = 0;
+      for (int q = 0; q < c; ++q) rank += ids[q] < v;
+      if (rank < width) row[rank] = v;
     }
-    if (c > width) {  // keep the `width` smallest ids
-      for (int k = width; k < c; ++k) {
-        int v = d.w.id[d.nbr[(size_t)k * d.cap + i]];
-        if (v >= row[width - 1]) continue;
-        int p = width - 1;
-        while (p > 0 && row[p - 1] > v) { row[p] = row[p - 1]; --p; }
-        row[p] = v;
-      }
-    }
-    for (int k = w; k < width; ++k) row[k] = -1;
-    num[id] = d.nbr_raw ? d.nbr_raw[i] : c;
+    for (int k = c + lane; k < width; k += 32) row[k] = -1;
+    if (lane == 0) num[id] = d.nbr_raw ? d.nbr_raw[i] : c;
+    __syncwarp();
   }
 }

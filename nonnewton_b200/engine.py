@@ -182,8 +182,11 @@ class Engine:
         self._rc(self.L.nn_run_pass(self.h, int(p)))
 
     def neighbors(self, n: int, width: int = 60):
-        num = torch.zeros(n, dtype=torch.int32, device=self.device)
-        lists = torch.full((n, width), -1, dtype=torch.int32, device=self.device)
+        whole = self._state is not None and n == self._state.n  # every row is then written
+        num = (torch.empty if whole else torch.zeros)(n, dtype=torch.int32, device=self.device)
+        lists = torch.empty((n, width), dtype=torch.int32, device=self.device)
+        if not whole:
+            lists.fill_(-1)
         self._rc(self.L.nn_get_neighbors(self.h, _ptr(num), _ptr(lists), int(width)))
         return num, lists
 
