@@ -272,12 +272,58 @@ __device__ __forceinline__ void sr_range_particles(const SrDev& s, int cx, int c
   }
 }
 
-// One warp per particle: lanes split the particles of the range and the moments are
-// reduced across the warp with shuffles.
-__global__ void k_sr_aniso_pre(SrDev s) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < s.n; i += warps) {
+// A block takes 8 * ppw particles: its warps gather the moments of ppw particles each
+// (lanes split the particles of the range, the sums are reduced with shuffles), then one
+// thread per particle does the rest, the FP64 eigen-decomposition above all. On lane 0 of
+// the particle's warp that tail was a third of the kernel's issue slots with one lane of 32
+// active (20.9 threads per instruction). ppw grows to SR_PRE_PPW with the particles, so
+// that a small set still spreads over the chip (sr_pre_ppw).
+#define SR_PRE_PPW 8
+#define SR_PRE_WARPS 8
+struct SrMoments { double tw, m1[3], m2[6]; int nnb; };
+
+__device__ __forceinline__ void sr_aniso_kernel_of(const SrDev& s, int i, const SrMoments& a) {
+  const float px = s.pos[3 * i], py = s.pos[3 * i + 1], pz = s.pos[3 * i + 2];
+  const double tw = a.tw;
+  const double *m1 = a.m1, *m2 = a.m2;
+  double db[3] = {0.0, 0.0, 0.0}, C[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+  if (tw != 0.0) {
+    db[0] = m1[0] / tw; db[1] = m1[1] / tw; db[2] = m1[2] / tw;
+    C[0][0] = m2[0] / tw - db[0] * db[0]; C[1][1] = m2[1] / tw - db[1] * db[1]; C[2][2] = m2[2] / tw - db[2] * db[2];
+    C[0][1] = C[1][0] = m2[3] / tw - db[0] * db[1];
+    C[0][2] = C[2][0] = m2[4] / tw - db[0] * db[2];
+    C[1][2] = C[2][1] = m2[5] / tw - db[1] * db[2];
+  }
+  const double xw[3] = {tw != 0.0 ? px + db[0] : 0.0, tw != 0.0 ? py + db[1] : 0.0, tw != 0.0 ? pz + db[2] : 0.0};
+  const double lam_ = 0.9;  // akLambda
+  s.xbar[3 * i] = (float)((1 - lam_) * px + lam_ * xw[0]);
+  s.xbar[3 * i + 1] = (float)((1 - lam_) * py + lam_ * xw[1]);
+  s.xbar[3 * i + 2] = (float)((1 - lam_) * pz + lam_ * xw[2]);
+  double lam[3], V[3][3];
+  sr_sym_eig(C, lam, V);
+  double sg[3] = {lam[0], lam[1], lam[2]};
+  if (a.nnb > 25) {  // Nvep, kr = 4, ks = 1400 (srtool.py:910-914, 1072-1079)
+    sg[1] = fmax(sg[1], sg[0] / 4.0);
+    sg[2] = fmax(sg[2], sg[0] / 4.0);
+    sg[0] *= 1400.0; sg[1] *= 1400.0; sg[2] *= 1400.0;
+  } else {
+    sg[0] = sg[1] = sg[2] = 0.5;  // kn
+  }
+#pragma unroll
+  for (int a_ = 0; a_ < 3; ++a_)
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const double m = V[a_][0] * V[b][0] / sg[0] + V[a_][1] * V[b][1] / sg[1] + V[a_][2] * V[b][2] / sg[2];
+      s.G[9 * i + 3 * a_ + b] = (float)(tw != 0.0 ? m / (double)s.sr : (a_ == b ? 1.0 : 0.0));
+    }
+}
+
+__global__ void __launch_bounds__(SR_PRE_WARPS * 32) k_sr_aniso_pre(SrDev s, int ppw) {
+  __shared__ SrMoments mom[SR_PRE_WARPS * SR_PRE_PPW];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int per = SR_PRE_WARPS * ppw, base = blockIdx.x * per;
+  for (int k = w; k < per && base + k < s.n; k += SR_PRE_WARPS) {
+    const int i = base + k;
     if (i == 0) continue;  // the reference's loop starts at 1 (srtool.py:1013)
     const float px = s.pos[3 * i], py = s.pos[3 * i + 1], pz = s.pos[3 * i + 2];
     int cx, cy, cz;
@@ -289,8 +335,8 @@ __global__ void k_sr_aniso_pre(SrDev s) {
     double tw = 0.0, m1[3] = {0.0, 0.0, 0.0}, m2[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     int nnb = 0;
     // a margin of one voxel on the pruning distance keeps every pair with w > 0
-    sr_range_particles(s, cx, cy, cz, px, py, pz, rr + s.g.vs, lane, [&](uint32_t k) {
-      const float4 pj = s.spos[k];
+    sr_range_particles(s, cx, cy, cz, px, py, pz, rr + s.g.vs, lane, [&](uint32_t q_) {
+      const float4 pj = s.spos[q_];
       const float dx = __fsub_rn(px, pj.x), dy = __fsub_rn(py, pj.y), dz = __fsub_rn(pz, pj.z);
       const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
       // |x_i - x_j| in f32 (unfused, as any f32 evaluation of it) < 2 r_s, decided on
@@ -298,14 +344,14 @@ __global__ void k_sr_aniso_pre(SrDev s) {
       if (d2 < s.rr_thr) {
         const float dn = __fsqrt_rn(d2);
         const float q = dn / rr;
-        const double w = 1.0 - (double)(q * q * q);  // isoweight, srtool.py:993-999
+        const double w_ = 1.0 - (double)(q * q * q);  // isoweight, srtool.py:993-999
         const double d[3] = {(double)pj.x - px, (double)pj.y - py, (double)pj.z - pz};
-        tw += w;
-        m1[0] += w * d[0]; m1[1] += w * d[1]; m1[2] += w * d[2];
-        if (w > 0) {
+        tw += w_;
+        m1[0] += w_ * d[0]; m1[1] += w_ * d[1]; m1[2] += w_ * d[2];
+        if (w_ > 0) {
           ++nnb;
-          m2[0] += w * d[0] * d[0]; m2[1] += w * d[1] * d[1]; m2[2] += w * d[2] * d[2];
-          m2[3] += w * d[0] * d[1]; m2[4] += w * d[0] * d[2]; m2[5] += w * d[1] * d[2];
+          m2[0] += w_ * d[0] * d[0]; m2[1] += w_ * d[1] * d[1]; m2[2] += w_ * d[2] * d[2];
+          m2[3] += w_ * d[0] * d[1]; m2[4] += w_ * d[0] * d[2]; m2[5] += w_ * d[1] * d[2];
         }
       }
     });
@@ -313,44 +359,27 @@ __global__ void k_sr_aniso_pre(SrDev s) {
     for (int o = 16; o > 0; o >>= 1) {
       tw += __shfl_xor_sync(0xffffffffu, tw, o);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) m1[k] += __shfl_xor_sync(0xffffffffu, m1[k], o);
+      for (int q = 0; q < 3; ++q) m1[q] += __shfl_xor_sync(0xffffffffu, m1[q], o);
 #pragma unroll
-      for (int k = 0; k < 6; ++k) m2[k] += __shfl_xor_sync(0xffffffffu, m2[k], o);
+      for (int q = 0; q < 6; ++q) m2[q] += __shfl_xor_sync(0xffffffffu, m2[q], o);
       nnb += __shfl_xor_sync(0xffffffffu, nnb, o);
     }
-    if (lane != 0) continue;
-    double db[3] = {0.0, 0.0, 0.0}, C[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    if (tw != 0.0) {
-      db[0] = m1[0] / tw; db[1] = m1[1] / tw; db[2] = m1[2] / tw;
-      C[0][0] = m2[0] / tw - db[0] * db[0]; C[1][1] = m2[1] / tw - db[1] * db[1]; C[2][2] = m2[2] / tw - db[2] * db[2];
-      C[0][1] = C[1][0] = m2[3] / tw - db[0] * db[1];
-      C[0][2] = C[2][0] = m2[4] / tw - db[0] * db[2];
-      C[1][2] = C[2][1] = m2[5] / tw - db[1] * db[2];
-    }
-    const double xw[3] = {tw != 0.0 ? px + db[0] : 0.0, tw != 0.0 ? py + db[1] : 0.0, tw != 0.0 ? pz + db[2] : 0.0};
-    const double lam_ = 0.9;  // akLambda
-    s.xbar[3 * i] = (float)((1 - lam_) * px + lam_ * xw[0]);
-    s.xbar[3 * i + 1] = (float)((1 - lam_) * py + lam_ * xw[1]);
-    s.xbar[3 * i + 2] = (float)((1 - lam_) * pz + lam_ * xw[2]);
-    double lam[3], V[3][3];
-    sr_sym_eig(C, lam, V);
-    double sg[3] = {lam[0], lam[1], lam[2]};
-    if (nnb > 25) {  // Nvep, kr = 4, ks = 1400 (srtool.py:910-914, 1072-1079)
-      sg[1] = fmax(sg[1], sg[0] / 4.0);
-      sg[2] = fmax(sg[2], sg[0] / 4.0);
-      sg[0] *= 1400.0; sg[1] *= 1400.0; sg[2] *= 1400.0;
-    } else {
-      sg[0] = sg[1] = sg[2] = 0.5;  // kn
-    }
+    if (lane == 0) {
+      SrMoments& a = mom[k];
+      a.tw = tw;
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+      for (int q = 0; q < 3; ++q) a.m1[q] = m1[q];
 #pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        const double m = V[a][0] * V[b][0] / sg[0] + V[a][1] * V[b][1] / sg[1] + V[a][2] * V[b][2] / sg[2];
-        s.G[9 * i + 3 * a + b] = (float)(tw != 0.0 ? m / (double)s.sr : (a == b ? 1.0 : 0.0));
-      }
+      for (int q = 0; q < 6; ++q) a.m2[q] = m2[q];
+      a.nnb = nnb;
+    }
   }
+  __syncthreads();
+  const int k = (int)threadIdx.x;
+  if (k < per && base + k < s.n && base + k != 0) sr_aniso_kernel_of(s, base + k, mom[k]);
 }
+// Particles per warp of the pre-pass: one until every SM has two blocks' worth.
+static int sr_pre_ppw(int n, int sms) { return std::min(std::max(n / (SR_PRE_WARPS * 2 * sms), 1), SR_PRE_PPW); }
 
 // ---- 4. anisotropic splat (generate_smooth_fluid_field_impl) -------------------------
 // One warp per particle; each lane owns (x, y) columns of the kernel's support box and
@@ -1180,7 +1209,8 @@ static int sr_run(nn_sr_ctx* c, const nn_sr_params* p, const float* pos, const f
     if (p->use_smooth_field) {
       // 3-4. anisotropic kernels and splat (one warp per particle each)
       const int grid_w = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * 32 + B - 1) / B, c->sms * 16));
-      k_sr_aniso_pre<<<grid_w, B, 0, st>>>(s);
+      const int ppw = sr_pre_ppw(n, c->sms), per = SR_PRE_WARPS * ppw;
+      k_sr_aniso_pre<<<(n + per - 1) / per, SR_PRE_WARPS * 32, 0, st>>>(s, ppw);
       k_sr_aniso_splat<<<grid_w, B, 0, st>>>(s);
       if (vel) k_sr_vel_splat<<<grid_w, B, 0, st>>>(s);
     }
