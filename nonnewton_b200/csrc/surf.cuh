@@ -57,6 +57,8 @@ struct SrGrid {
   }
 };
 
+struct SrResult { uint32_t nv, ni; int32_t status, pad; double sd; };  // what the host reads back
+
 struct SrDev {
   SrGrid g;
   int n;
@@ -75,6 +77,8 @@ struct SrDev {
   float* G;                 // [n,9]
   float* xbar;              // [n,3]
   double* stats;            // sum, count, var, sd
+  int32_t* scan_n;          // [2]: last index of the next scan
+  SrResult* result;
   uint32_t* vflag;          // [cells+1] crossing-cube flags, then vertex ids
   uint32_t* tcount;         // [cells+1] index counts, then offsets
   uint32_t* cube_of;        // [max_v] cube (linear index) of each vertex id
@@ -98,6 +102,20 @@ __constant__ int8_t c_sr_off[8][3] = {{0, 1, 0}, {1, 1, 0}, {1, 0, 0}, {0, 0, 0}
 __constant__ int8_t c_sr_edge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, {5, 6},
                                         {6, 7}, {7, 4}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
 
+// The dense passes walk the vertices by rows of one block: a warp takes the 32 x-neighbours
+// (x, y, z) of a block's row, so coordinates cost three 32-bit divisions per warp instead of
+// three 64-bit ones per vertex, and the block's activity (`act`) is uniform in the warp.
+#define FOR_SR_ROWS(s, x, y, z, c, act)                                                                  \
+  for (uint32_t _w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5,                                       \
+                _bx = (uint32_t)(s).g.bx, _rows = _bx * (uint32_t)(s).g.ny * (uint32_t)(s).g.nz;         \
+       _w < _rows; _w += (gridDim.x * blockDim.x) >> 5)                                                  \
+    for (int x = (int)(_w % _bx) * NN_SR_BLOCK + (int)(threadIdx.x & 31), _r = (int)(_w / _bx),          \
+             y = _r % (s).g.ny, z = _r / (s).g.ny, _once = 1;                                            \
+         _once; _once = 0)                                                                               \
+      if (const int64_t c = (s).g.idx(x, y, z); x < (s).g.nx)                                            \
+        for (bool act = (s).active[(s).g.bidx(x, y, z)]; _once; _once = 0)
+static_assert(NN_SR_BLOCK == 32, "a warp covers a block's row");
+
 __device__ __forceinline__ void sr_fail(const SrDev& s, int code) { atomicCAS(s.status, 0, code); }
 
 __device__ __forceinline__ void sr_add(const SrDev& s, int64_t c, double val) {
@@ -107,7 +125,8 @@ __device__ __forceinline__ void sr_add(const SrDev& s, int64_t c, double val) {
 }
 
 // ---- 1. voxel binning --------------------------------------------------------------
-__global__ void k_sr_keys(SrDev s) {
+__global__ void k_sr_keys(SrDev s, int32_t cells) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.scan_n[2] = cells;
   GRID_STRIDE(i, s.n) {
     int x, y, z;
     s.g.voxel_of(s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2], x, y, z);
@@ -376,7 +395,14 @@ __global__ void __launch_bounds__(SR_PRE_WARPS * 32) k_sr_aniso_pre(SrDev s, int
   }
   __syncthreads();
   const int k = (int)threadIdx.x;
-  if (k < per && base + k < s.n && base + k != 0) sr_aniso_kernel_of(s, base + k, mom[k]);
+  if (k < per && base + k < s.n) {
+    if (base + k != 0) {
+      sr_aniso_kernel_of(s, base + k, mom[k]);
+    } else {
+      for (int q = 0; q < 9; ++q) s.G[q] = 0.f;
+      for (int q = 0; q < 3; ++q) s.xbar[q] = 0.f;
+    }
+  }
 }
 // Particles per warp of the pre-pass: one until every SM has two blocks' worth.
 static int sr_pre_ppw(int n, int sms) { return std::min(std::max(n / (SR_PRE_WARPS * 2 * sms), 1), SR_PRE_PPW); }
@@ -650,45 +676,61 @@ __global__ void k_sr_mesh_velocity(SrDev s, int nv) {
   }
 }
 
-__global__ void k_sr_fix_to_field(SrDev s, int64_t cells) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < cells; c += (int64_t)gridDim.x * blockDim.x) {
-    const float v = (float)((double)(long long)s.fix[c] / SR_FIX);
-    s.splat[c] = v;
-    s.field[c] = v;
+// Sum of two values over the block into dst[0] and dst[1]: one atomic each per block (one
+// per warp, on the same two addresses, took 49 us on a 3 M vertex grid).
+__device__ __forceinline__ void sr_block_add(double a, double b, double* dst, bool second) {
+  __shared__ double sh[2][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if (lane == 0) { sh[0][w] = a; sh[1][w] = b; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a = b = 0.0;
+    for (int k = 0; k < nw; ++k) { a += sh[0][k]; b += sh[1][k]; }
+    if (a != 0.0) atomicAdd(&dst[0], a);
+    if (second && b != 0.0) atomicAdd(&dst[1], b);
   }
 }
 
-// ---- 5. smoothing (smooth_sdf) --------------------------------------------------------
-__device__ __forceinline__ bool sr_act(const SrDev& s, int x, int y, int z) {
-  return s.g.in(x, y, z) && s.active[s.g.bidx(x, y, z)];
+// The splat field in floats, and the first pass of the smoothing's statistics over it (the
+// sum and count of its negative values; only active blocks hold any).
+__global__ void k_sr_fix_to_field(SrDev s, int32_t cells) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.scan_n[2] = cells;
+  double a = 0.0, b = 0.0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
+    const float v = (float)((double)(long long)s.fix[c] / SR_FIX);
+    s.splat[c] = v;
+    s.field[c] = v;
+    if (v < 0.f) { a += v; b += 1.0; }
+  }
+  sr_block_add(a, b, &s.stats[0], true);
 }
+
+// ---- 5. smoothing (smooth_sdf) --------------------------------------------------------
+// A field's value at a vertex, 0 outside the grid. Vertices of inactive blocks hold 0: no
+// splat reaches them and the smoothing writes 0 there.
 __device__ __forceinline__ float sr_get(const SrDev& s, const float* f, int x, int y, int z) {
-  return sr_act(s, x, y, z) ? f[s.g.idx(x, y, z)] : 0.f;
+  return s.g.in(x, y, z) ? f[s.g.idx(x, y, z)] : 0.f;
 }
 
 // density_field_stats (srtool.py:1436-1456): pass 0 sums the negative values of the
 // active vertices and counts them, pass 1 their squared deviations from the mean
-__global__ void k_sr_stats(SrDev s, int64_t cells, int pass) {
+__global__ void k_sr_stats(SrDev s, int pass) {
   double a = 0.0, b = 0.0;
   const double mean = pass ? s.stats[0] / s.stats[1] : 0.0;
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < cells; c += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(c % s.g.nx), y = (int)((c / s.g.nx) % s.g.ny), z = (int)(c / ((int64_t)s.g.nx * s.g.ny));
-    if (!s.active[s.g.bidx(x, y, z)]) continue;
+  FOR_SR_ROWS(s, x, y, z, c, act) {
+    if (!act) continue;
     const float v = s.field[c];
     if (v < 0.f) {
       if (pass == 0) { a += v; b += 1.0; }
       else { const double d = v - mean; a += d * d; }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (pass == 0) { atomicAdd(&s.stats[0], a); atomicAdd(&s.stats[1], b); }
-    else atomicAdd(&s.stats[2], a);
-  }
+  sr_block_add(a, b, &s.stats[pass ? 2 : 0], pass == 0);
 }
 __global__ void k_sr_sd(SrDev s) {
   // 0/0 = NaN without negative values, as in the reference (the smoothing then
@@ -696,24 +738,36 @@ __global__ void k_sr_sd(SrDev s) {
   if (threadIdx.x == 0) s.stats[3] = sqrt(s.stats[2] / s.stats[1]);
 }
 
-__global__ void k_sr_smooth(SrDev s, int64_t cells) {
+// Equal values, above all the zeros around the splats, take the weight of a zero difference,
+// computed once; the others the exponential and the division.
+template <int RT>
+__global__ void k_sr_smooth(SrDev s) {
   const float sd = (float)s.stats[3];
   const float inv2s2 = 1.f / (2.f * sd * sd);
   const float norm = powf(2.f * (float)SR_PI * sd * sd, 1.5f);
-  const int R = s.smooth_cells;
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < cells; c += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(c % s.g.nx), y = (int)((c / s.g.nx) % s.g.ny), z = (int)(c / ((int64_t)s.g.nx * s.g.ny));
-    if (!s.active[s.g.bidx(x, y, z)]) { s.tmp[c] = 0.f; continue; }
+  auto gauss = [&](float diff) { return expf(-diff * diff * inv2s2) / norm; };  // gaussian_blur, srtool.py:1432-1434
+  const float g0 = gauss(0.f);
+  const int R = RT ? RT : s.smooth_cells;
+  const int64_t sy = s.g.nx, sz = (int64_t)s.g.nx * s.g.ny;
+  FOR_SR_ROWS(s, x, y, z, c, act) {
+    if (!act) { s.tmp[c] = 0.f; continue; }
     const float v0 = s.field[c];
     float avg = 0.f, wsum = 0.f;
+    const bool inside = x >= R && y >= R && z >= R && x + R < s.g.nx && y + R < s.g.ny && z + R < s.g.nz;
     for (int dz = -R; dz <= R; ++dz)
       for (int dy = -R; dy <= R; ++dy)
+#pragma unroll
         for (int dx = -R; dx <= R; ++dx) {
-          const int a = x + dx, b = y + dy, e = z + dz;
-          if (a < 0 || b < 0 || e < 0) continue;
-          const float vv = sr_get(s, s.field, a, b, e);
+          float vv;
+          if (inside) {
+            vv = s.field[c + dx + dy * sy + dz * sz];
+          } else {
+            const int a = x + dx, b = y + dy, e = z + dz;
+            if (a < 0 || b < 0 || e < 0) continue;
+            vv = sr_get(s, s.field, a, b, e);
+          }
           const float diff = fabsf(v0 - vv);
-          const float gw = expf(-diff * diff * inv2s2) / norm;  // gaussian_blur, srtool.py:1432-1434
+          const float gw = diff == 0.f ? g0 : gauss(diff);
           avg += gw * vv;
           wsum += gw;
         }
@@ -734,11 +788,11 @@ __device__ __forceinline__ bool sr_edge_cross(int ci, int w) {
   return ((ci >> c_sr_edge[w][0]) ^ (ci >> c_sr_edge[w][1])) & 1;
 }
 
-__global__ void k_sr_dc_flag(SrDev s, int64_t cells) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < cells; c += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(c % s.g.nx), y = (int)((c / s.g.nx) % s.g.ny), z = (int)(c / ((int64_t)s.g.nx * s.g.ny));
+__global__ void k_sr_dc_flag(SrDev s, int32_t cells) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.vflag[cells] = 0u;
+  FOR_SR_ROWS(s, x, y, z, c, act) {
     uint32_t f = 0u;
-    if (s.active[s.g.bidx(x, y, z)]) {
+    if (act) {
       const int ci = sr_cube_mask(s, x, y, z);
       f = (ci != 0 && ci != 255) ? 1u : 0u;
     }
@@ -776,8 +830,8 @@ __device__ void sr_normal_at(const SrDev& s, const double p[3], double n[3]) {
 }
 
 // The crossing cubes in vertex-id order, so that the QEF kernel runs on dense work.
-__global__ void k_sr_dc_list(SrDev s, int64_t cells) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < cells; c += (int64_t)gridDim.x * blockDim.x) {
+__global__ void k_sr_dc_list(SrDev s, int32_t cells) {
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
     const uint32_t id = s.vflag[c];
     if (s.vflag[c + 1] != id && (int64_t)id < s.max_v) s.cube_of[id] = (uint32_t)c;
   }
@@ -850,40 +904,49 @@ __device__ __forceinline__ int64_t sr_vid(const SrDev& s, int x, int y, int z) {
   return s.vflag[c + 1] != s.vflag[c] ? (int64_t)s.vflag[c] : -1;
 }
 
-// pass 0 counts the indices each cube emits, pass 1 writes them at the scanned offsets
+// pass 0 counts the indices each crossing cube emits (into tcount, by vertex id, which
+// follows the cube order), pass 1 writes them at the scanned offsets
 __global__ void k_sr_tris(SrDev s, int64_t cells, int pass) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < cells; c += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(c % s.g.nx), y = (int)((c / s.g.nx) % s.g.ny), z = (int)(c / ((int64_t)s.g.nx * s.g.ny));
+  const int nv = (int)min((int64_t)s.vflag[cells], (int64_t)s.max_v);
+  if (!pass && blockIdx.x == 0 && threadIdx.x == 0) { s.tcount[nv] = 0u; s.scan_n[2] = nv; }
+  GRID_STRIDE(v, nv) {
+    const int c = (int)s.cube_of[v];
+    const int x = c % s.g.nx, y = (c / s.g.nx) % s.g.ny, z = c / (s.g.nx * s.g.ny);
     uint32_t cnt = 0;
-    if (s.vflag[c + 1] != s.vflag[c]) {
-      const int ci = sr_cube_mask(s, x, y, z);
-      int64_t o = pass ? (int64_t)s.tcount[c] : 0;
-      for (int k = 0; k < 3; ++k) {
-        const int w = k == 0 ? 2 : k == 1 ? 3 : 11;
-        if (!sr_edge_cross(ci, w)) continue;
-        int d[4][3];
-        sr_edge_cubes(w, d);
-        int64_t id[4];
-        bool ok = true;
-        for (int q = 0; q < 4; ++q) {
-          id[q] = sr_vid(s, x + d[q][0], y + d[q][1], z + d[q][2]);
-          ok = ok && id[q] >= 0;
-        }
-        if (!ok) continue;
-        cnt += 6;
-        if (pass) {
-          if (o + 6 > s.max_i) { sr_fail(s, NN_ERR_CAPACITY); continue; }
-          const bool cond0 = (ci >> c_sr_edge[w][0]) & 1;
-          const bool flip = cond0 != (w == 11);
-          const int64_t t[6] = {id[2], id[1], id[0], id[3], id[2], id[0]};
-          const int64_t tf[6] = {id[0], id[1], id[2], id[0], id[2], id[3]};
-          for (int q = 0; q < 6; ++q) s.tri[o + q] = (int32_t)(flip ? tf[q] : t[q]);
-          o += 6;
-        }
+    const int ci = sr_cube_mask(s, x, y, z);
+    int64_t o = pass ? (int64_t)s.tcount[v] : 0;
+    for (int k = 0; k < 3; ++k) {
+      const int w = k == 0 ? 2 : k == 1 ? 3 : 11;
+      if (!sr_edge_cross(ci, w)) continue;
+      int d[4][3];
+      sr_edge_cubes(w, d);
+      int64_t id[4];
+      bool ok = true;
+      for (int q = 0; q < 4; ++q) {
+        id[q] = sr_vid(s, x + d[q][0], y + d[q][1], z + d[q][2]);
+        ok = ok && id[q] >= 0;
+      }
+      if (!ok) continue;
+      cnt += 6;
+      if (pass) {
+        if (o + 6 > s.max_i) { sr_fail(s, NN_ERR_CAPACITY); continue; }
+        const bool cond0 = (ci >> c_sr_edge[w][0]) & 1;
+        const bool flip = cond0 != (w == 11);
+        const int64_t t[6] = {id[2], id[1], id[0], id[3], id[2], id[0]};
+        const int64_t tf[6] = {id[0], id[1], id[2], id[0], id[2], id[3]};
+        for (int q = 0; q < 6; ++q) s.tri[o + q] = (int32_t)(flip ? tf[q] : t[q]);
+        o += 6;
       }
     }
-    if (!pass) s.tcount[c] = cnt;
+    if (!pass) s.tcount[v] = cnt;
   }
+}
+
+// What the host reads back, in one copy.
+__global__ void k_sr_result(SrDev s, int64_t cells, int marching_cubes) {
+  const uint32_t nv = s.vflag[cells];
+  *s.result = SrResult{nv, s.tcount[marching_cubes ? cells : min((int64_t)nv, (int64_t)s.max_v)], *s.status, 0,
+                       s.stats[3]};
 }
 
 // ---- 6b. marching cubes (marching_cube_impl, srtool.py:1765-1800) ----------------------
@@ -963,9 +1026,10 @@ __constant__ SrMcTable c_sr_mc = sr_make_mc_table();
 
 // pass 0: vertices (crossing edges) and indices per cube into vflag / tcount;
 // pass 1: both written at the scanned offsets, in edge order within a cube
-__global__ void k_sr_mc(SrDev s, int64_t cells, int pass) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < cells; c += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(c % s.g.nx), y = (int)((c / s.g.nx) % s.g.ny), z = (int)(c / ((int64_t)s.g.nx * s.g.ny));
+__global__ void k_sr_mc(SrDev s, int32_t cells, int pass) {
+  if (!pass && blockIdx.x == 0 && threadIdx.x == 0) s.vflag[cells] = s.tcount[cells] = 0u;
+  FOR_SR_ROWS(s, x, y, z, c, act) {
+    (void)act;
     if (pass == 1 && s.vflag[c + 1] == s.vflag[c]) continue;
     // a cube with a crossing has a nonzero corner, which lies in an active block: the
     // reference's visit of the cubes around the active vertices reaches every such cube
@@ -1016,8 +1080,8 @@ struct nn_sr_ctx {
   int sms = 148;
   int32_t max_particles = 0, max_v = 0, max_i = 0;
   int64_t max_cells = 0, blocks = 0;
-  int32_t* d_n = nullptr;  // scan sizes ([2] = last index of the current scan)
-  int32_t* status = nullptr;
+  int32_t* d_n = nullptr;  // scan sizes ([2] = last index of the current scan, set on the device)
+  int32_t* status = nullptr;  // behind the four stats
   uint32_t *vcount = nullptr, *vkey = nullptr, *vrank = nullptr, *vflag = nullptr, *tcount = nullptr,
            *tile_sums = nullptr, *cube_of = nullptr;
   int32_t *vsrc = nullptr, *tri = nullptr;
@@ -1028,6 +1092,7 @@ struct nn_sr_ctx {
   float *splat = nullptr, *fa = nullptr, *fb = nullptr, *G = nullptr, *xbar = nullptr, *vert = nullptr, *nrm = nullptr;
   uint8_t* active = nullptr;
   double* stats = nullptr;
+  SrResult *result = nullptr, *h_result = nullptr;  // h_result: pinned
   // last call
   SrDev last{};
   int64_t cells = 0;
@@ -1053,20 +1118,20 @@ static int sr_fail_host(nn_sr_ctx* c, int code, const char* fmt, ...) {
   } while (0)
 
 static void sr_free(nn_sr_ctx* c) {
-  void* bufs[] = {c->d_n, c->status, c->vcount, c->vkey, c->vrank, c->vflag, c->tcount, c->tile_sums, c->vsrc,
+  if (c->h_result) cudaFreeHost(c->h_result);
+  void* bufs[] = {c->d_n, c->result, c->vcount, c->vkey, c->vrank, c->vflag, c->tcount, c->tile_sums, c->vsrc,
                   c->tri, c->fix, c->splat, c->fa, c->fb, c->G, c->xbar, c->vert, c->nrm, c->active, c->stats,
                   c->cube_of, c->spos, c->vfix, c->mvel};
   for (void* b : bufs) cudaFree(b);
 }
 
-// An exclusive scan of a[0 .. len) in place with the neighbour search's scan kernels.
+// An exclusive scan in place with the neighbour search's scan kernels, of a[0 .. d_n[2]],
+// at most len entries.
 static int sr_scan(nn_sr_ctx* c, uint32_t* a, int64_t len, cudaStream_t st) {
   Dev d{};
   d.d_n = c->d_n;
   d.cell_count = a;
   d.tile_sums = c->tile_sums;
-  const int32_t hn[3] = {0, 0, (int32_t)(len - 1)};
-  SRCK(cudaMemcpyAsync(c->d_n, hn, sizeof(hn), cudaMemcpyHostToDevice, st));
   const int tiles = (int)((len + SCAN_TILE - 1) / SCAN_TILE);
   k_scan_tiles<<<std::max(1, std::min(tiles, c->sms * 2)), SCAN_THREADS, 0, st>>>(d);
   k_scan_apply<<<std::max(1, std::min(tiles, c->sms * 2)), SCAN_THREADS, 0, st>>>(d);
@@ -1097,7 +1162,9 @@ int nn_sr_create(int32_t max_particles, int64_t max_cells, int32_t max_vertices,
   auto al = [&](auto** p, size_t cnt) {
     if (e == cudaSuccess) e = cudaMalloc((void**)p, cnt * sizeof(**p));
   };
-  al(&c->d_n, 4); al(&c->status, 1); al(&c->stats, 4);
+  al(&c->d_n, 4); al(&c->stats, 5); al(&c->result, 1);
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_result, sizeof(SrResult));
+  c->status = reinterpret_cast<int32_t*>(c->stats + 4);
   al(&c->vcount, CL); al(&c->vflag, CL); al(&c->tcount, CL); al(&c->tile_sums, tiles);
   al(&c->vkey, N); al(&c->vrank, N); al(&c->vsrc, N); al(&c->spos, N); al(&c->G, 9 * N); al(&c->xbar, 3 * N);
   al(&c->fix, CL); al(&c->splat, CL); al(&c->fa, CL); al(&c->fb, CL); al(&c->active, blocks);
@@ -1156,7 +1223,7 @@ static int sr_run(nn_sr_ctx* c, const nn_sr_params* p, const float* pos, const f
   s.n = n; s.pos = pos; s.status = c->status;
   s.vcount = c->vcount; s.vkey = c->vkey; s.vrank = c->vrank; s.vsrc = c->vsrc; s.spos = c->spos;
   s.fix = c->fix; s.splat = c->splat; s.field = c->fa; s.tmp = c->fb; s.active = c->active;
-  s.G = c->G; s.xbar = c->xbar; s.stats = c->stats; s.vflag = c->vflag; s.tcount = c->tcount;
+  s.G = c->G; s.xbar = c->xbar; s.stats = c->stats; s.scan_n = c->d_n; s.result = c->result; s.vflag = c->vflag; s.tcount = c->tcount;
   s.vert = c->vert; s.tri = c->tri; s.nrm = c->nrm; s.max_v = c->max_v; s.max_i = c->max_i;
   s.cube_of = c->cube_of;
   s.vel = vel; s.vfix = c->vfix; s.mvel = c->mvel;
@@ -1189,17 +1256,20 @@ static int sr_run(nn_sr_ctx* c, const nn_sr_params* p, const float* pos, const f
   const int B = 256;
   const int grid_n = std::max(1, std::min((n + B - 1) / B, c->sms * 8));
   const int grid_c = (int)std::max<int64_t>(1, std::min<int64_t>((cells + B - 1) / B, (int64_t)c->sms * 16));
-  SRCK(cudaMemsetAsync(c->status, 0, sizeof(int32_t), st));
-  SRCK(cudaMemsetAsync(c->stats, 0, 4 * sizeof(double), st));
+  const int grid_r = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)bx * s.g.ny * s.g.nz * 32 + B - 1) / B,
+                                                                 (int64_t)c->sms * 16));  // rows, a warp each
+  SRCK(cudaMemsetAsync(c->stats, 0, 5 * sizeof(double), st));  // and the status
   SRCK(cudaMemsetAsync(c->vcount, 0, (cells + 1) * sizeof(uint32_t), st));
   SRCK(cudaMemsetAsync(c->fix, 0, cells * sizeof(unsigned long long), st));
   if (vel) SRCK(cudaMemsetAsync(c->vfix, 0, 3 * cells * sizeof(unsigned long long), st));
   SRCK(cudaMemsetAsync(c->active, 0, blocks, st));
-  SRCK(cudaMemsetAsync(c->G, 0, 9 * (size_t)std::max(n, 1) * sizeof(float), st));
-  SRCK(cudaMemsetAsync(c->xbar, 0, 3 * (size_t)std::max(n, 1) * sizeof(float), st));
+  if (!p->use_smooth_field) {  // else the pre-pass writes every particle's
+    SRCK(cudaMemsetAsync(c->G, 0, 9 * (size_t)std::max(n, 1) * sizeof(float), st));
+    SRCK(cudaMemsetAsync(c->xbar, 0, 3 * (size_t)std::max(n, 1) * sizeof(float), st));
+  }
   if (n > 0) {
     // 1. binning
-    k_sr_keys<<<grid_n, B, 0, st>>>(s);
+    k_sr_keys<<<grid_n, B, 0, st>>>(s, (int32_t)cells);
     RC(sr_scan(c, c->vcount, cells + 1, st));
     k_sr_scatter<<<grid_n, B, 0, st>>>(s);
     k_sr_voxel_sort<<<grid_c, B, 0, st>>>(s, cells);
@@ -1215,46 +1285,45 @@ static int sr_run(nn_sr_ctx* c, const nn_sr_params* p, const float* pos, const f
       if (vel) k_sr_vel_splat<<<grid_w, B, 0, st>>>(s);
     }
   }
-  k_sr_fix_to_field<<<grid_c, B, 0, st>>>(s, cells);
-  // 5. smoothing
+  k_sr_fix_to_field<<<grid_c, B, 0, st>>>(s, (int32_t)cells);
+  // 5. smoothing (the first iteration's pass 0 ran with the conversion)
   for (int it = 0; it < p->smooth_iterations; ++it) {
-    SRCK(cudaMemsetAsync(c->stats, 0, 4 * sizeof(double), st));
-    k_sr_stats<<<grid_c, B, 0, st>>>(s, cells, 0);
-    k_sr_stats<<<grid_c, B, 0, st>>>(s, cells, 1);
+    if (it > 0) {
+      SRCK(cudaMemsetAsync(c->stats, 0, 4 * sizeof(double), st));
+      k_sr_stats<<<grid_r, B, 0, st>>>(s, 0);
+    }
+    k_sr_stats<<<grid_r, B, 0, st>>>(s, 1);
     k_sr_sd<<<1, 32, 0, st>>>(s);
-    k_sr_smooth<<<grid_c, B, 0, st>>>(s, cells);
+    if (p->smooth_cells == 1) k_sr_smooth<1><<<grid_r, B, 0, st>>>(s);
+    else k_sr_smooth<0><<<grid_r, B, 0, st>>>(s);
     std::swap(s.field, s.tmp);
   }
-  SRCK(cudaMemsetAsync(c->vflag, 0, (cells + 1) * sizeof(uint32_t), st));
-  SRCK(cudaMemsetAsync(c->tcount, 0, (cells + 1) * sizeof(uint32_t), st));
   if (marching_cubes) {
     // 6b. marching cubes: count, scan, write
-    k_sr_mc<<<grid_c, B, 0, st>>>(s, cells, 0);
+    k_sr_mc<<<grid_r, B, 0, st>>>(s, (int32_t)cells, 0);
     RC(sr_scan(c, c->vflag, cells + 1, st));
     RC(sr_scan(c, c->tcount, cells + 1, st));
-    k_sr_mc<<<grid_c, B, 0, st>>>(s, cells, 1);
+    k_sr_mc<<<grid_r, B, 0, st>>>(s, (int32_t)cells, 1);
   } else {
     // 6. dual contouring
-    k_sr_dc_flag<<<grid_c, B, 0, st>>>(s, cells);
+    const int64_t most = std::min<int64_t>(cells, s.max_v);  // vertices
+    const int grid_v = (int)std::max<int64_t>(1, std::min<int64_t>((most + 127) / 128, (int64_t)c->sms * 16));
+    k_sr_dc_flag<<<grid_r, B, 0, st>>>(s, (int32_t)cells);
     RC(sr_scan(c, c->vflag, cells + 1, st));
-    k_sr_dc_list<<<grid_c, B, 0, st>>>(s, cells);
+    k_sr_dc_list<<<grid_c, B, 0, st>>>(s, (int32_t)cells);
     k_sr_dc_point<<<c->sms * 4, 128, 0, st>>>(s, cells);
-    k_sr_tris<<<grid_c, B, 0, st>>>(s, cells, 0);
-    RC(sr_scan(c, c->tcount, cells + 1, st));
-    k_sr_tris<<<grid_c, B, 0, st>>>(s, cells, 1);
+    k_sr_tris<<<grid_v, 128, 0, st>>>(s, cells, 0);
+    RC(sr_scan(c, c->tcount, most + 1, st));
+    k_sr_tris<<<grid_v, 128, 0, st>>>(s, cells, 1);
   }
+  k_sr_result<<<1, 1, 0, st>>>(s, cells, marching_cubes ? 1 : 0);
   SRCK(cudaGetLastError());
-  uint32_t counts[2];
-  int32_t status = 0;
-  double sd = 0.0;
-  SRCK(cudaMemcpyAsync(&counts[0], c->vflag + cells, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  SRCK(cudaMemcpyAsync(&counts[1], c->tcount + cells, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  SRCK(cudaMemcpyAsync(&status, c->status, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  SRCK(cudaMemcpyAsync(&sd, c->stats + 3, sizeof(double), cudaMemcpyDeviceToHost, st));
+  SRCK(cudaMemcpyAsync(c->h_result, c->result, sizeof(SrResult), cudaMemcpyDeviceToHost, st));
   SRCK(cudaStreamSynchronize(st));
-  c->nv = (int32_t)counts[0];
-  c->ni = (int32_t)counts[1];
-  c->sd = sd;
+  int32_t status = c->h_result->status;
+  c->nv = (int32_t)c->h_result->nv;
+  c->ni = (int32_t)c->h_result->ni;
+  c->sd = c->h_result->sd;
   if (status == 0 && (c->nv > c->max_v || c->ni > c->max_i)) status = NN_ERR_CAPACITY;
   if (status != 0) {
     if (status == NN_ERR_INVALID_ARG) return sr_fail_host(c, status, "a particle lies outside the grid");
