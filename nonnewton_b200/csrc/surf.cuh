@@ -448,14 +448,15 @@ __device__ __forceinline__ float rsqrt_min(float x) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(x, 1.17549435e-38f)));
   return r;
 }
-__global__ void __launch_bounds__(SR_SPLAT_WARPS * 32) k_sr_aniso_splat(SrDev s) {
+__global__ void __launch_bounds__(SR_SPLAT_WARPS * 32) k_sr_aniso_splat(SrDev s, int parts) {
   // per pair of planes: the z terms G[.][2] d2 and the scale (2^32 x multiplicity, times the
   // volume where the conversion is the narrow one)
   __shared__ __align__(16) float zt_all[SR_SPLAT_WARPS][4 * SR_ZC];
   float* zt = zt_all[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < s.n; i += warps) {
+  for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < s.n * parts; k += warps) {
+    const int i = k / parts, part = k % parts;
     const SrGrid& g = s.g;
     int cx, cy, cz;
     g.voxel_of(s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2], cx, cy, cz);
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(SR_SPLAT_WARPS * 32) k_sr_aniso_splat(SrDev s)
         e[6] = narrow ? s.volume * (4294967296.f * (float)mz) : 4294967296.f * (float)mz;
       }
       __syncwarp();
-      for (int col = lane; col < ncol; col += 32) {
+      for (int col = lane + 32 * part; col < ncol; col += 32 * parts) {
         const int x = w0[0] + col % nxw, y = w0[1] + col / nxw;
         const int mxy = ((x - 1 >= lo[0] && x - 1 <= hi[0]) + (x >= lo[0] && x <= hi[0])) *
                         ((y - 1 >= lo[1] && y - 1 <= hi[1]) + (y >= lo[1] && y <= hi[1]));
@@ -838,39 +839,84 @@ __global__ void k_sr_dc_list(SrDev s, int32_t cells) {
 }
 
 // One point per crossing cube: the mass point of the edge crossings plus the clamped
-// QEF solution, kept only if it stays in its cube (srtool.py:1536-1596)
-__global__ void k_sr_dc_point(SrDev s, int64_t cells) {
-  const int64_t nv = min((int64_t)s.vflag[cells], (int64_t)s.max_v);
-  for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < nv; id += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t c = s.cube_of[id];
-    const int x = (int)(c % s.g.nx), y = (int)((c / s.g.nx) % s.g.ny), z = (int)(c / ((int64_t)s.g.nx * s.g.ny));
+// QEF solution, kept only if it stays in its cube (srtool.py:1536-1596).
+//
+// Bound by the FP64 chain per cube, above all the field normals at its 4 to 12 crossings
+// (8 vertex normals each). SR_QEF_LANES lanes share a cube: lane l takes the crossings
+// l, l + 4, l + 8 of its edge order, and all of them fold the crossings' terms in that
+// order by shuffles, so the sums are the one-thread sums. 52 -> 25 us on 5,400 cubes,
+// 90 -> 94 us on 61,000 (the eigen-decomposition is every lane's).
+#define SR_QEF_LANES 4
+__global__ void __launch_bounds__(128) k_sr_dc_point(SrDev s, int64_t cells) {
+  constexpr int L = SR_QEF_LANES, SLOTS = 12 / L;
+  const unsigned full = 0xffffffffu;
+  const int nv = (int)min((int64_t)s.vflag[cells], (int64_t)s.max_v);
+  const int l = (int)threadIdx.x & (L - 1), g0 = (int)threadIdx.x & 31 & ~(L - 1);
+  // the warp's first cube decides, so that all its lanes reach the shuffles
+  for (int first = (int)(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / L; first < nv;
+       first += (int)(gridDim.x * blockDim.x) / L) {
+    const int id = min(first + (int)(threadIdx.x & 31) / L, nv - 1);
+    const int c = (int)s.cube_of[id];
+    const int x = c % s.g.nx, y = (c / s.g.nx) % s.g.ny, z = c / (s.g.nx * s.g.ny);
     const int ci = sr_cube_mask(s, x, y, z);
-    double P[12][3];
-    int cnt = 0;
-    double mean[3] = {0.0, 0.0, 0.0};
-    for (int w = 0; w < 12; ++w) {
-      if (!sr_edge_cross(ci, w)) continue;
-      const int a = c_sr_edge[w][0], b = c_sr_edge[w][1];
-      const int ax = x + c_sr_off[a][0], ay = y + c_sr_off[a][1], az = z + c_sr_off[a][2];
-      const int bx = x + c_sr_off[b][0], by = y + c_sr_off[b][1], bz = z + c_sr_off[b][2];
-      const double v1 = sr_get(s, s.field, ax, ay, az), v2 = sr_get(s, s.field, bx, by, bz);
-      const double delta = v2 - v1;
-      const double t = fabs(delta) < 1e-5 ? 0.5 : ((double)s.iso - v1) / delta;  // vertex_interpolate
-      const double p1[3] = {ax * s.g.dvs + s.g.dox, ay * s.g.dvs + s.g.doy, az * s.g.dvs + s.g.doz};
-      const double p2[3] = {bx * s.g.dvs + s.g.dox, by * s.g.dvs + s.g.doy, bz * s.g.dvs + s.g.doz};
-      for (int k = 0; k < 3; ++k) { P[cnt][k] = p1[k] + t * (p2[k] - p1[k]); mean[k] += P[cnt][k]; }
-      ++cnt;
-    }
-    for (int k = 0; k < 3; ++k) mean[k] /= cnt;
-    double NtN[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, Ntb[3] = {0, 0, 0};
-    for (int r = 0; r < cnt; ++r) {
-      double n[3];
-      sr_normal_at(s, P[r], n);
-      const double bb = n[0] * (P[r][0] - mean[0]) + n[1] * (P[r][1] - mean[1]) + n[2] * (P[r][2] - mean[2]);
-      for (int i = 0; i < 3; ++i) {
-        Ntb[i] += n[i] * bb;
-        for (int j = 0; j < 3; ++j) NtN[i][j] += n[i] * n[j];
+    uint32_t em = 0u;
+#pragma unroll
+    for (int w = 0; w < 12; ++w) em |= (uint32_t)sr_edge_cross(ci, w) << w;
+    const int cnt = __popc(em);
+    double P[SLOTS][3], N[SLOTS][3], bb[SLOTS];
+    for (int k = 0; k < l; ++k) em &= em - 1u;  // to this lane's first crossing
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+      if (q * L + l < cnt) {
+        const int w = __ffs(em) - 1;
+#pragma unroll
+        for (int k = 0; k < L; ++k) em &= em - 1u;
+        const int a = c_sr_edge[w][0], b = c_sr_edge[w][1];
+        const int ax = x + c_sr_off[a][0], ay = y + c_sr_off[a][1], az = z + c_sr_off[a][2];
+        const int bx = x + c_sr_off[b][0], by = y + c_sr_off[b][1], bz = z + c_sr_off[b][2];
+        const double v1 = sr_get(s, s.field, ax, ay, az), v2 = sr_get(s, s.field, bx, by, bz);
+        const double delta = v2 - v1;
+        const double t = fabs(delta) < 1e-5 ? 0.5 : ((double)s.iso - v1) / delta;  // vertex_interpolate
+        const double p1[3] = {ax * s.g.dvs + s.g.dox, ay * s.g.dvs + s.g.doy, az * s.g.dvs + s.g.doz};
+        const double p2[3] = {bx * s.g.dvs + s.g.dox, by * s.g.dvs + s.g.doy, bz * s.g.dvs + s.g.doz};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) P[q][k] = p1[k] + t * (p2[k] - p1[k]);
+      } else {
+        P[q][0] = P[q][1] = P[q][2] = 0.0;
       }
+    }
+    double mean[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int r = 0; r < 12; ++r)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const double v = __shfl_sync(full, P[r / L][k], g0 + r % L);
+        if (r < cnt) mean[k] += v;
+      }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) mean[k] /= cnt;
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+      N[q][0] = N[q][1] = N[q][2] = bb[q] = 0.0;
+      if (q * L + l < cnt) {
+        sr_normal_at(s, P[q], N[q]);
+        bb[q] = N[q][0] * (P[q][0] - mean[0]) + N[q][1] * (P[q][1] - mean[1]) + N[q][2] * (P[q][2] - mean[2]);
+      }
+    }
+    double NtN[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, Ntb[3] = {0, 0, 0};
+#pragma unroll
+    for (int r = 0; r < 12; ++r) {
+      double n[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) n[k] = __shfl_sync(full, N[r / L][k], g0 + r % L);
+      const double b = __shfl_sync(full, bb[r / L], g0 + r % L);
+      if (r < cnt)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          Ntb[i] += n[i] * b;
+#pragma unroll
+          for (int k = 0; k < 3; ++k) NtN[i][k] += n[i] * n[k];
+        }
     }
     double lam[3], V[3][3], res[3] = {0.0, 0.0, 0.0};
     sr_sym_eig(NtN, lam, V);
@@ -883,7 +929,8 @@ __global__ void k_sr_dc_point(SrDev s, int64_t cells) {
     int qx, qy, qz;
     s.g.voxel_of((float)(res[0] + mean[0]), (float)(res[1] + mean[1]), (float)(res[2] + mean[2]), qx, qy, qz);
     const bool keep = qx == x && qy == y && qz == z;
-    for (int k = 0; k < 3; ++k) s.vert[3 * id + k] = (float)(keep ? res[k] + mean[k] : mean[k]);
+    if (l != 0 || id != first + (int)(threadIdx.x & 31) / L) continue;
+    for (int k = 0; k < 3; ++k) s.vert[3 * (int64_t)id + k] = (float)(keep ? res[k] + mean[k] : mean[k]);
   }
 }
 
@@ -1281,7 +1328,12 @@ static int sr_run(nn_sr_ctx* c, const nn_sr_params* p, const float* pos, const f
       const int grid_w = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * 32 + B - 1) / B, c->sms * 16));
       const int ppw = sr_pre_ppw(n, c->sms), per = SR_PRE_WARPS * ppw;
       k_sr_aniso_pre<<<(n + per - 1) / per, SR_PRE_WARPS * 32, 0, st>>>(s, ppw);
-      k_sr_aniso_splat<<<grid_w, B, 0, st>>>(s);
+      // several warps share a particle's columns in a small set, whose warps (one chain of
+      // 20 column rounds each) would leave most of an SM's 24 slots empty: 71 -> 53 us on
+      // 1,791 particles (2 warps 58, 8 58)
+      const int parts = std::min(std::max((48 * c->sms + n / 2) / n, 1), 8);
+      const int grid_s = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * parts * 32 + B - 1) / B, c->sms * 16));
+      k_sr_aniso_splat<<<grid_s, B, 0, st>>>(s, parts);
       if (vel) k_sr_vel_splat<<<grid_w, B, 0, st>>>(s);
     }
   }
@@ -1311,7 +1363,7 @@ static int sr_run(nn_sr_ctx* c, const nn_sr_params* p, const float* pos, const f
     k_sr_dc_flag<<<grid_r, B, 0, st>>>(s, (int32_t)cells);
     RC(sr_scan(c, c->vflag, cells + 1, st));
     k_sr_dc_list<<<grid_c, B, 0, st>>>(s, (int32_t)cells);
-    k_sr_dc_point<<<c->sms * 4, 128, 0, st>>>(s, cells);
+    k_sr_dc_point<<<grid_v, 128, 0, st>>>(s, cells);
     k_sr_tris<<<grid_v, 128, 0, st>>>(s, cells, 0);
     RC(sr_scan(c, c->tcount, most + 1, st));
     k_sr_tris<<<grid_v, 128, 0, st>>>(s, cells, 1);
