@@ -4,8 +4,10 @@
 
 // Sorted working set: particles in cell order ("slots").
 struct WorkSet {
-  real4* pos;       // x, y, z, volume (negative for solids)
-  real4* vel;       // v, w = mass (a copy of `mass`, so neighbour loops get it with v)
+  real4* pos;       // x, y, z, volume (negative for solids) at the search: what the passes gather
+                    // that need no velocity (advection and rigid bodies move pv only)
+  real4* pv;        // [2i] the same, moved on by the step's end, and [2i + 1] the velocity, w = mass
+                    // (a copy of `mass`): one sector, see load_pv
   real* mass;
   real* dens;
   uint32_t* flags;   // class bits | scene << NN_SCENE_SHIFT
@@ -52,8 +54,8 @@ struct Dev {
   real* mu;
   // implicit viscosity CG (slot order)
   real4* cg_x; real4* cg_r; real4* cg_z; real4* cg_Ap;
-  real4* cg_p;                 // search direction; w = mu_i (read by the matvec)
-  real4* cg_pos;               // matvec positions: fluid (x_i, m_i / rho_i), solid (x_i, -V_i) as pos
+  real4* cg_pp;                // the matvec's operands: [2i] positions, fluid (x_i, m_i / rho_i), solid
+                               // (x_i, -V_i) as pos; [2i + 1] search direction, w = mu_i
   real2* cg_aux;               // fluid: mu_i, m_i / rho_i; solid: 0, 1 if dynamic
   real* cg_pinv;               // [6][cap] symmetric inverse of the diagonal block
   // elasticity (e-space: elastic particles in id order)
@@ -80,6 +82,25 @@ struct Dev {
   unsigned long long loop_handle; // cudaGraphConditionalHandle (0 when not in a graph)
   int32_t* body_count;         // [4] executed loop bodies (div, pressure, cg, elastic)
 };
+
+// The pair of float4 of a slot, position and velocity (or the matvec's), in one 256-bit
+// load (ld.global.nc.v8.f32): one request and one sector per neighbour, where two float4
+// gathers took two requests that each used half of theirs.
+struct GPV { real4 p, v; };
+__device__ __forceinline__ GPV load_pv(const real4* pv, int j) {
+  const real4* q = pv + 2 * (size_t)j;
+#ifdef NN_FP64
+  return GPV{ldg(q), ldg(q + 1)};
+#else
+  GPV g;
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(g.p.x), "=f"(g.p.y), "=f"(g.p.z), "=f"(g.p.w), "=f"(g.v.x), "=f"(g.v.y), "=f"(g.v.z), "=f"(g.v.w)
+      : "l"(q));
+  return g;
+#endif
+}
+__device__ __forceinline__ real4& xyz_of(const Dev& d, int i) { return d.w.pv[2 * (size_t)i]; }
+__device__ __forceinline__ real4& vel_of(const Dev& d, int i) { return d.w.pv[2 * (size_t)i + 1]; }
 
 // A neighbour's position + volume in the neighbour passes (read-only there).
 __device__ __forceinline__ real4 pos_of(const Dev& d, int j) { return ldg(&d.w.pos[j]); }

@@ -89,7 +89,7 @@ struct nn_ctx {
   int32_t* slot_of_id = nullptr;
   uint32_t *key = nullptr, *rank = nullptr, *cell_count = nullptr, *tile_sums = nullptr;
   int32_t *src = nullptr, *nbr = nullptr, *nbr_cnt = nullptr;
-  real4 *cg_x = nullptr, *cg_r = nullptr, *cg_z = nullptr, *cg_p = nullptr, *cg_Ap = nullptr, *cg_pos = nullptr;
+  real4 *cg_x = nullptr, *cg_r = nullptr, *cg_z = nullptr, *cg_pp = nullptr, *cg_Ap = nullptr;
   real2* cg_aux = nullptr;
   real* cg_pinv = nullptr;
   int el_cap = 64, el_stride = 0;
@@ -185,7 +185,7 @@ static Dev make_dev(nn_ctx* c, int cur) {
   d.max_nb = c->max_nb;
   d.srn = c->srn;
   d.mu = c->mu;
-  d.cg_x = c->cg_x; d.cg_r = c->cg_r; d.cg_z = c->cg_z; d.cg_p = c->cg_p; d.cg_Ap = c->cg_Ap; d.cg_pos = c->cg_pos;
+  d.cg_x = c->cg_x; d.cg_r = c->cg_r; d.cg_z = c->cg_z; d.cg_pp = c->cg_pp; d.cg_Ap = c->cg_Ap;
   d.cg_aux = c->cg_aux;
   d.cg_pinv = c->cg_pinv;
   d.el_id = c->el_id; d.el_slot = c->el_slot; d.e_of_id = c->e_of_id; d.el_x0 = c->el_x0;
@@ -245,15 +245,14 @@ static int launch1(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), Args... args)
   return NN_OK;
 }
 
-// Each one-lane pass's neighbour-batch depth at unroll 0, measured against the other depth on
-// the 2.4M-particle dam break (early and settled states): the update passes, with
-// little arithmetic per pair, keep 2 neighbours in flight (at 1: k_pressure_update
-// +17-31 %, k_density_adv +3 %); the passes with more arithmetic per pair gather one
-// at a time, with 8 list entries loaded ahead (k_density_change_np -9 %, k_cg_setup
-// -7 %, k_density_factor -6 %, k_cg_matvec -4 %, k_density_change -2 %). The force
-// pass keeps 2 (the 23k-particle dam break: 29.0 against 31.0 us at 1).
+// Each one-lane pass's neighbour-batch depth at unroll 0. With the 256-bit gathers
+// (load_pv) one neighbour at a time, with 8 list entries loaded ahead, is the fastest for
+// all of them: more gathers in flight per thread thrash L1 (2.4M-particle dam break, us at
+// 1 / 2 / 4 in flight: k_density_adv 218 / 236 / 242, k_density_factor 258 / 320 / 333,
+// k_divergence_update 208 / 227 / 227, k_cg_setup 315 / 357 / 538; k_forces with the
+// explicit viscosity on 125,000 fluid 33 / 47).
 enum : int {
-  U_PRESSURE_UPDATE = 2, U_DENSITY_ADV = 2, U_DIVERGENCE_UPDATE = 2, U_BOUNDARY_VOLUME = 2, U_FORCES = 2,
+  U_PRESSURE_UPDATE = 1, U_DENSITY_ADV = 1, U_DIVERGENCE_UPDATE = 1, U_BOUNDARY_VOLUME = 2, U_FORCES = 1,
   U_DENSITY_FACTOR = 1, U_DENSITY_CHANGE = 1, U_DENSITY_CHANGE_NP = 1, U_CG_SETUP = 1, U_CG_MATVEC = 1
 };
 static inline int ku(const nn_ctx* c, int pass_default) { return c->unroll ? c->unroll : pass_default; }
@@ -725,16 +724,18 @@ int nn_ctx_create(int32_t max_particles, int32_t max_scenes, int32_t max_neighbo
     if (_e != cudaSuccess) return bail(fail(nullptr, NN_ERR_OOM, "cudaMalloc %s: %s", #p, cudaGetErrorString(_e))); \
   } while (0)
   for (int k = 0; k < 2; ++k) {
-    AL(c->set[k].pos, N); AL(c->set[k].vel, N); AL(c->set[k].mass, N); AL(c->set[k].dens, N);
+    AL(c->set[k].pv, 2 * N); AL(c->set[k].mass, N); AL(c->set[k].dens, N);
     AL(c->set[k].flags, N); AL(c->set[k].id, N);
   }
+  AL(c->set[0].pos, N);  // one for both sets: the previous slots' positions are read from their pv
+  c->set[1].pos = c->set[0].pos;
   AL(c->d_n, 4); AL(c->d_sc, (size_t)max_scenes); AL(c->d_dyn, (size_t)max_scenes);
   AL(c->d_acc, (size_t)max_scenes * ACC_COUNT * NN_STRIPES);
   AL(c->d_scene_of_id, N); AL(c->d_src_flag, 1); AL(c->acc4, N);
   AL(c->alpha, N); AL(c->rho_adv, N); AL(c->kappa, N); AL(c->srn, N); AL(c->mu, N);
   AL(c->slot_of_id, N); AL(c->key, N); AL(c->rank, N); AL(c->src, N);
   AL(c->nbr, N * (size_t)max_neighbors); AL(c->nbr_cnt, N);
-  AL(c->cg_x, N); AL(c->cg_r, N); AL(c->cg_z, N); AL(c->cg_p, N); AL(c->cg_Ap, N); AL(c->cg_pos, N); AL(c->cg_aux, N);
+  AL(c->cg_x, N); AL(c->cg_r, N); AL(c->cg_z, N); AL(c->cg_pp, 2 * N); AL(c->cg_Ap, N); AL(c->cg_aux, N);
   AL(c->cg_pinv, 6 * N);
   AL(c->e_of_id, N);
   AL(c->d_any, 1); AL(c->d_body, 4);
@@ -764,12 +765,12 @@ int nn_ctx_destroy(nn_ctx* c) {
   if (!c) return NN_OK;
   drop_graphs(c);
   for (int k = 0; k < 2; ++k) {
-    cudaFree(c->set[k].pos); cudaFree(c->set[k].vel); cudaFree(c->set[k].mass); cudaFree(c->set[k].dens);
+    cudaFree(c->set[k].pv); cudaFree(c->set[k].mass); cudaFree(c->set[k].dens);
     cudaFree(c->set[k].flags); cudaFree(c->set[k].id);
   }
-  void* bufs[] = {c->d_n, c->d_sc, c->d_dyn, c->d_acc, c->d_scene_of_id, c->d_src_flag, c->acc4, c->alpha,
+  void* bufs[] = {c->set[0].pos, c->d_n, c->d_sc, c->d_dyn, c->d_acc, c->d_scene_of_id, c->d_src_flag, c->acc4, c->alpha,
                   c->rho_adv, c->kappa, c->srn, c->mu, c->slot_of_id, c->key, c->rank, c->src, c->nbr,
-                  c->nbr_cnt, c->cg_x, c->cg_r, c->cg_z, c->cg_p, c->cg_Ap, c->cg_pos, c->cg_aux, c->cg_pinv,
+                  c->nbr_cnt, c->cg_x, c->cg_r, c->cg_z, c->cg_pp, c->cg_Ap, c->cg_aux, c->cg_pinv,
                   c->e_of_id, c->d_any, c->d_body, c->cell_count, c->tile_sums};
   for (void* b : bufs) cudaFree(b);
   free_elastic(c);

@@ -67,7 +67,7 @@ __global__ void k_keys(Dev d) {
       x = X[3 * s]; y = X[3 * s + 1]; z = X[3 * s + 2];
       sc = d.scene_of_id[s];
     } else {
-      real4 p = d.wo.pos[s];
+      const real4 p = d.wo.pv[2 * (size_t)s];
       x = p.x; y = p.y; z = p.z;
       sc = slot_scene(d.wo.flags[s]);
     }
@@ -281,14 +281,16 @@ __global__ void k_gather(Dev d) {
              ((uint32_t)sc << NN_SCENE_SHIFT);
       } else {
         id = d.wo.id[s];
-        p = d.wo.pos[s];
-        v = d.wo.vel[s];
+        const GPV g = load_pv(d.wo.pv, s);
+        p = g.p;
+        v = g.v;
         m = d.wo.mass[s];
         rho = d.wo.dens[s];
         fl = d.wo.flags[s];
       }
       d.w.pos[i] = p;
-      d.w.vel[i] = v;
+      d.w.pv[2 * (size_t)i] = p;
+      d.w.pv[2 * (size_t)i + 1] = v;
       d.w.mass[i] = m;
       d.w.dens[i] = rho;
       d.w.flags[i] = fl;

@@ -16,7 +16,6 @@
   for (int _k = 0, _c = (d).nbr_cnt[i]; _k < _c; ++_k)     \
     for (int j = (d).nbr[(size_t)_k * (d).cap + (i)], _o = 1; _o; _o = 0)
 
-struct GPV { real4 p, v; };
 
 // ---------------------------------------------------------------------------
 // compute_static_boundary_volume / compute_moving_boundary_volume (SPH/main.py:1010-1035)
@@ -37,7 +36,7 @@ __global__ void k_boundary_volume(Dev d, int moving) {
                    return w_fluid(pj.w) ? real(0) : kw_r2(dot3(r, r), s);
                  },
                  [&](real w) { delta += w; });
-    if (work && sub == 0) d.w.pos[i].w = -(1.f / delta * 3.f);
+    if (work && sub == 0) d.w.pos[i].w = xyz_of(d, i).w = -(1.f / delta * 3.f);
   }
 }
 
@@ -89,7 +88,7 @@ __global__ void k_density_factor(Dev d, int do_density, int do_factor) {
     const int self = work ? i : 0;
     const real4 pi = d.w.pos[self];
     const real3 xi = f3(pi);
-    const real3 vi = f3(d.w.vel[self]);
+    const real3 vi = f3(vel_of(d, self));
     const int c = work ? d.nbr_cnt[i] : 0;
     real den = 0.f, sum_grad = 0.f, dd = 0.f;
     real3 gpi = make_real3(0.f, 0.f, 0.f);
@@ -112,7 +111,7 @@ __global__ void k_density_factor(Dev d, int do_density, int do_factor) {
       if (CHANGE) dd = fma(t.V, t.dv, dd);
     };
     if constexpr (CHANGE) {
-      nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
+      nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv(d.w.pv, j); },
                    [&](const GPV& g) { return term(g.p, g.v); }, fold);
     } else {
       nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return pos_of(d, j); },
@@ -186,11 +185,11 @@ __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int 
       const SceneDev& s = d.sc[scn];
       const int self = work ? i : 0;
       const real3 xi = f3(d.w.pos[self]);
-      const real3 vi = f3(d.w.vel[self]);
+      const real3 vi = f3(vel_of(d, self));
       const int c = work ? d.nbr_cnt[i] : 0;
       real dd = 0.f;
       if constexpr (!NP) {
-        nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
+        nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv(d.w.pv, j); },
                      [&](const GPV& g) {
                        const real3 r = xi - f3(g.p);
                        return TDiv{fabs(g.p.w), dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s))};
@@ -202,7 +201,7 @@ __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int 
         const real mi = d.w.mass[self];
         real3 st = make_real3(0.f, 0.f, 0.f);
         real S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // strain-rate sum: 00 11 22 01 02 12
-        auto load = [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; };
+        auto load = [&](int j) { return load_pv(d.w.pv, j); };
         auto add_st = [&](real3 b, real sw) { st = make_real3(fma(-b.x, sw, st.x), fma(-b.y, sw, st.y), fma(-b.z, sw, st.z)); };
         auto add_sr = [&](const real (&e)[6], real m) {
 #pragma unroll
@@ -326,9 +325,9 @@ __device__ __forceinline__ void divergence_update_body(const Dev& d) {
                  [&](const GPK& g) { return push_term(xi, g, k_i, dt, s); },
                  [&](const TPush& t) { push_fold(dv, t); });
     if (work && sub == 0) {
-      real4 v = d.w.vel[i];
+      real4 v = vel_of(d, i);
       v.x += dv.x; v.y += dv.y; v.z += dv.z;
-      d.w.vel[i] = v;
+      vel_of(d, i) = v;
     }
   }
 }
@@ -368,10 +367,10 @@ __device__ __forceinline__ void density_adv_body(const Dev& d, int mode) {
       const real dt = d.dyn[scn].dt;
       const int self = work ? i : 0;
       const real3 xi = f3(d.w.pos[self]);
-      const real3 vi = f3(d.w.vel[self]);
+      const real3 vi = f3(vel_of(d, self));
       real delta = 0.f;
       nb_sum<U, L, true>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, self, sub,
-                 [&](int j) { return GPV{pos_of(d, j), ldg(&d.w.vel[j])}; },
+                 [&](int j) { return load_pv(d.w.pv, j); },
                  [&](const GPV& g) {
                    const real3 r = xi - f3(g.p);
                    return TDiv{fabs(g.p.w), dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s))};
@@ -420,12 +419,12 @@ __device__ __forceinline__ void pressure_update_body(const Dev& d) {
     auto load = [&](int j) { return GPK{pos_of(d, j), ldg(&d.kappa[j])}; };
     if (L == 1 ? fluid : __any_sync(0xffffffffu, work && fluid)) {
       const real k_i = d.kappa[self];
-      const real4 v4 = d.w.vel[self];
+      const real4 v4 = vel_of(d, self);
       real3 vi = f3(v4);
       nb_sum<U, L, true>(d.nbr + i, d.cap, fluid ? c : 0, self, sub, load,
                          [&](const GPK& g) { return push_term(xi, g, k_i, dt, s); },
                          [&](const TPush& t) { push_fold(vi, t); });
-      if (work && fluid && sub == 0) d.w.vel[i] = make_real4(vi.x, vi.y, vi.z, v4.w);
+      if (work && fluid && sub == 0) vel_of(d, i) = make_real4(vi.x, vi.y, vi.z, v4.w);
     }
     if (L == 1 ? !fluid : __any_sync(0xffffffffu, work && !fluid)) {
       const real Vi = fabs(pi.w);
@@ -544,9 +543,9 @@ __global__ void k_np_advect(Dev d) {
     if (!cls_fluid(fl) || !(fl & NN_CLS_DYNAMIC)) continue;
     const real dt = d.dyn[slot_scene(fl)].dt;
     const real4 a = d.acc4[i];
-    real4 v = d.w.vel[i];
+    real4 v = vel_of(d, i);
     v.x += dt * a.x; v.y += dt * a.y; v.z += dt * a.z;
-    d.w.vel[i] = v;
+    vel_of(d, i) = v;
   }
 }
 
@@ -673,7 +672,7 @@ __device__ __forceinline__ void forces_body(const Dev& d, int clear) {
     const int self = work ? i : 0;
     const real4 pi = d.w.pos[self];
     const real3 xi = f3(pi);
-    const real3 vi = f3(d.w.vel[self]);
+    const real3 vi = f3(vel_of(d, self));
     real4 a;
     if (clear) a = cls_static_solid(fl) ? make_real4(0.f, 0.f, 0.f, 0.f) : make_real4(s.g[0], s.g[1], s.g[2], 0.f);
     else a = d.acc4[self];
@@ -687,7 +686,8 @@ __device__ __forceinline__ void forces_body(const Dev& d, int clear) {
       const real Vi = fabs(pi.w);
       const bool need_rho = vi_on || vb_on;  // density and id only where a term reads them
       auto load = [&](int j) {
-        return GF{pos_of(d, j), ldg(&d.w.vel[j]), need_rho ? ldg(&d.w.dens[j]) : 1.f, quirks ? ldg(&d.w.id[j]) : 0};
+        const GPV g = load_pv(d.w.pv, j);
+        return GF{g.p, g.v, need_rho ? ldg(&d.w.dens[j]) : 1.f, quirks ? ldg(&d.w.id[j]) : 0};
       };
       auto term = [&](const GF& g) {
         T t;
@@ -811,15 +811,14 @@ __device__ __forceinline__ bool cg_row(const Dev& d, int i, uint32_t fl) {
 // A p for one row; in the setup also the diagonal block D and the right-hand-side
 // correction of moving boundaries (SETUP: `vec` is the velocity field).
 // The setup gathers a neighbour's pos, v and coefficients (mu_j, m_j / rho_j). It leaves
-// mu_i in p.w and writes cg_pos = (x_i, m_i / rho_i) for fluid and pos = (x_i, -V_i) for
+// mu_i in p.w and writes positions (x_i, m_i / rho_i) for fluid and pos = (x_i, -V_i) for
 // solids, so the matvec reads the same operands in two float4 gathers (32 B per pair)
 // instead of three loads (40 B): the matvec 0.302 -> 0.265 ms on the 2.4M scene.
 struct GCG { real4 p, x; real2 a; };
 struct TMatvec { real x, y, z, c; };                             // grad W, c
 struct TSetup { real x, y, z, c, b, wx, wy, wz, rx, ry, rz; };   // and b of bcorr, c w grad W, r
 template <int U, int L, bool SETUP>
-__device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool work, const real4* __restrict__ vec,
-                                           real3 vi, const SceneDev& s, real dt, real* D, real3* bcorr) {
+__device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool work, real3 vi, const SceneDev& s, real dt, real* D, real3* bcorr) {
   const int self = work ? i : 0;
   const real3 xi = f3(d.w.pos[self]);
   const real2 ai = d.cg_aux[self];
@@ -831,7 +830,10 @@ __device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool wor
   const int cnt = work ? d.nbr_cnt[i] : 0;
   auto add = [&](real3& sum, real3 g, real c) { sum = make_real3(fma(-g.x, c, sum.x), fma(-g.y, c, sum.y), fma(-g.z, c, sum.z)); };
   if constexpr (SETUP) {
-    auto load = [&](int j) { return GCG{pos_of(d, j), ldg(&vec[j]), ldg(&d.cg_aux[j])}; };
+    auto load = [&](int j) {
+      const GPV g = load_pv(d.w.pv, j);
+      return GCG{g.p, g.v, ldg(&d.cg_aux[j])};
+    };
     auto add_diag = [&](real3 wg, real3 r) {
       D[0] = fma(-wg.x, r.x, D[0]); D[1] = fma(-wg.y, r.y, D[1]); D[2] = fma(-wg.z, r.z, D[2]);
       D[3] = fma(-wg.x, r.y, D[3]); D[4] = fma(-wg.x, r.z, D[4]); D[5] = fma(-wg.y, r.z, D[5]);
@@ -884,7 +886,7 @@ __device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool wor
     }
   } else {
     nb_sum<U, L>(d.nbr + i, d.cap, cnt, self, sub,
-                 [&](int j) { return GPV{ldg(&d.cg_pos[j]), ldg(&vec[j])}; },
+                 [&](int j) { return load_pv(d.cg_pp, j); },
                  [&](const GPV& g) {  // fluid j: (mu_j, m_j / rho_j) in v.w, p.w
                    const real3 r = xi - f3(g.p);
                    const real r2 = dot3(r, r);
@@ -920,16 +922,16 @@ __device__ __forceinline__ void cg_setup_body(const Dev& d) {
     const bool work = valid && cg_row(d, i, fl);
     double rr = 0, bb = 0, rz = 0;
     // a solid neighbour's matvec operands: its pos (x, -V); its p is not read
-    if (valid && sub == 0 && cls_solid(fl) && scene_implicit(d.sc[scn])) d.cg_pos[i] = d.w.pos[i];
+    if (valid && sub == 0 && cls_solid(fl) && scene_implicit(d.sc[scn])) d.cg_pp[2 * (size_t)i] = d.w.pos[i];
     if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
       const SceneDev& s = d.sc[scn];
       const real dt = d.dyn[scn].dt;
       const int self = work ? i : 0;
       const real mi = d.w.mass[self];
-      const real3 vi = f3(d.w.vel[self]);
+      const real3 vi = f3(vel_of(d, self));
       real D[6] = {mi, mi, mi, 0.f, 0.f, 0.f};
       real3 bc = make_real3(0.f, 0.f, 0.f);
-      const real3 Av = cg_apply<U, L, true>(d, i, sub, work, d.w.vel, vi, s, dt, D, &bc);
+      const real3 Av = cg_apply<U, L, true>(d, i, sub, work, vi, s, dt, D, &bc);
       if (work && sub == 0) {
         const real3 b = vi * mi + bc;
         // symmetric 3x3 inverse in double
@@ -948,8 +950,8 @@ __device__ __forceinline__ void cg_setup_body(const Dev& d) {
         d.cg_z[i] = make_real4(z.x, z.y, z.z, 0.f);
         const real2 ai = d.cg_aux[i];
         const real3 xi = f3(d.w.pos[i]);
-        d.cg_pos[i] = make_real4(xi.x, xi.y, xi.z, ai.y);
-        d.cg_p[i] = make_real4(z.x, z.y, z.z, ai.x);
+        d.cg_pp[2 * (size_t)i] = make_real4(xi.x, xi.y, xi.z, ai.y);
+        d.cg_pp[2 * (size_t)(i) + 1] = make_real4(z.x, z.y, z.z, ai.x);
         rr = (double)r.x * r.x + (double)r.y * r.y + (double)r.z * r.z;
         bb = (double)b.x * b.x + (double)b.y * b.y + (double)b.z * b.z;
         rz = (double)r.x * z.x + (double)r.y * z.y + (double)r.z * z.z;
@@ -1005,8 +1007,8 @@ __device__ __forceinline__ void cg_matvec_body(const Dev& d) {
     double pap = 0;
     if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
       const SceneDev& s = d.sc[scn];
-      const real3 p = f3(d.cg_p[work ? i : 0]);
-      const real3 Ap = cg_apply<U, L, false>(d, i, sub, work, d.cg_p, p, s, d.dyn[scn].dt, nullptr, nullptr);
+      const real3 p = f3(d.cg_pp[2 * (size_t)(work ? i : 0) + 1]);
+      const real3 Ap = cg_apply<U, L, false>(d, i, sub, work, p, s, d.dyn[scn].dt, nullptr, nullptr);
       if (work && sub == 0) {
         d.cg_Ap[i] = make_real4(Ap.x, Ap.y, Ap.z, 0.f);
         pap = (double)p.x * Ap.x + (double)p.y * Ap.y + (double)p.z * Ap.z;
@@ -1031,7 +1033,7 @@ __global__ void k_cg_update(Dev d) {
     if (work) {
       const real al = (real)d.dyn[scn].cg_alpha;
       real3 x = f3(d.cg_x[i]), r = f3(d.cg_r[i]);
-      const real3 p = f3(d.cg_p[i]), Ap = f3(d.cg_Ap[i]);
+      const real3 p = f3(d.cg_pp[2 * (size_t)(i) + 1]), Ap = f3(d.cg_Ap[i]);
       x += p * al;
       r -= Ap * al;
       real P[6];
@@ -1099,9 +1101,9 @@ __global__ void k_cg_pupdate(Dev d) {
     if (!cg_row(d, i, fl) || !d.dyn[scn].act_cg) continue;
     const real be = (real)d.dyn[scn].cg_beta;
     const real3 z = f3(d.cg_z[i]);
-    const real4 p4 = d.cg_p[i];
+    const real4 p4 = d.cg_pp[2 * (size_t)(i) + 1];
     const real3 np = z + f3(p4) * be;
-    d.cg_p[i] = make_real4(np.x, np.y, np.z, p4.w);  // w: mu_i
+    d.cg_pp[2 * (size_t)(i) + 1] = make_real4(np.x, np.y, np.z, p4.w);  // w: mu_i
   }
 }
 
@@ -1118,7 +1120,7 @@ __global__ void k_cg_finish(Dev d, int advect) {
     if (s.n_fluid == 0) continue;
     const real dt = d.dyn[scn].dt;
     real4 a = d.acc4[i];
-    const real4 v4 = d.w.vel[i];
+    const real4 v4 = vel_of(d, i);
     if (scene_implicit(s)) {
       const real inv_dt = d.dyn[scn].inv_dt;
       const real3 x = f3(d.cg_x[i]);
@@ -1127,7 +1129,7 @@ __global__ void k_cg_finish(Dev d, int advect) {
       a.z += (x.z - v4.z) * inv_dt;
       d.acc4[i] = a;
     }
-    if (advect && (fl & NN_CLS_DYNAMIC)) d.w.vel[i] = make_real4(v4.x + dt * a.x, v4.y + dt * a.y, v4.z + dt * a.z, v4.w);
+    if (advect && (fl & NN_CLS_DYNAMIC)) vel_of(d, i) = make_real4(v4.x + dt * a.x, v4.y + dt * a.y, v4.z + dt * a.z, v4.w);
   }
 }
 
@@ -1318,16 +1320,16 @@ __global__ void k_advect_boundary(Dev d, int do_advect, int do_boundary, int do_
     const bool move = do_anim && (an[0] != 0.f || an[1] != 0.f || an[2] != 0.f);
     if (!(fl & NN_CLS_DYNAMIC)) {
       if (move) {
-        real4 p = d.w.pos[i];
+        real4 p = xyz_of(d, i);
         p.x += an[0]; p.y += an[1]; p.z += an[2];
-        d.w.pos[i] = p;
+        xyz_of(d, i) = p;
       }
       continue;
     }
     const SceneDev& s = d.sc[scn];
     const real dt = d.dyn[scn].dt;
-    real4 p = d.w.pos[i];
-    real4 v = d.w.vel[i];
+    real4 p = xyz_of(d, i);
+    real4 v = vel_of(d, i);
     if (do_advect) {
       if (cls_dyn_solid(fl)) {
         const real4 a = d.acc4[i];
@@ -1356,8 +1358,8 @@ __global__ void k_advect_boundary(Dev d, int do_advect, int do_boundary, int do_
     }
     if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(v.x) && isfinite(v.y) && isfinite(v.z)))
       set_status(&d.dyn[scn], NN_ERR_NAN);
-    d.w.pos[i] = p;
-    d.w.vel[i] = v;
+    xyz_of(d, i) = p;
+    vel_of(d, i) = v;
   }
 }
 
@@ -1370,9 +1372,9 @@ __global__ void k_sync_out(Dev d, uint32_t mask) {
   const int n = d.d_n[0];
   GRID_STRIDE(id, n) {
     const int i = d.slot_of_id[id];
-    const real4 p = d.w.pos[i];
+    const real4 p = xyz_of(d, i);
     if (mask & 1u) { d.t.x[3 * id] = p.x; d.t.x[3 * id + 1] = p.y; d.t.x[3 * id + 2] = p.z; }
-    if (mask & 2u) { const real4 v = d.w.vel[i]; d.t.v[3 * id] = v.x; d.t.v[3 * id + 1] = v.y; d.t.v[3 * id + 2] = v.z; }
+    if (mask & 2u) { const real4 v = vel_of(d, i); d.t.v[3 * id] = v.x; d.t.v[3 * id + 1] = v.y; d.t.v[3 * id + 2] = v.z; }
     if (mask & 4u) { const real4 a = d.acc4[i]; d.t.a[3 * id] = a.x; d.t.a[3 * id + 1] = a.y; d.t.a[3 * id + 2] = a.z; }
     if (mask & 8u) d.t.volume[id] = fabs(p.w);
     if (mask & 16u) d.t.density[id] = d.w.dens[i];
@@ -1399,14 +1401,14 @@ __global__ void k_sync_in(Dev d, uint32_t mask) {
   const int n = d.d_n[0];
   GRID_STRIDE(i, n) {
     const int id = d.w.id[i];
-    real4 p = d.w.pos[i];
+    real4 p = xyz_of(d, i);
     if (mask & 1u) { p.x = d.t.x[3 * id]; p.y = d.t.x[3 * id + 1]; p.z = d.t.x[3 * id + 2]; }
     if (mask & 8u) p.w = cls_solid(d.w.flags[i]) ? -d.t.volume[id] : d.t.volume[id];
-    d.w.pos[i] = p;
+    d.w.pos[i] = xyz_of(d, i) = p;
     real m = d.w.mass[i];  // vel.w carries the mass
     if (mask & 256u) { m = d.t.m[id]; d.w.mass[i] = m; }
-    if (mask & 2u) d.w.vel[i] = make_real4(d.t.v[3 * id], d.t.v[3 * id + 1], d.t.v[3 * id + 2], m);
-    else if (mask & 256u) d.w.vel[i].w = m;
+    if (mask & 2u) vel_of(d, i) = make_real4(d.t.v[3 * id], d.t.v[3 * id + 1], d.t.v[3 * id + 2], m);
+    else if (mask & 256u) vel_of(d, i).w = m;
     if (mask & 4u) d.acc4[i] = make_real4(d.t.a[3 * id], d.t.a[3 * id + 1], d.t.a[3 * id + 2], 0.f);
     if (mask & 16u) d.w.dens[i] = d.t.density[id];
     if (mask & 32u) d.alpha[i] = d.t.dfsph_factor[id];
@@ -1457,8 +1459,8 @@ __global__ void k_rigid_ground(Dev d, int round, int rep) {
     if (!cls_solid(fl)) continue;
     const SceneDev& s = d.sc[slot_scene(fl)];
     if (!(s.flags & NN_F_RIGID) || round >= s.n_rigid || rep >= s.coupling) continue;
-    real4 p = d.w.pos[i];
-    if (p.y < s.padding) { p.y = s.padding; d.w.pos[i] = p; }
+    real4 p = xyz_of(d, i);
+    if (p.y < s.padding) { p.y = s.padding; xyz_of(d, i) = p; }
   }
 }
 
@@ -1476,7 +1478,7 @@ __global__ void k_rigid_com(Dev d, int round, int rest) {
         const int id = d.w.id[i];
         x = make_real3(d.t.x_0[3 * id], d.t.x_0[3 * id + 1], d.t.x_0[3 * id + 2]);
       } else {
-        x = f3(d.w.pos[i]);
+        x = f3(xyz_of(d, i));
       }
       v[0] = m * x.x; v[1] = m * x.y; v[2] = m * x.z; v[3] = m;
     }
@@ -1505,7 +1507,7 @@ __global__ void k_rigid_A(Dev d, int round) {
       const SceneDev& s = d.sc[slot_scene(d.w.flags[i])];
       const double m = (double)(s.V0 * d.w.dens[i]);
       const int id = d.w.id[i];
-      const real4 x = d.w.pos[i];
+      const real4 x = xyz_of(d, i);
       const double p[3] = {(double)x.x - d.rb_cm[3 * b], (double)x.y - d.rb_cm[3 * b + 1],
                            (double)x.z - d.rb_cm[3 * b + 2]};
       const double q[3] = {(double)d.t.x_0[3 * id] - d.rb_rest[3 * b], (double)d.t.x_0[3 * id + 1] - d.rb_rest[3 * b + 1],
@@ -1545,10 +1547,10 @@ __global__ void k_rigid_apply(Dev d, int round) {
     const double q[3] = {(double)d.t.x_0[3 * id] - d.rb_rest[3 * b], (double)d.t.x_0[3 * id + 1] - d.rb_rest[3 * b + 1],
                          (double)d.t.x_0[3 * id + 2] - d.rb_rest[3 * b + 2]};
     const double* R = &d.rb_R[9 * b];
-    real4 p = d.w.pos[i];
+    real4 p = xyz_of(d, i);
     p.x = (real)(d.rb_cm[3 * b] + R[0] * q[0] + R[1] * q[1] + R[2] * q[2]);
     p.y = (real)(d.rb_cm[3 * b + 1] + R[3] * q[0] + R[4] * q[1] + R[5] * q[2]);
     p.z = (real)(d.rb_cm[3 * b + 2] + R[6] * q[0] + R[7] * q[1] + R[8] * q[2]);
-    d.w.pos[i] = p;
+    xyz_of(d, i) = p;
   }
 }

@@ -41,8 +41,8 @@ class Request:
 
 
 # Device bytes of a resident particle, from what a server allocates per particle of
-# its capacity: the context's two sorted working sets (position+volume 16, velocity+mass
-# 16, mass 4, density 4, flags 4, id 4: 2 x 48), its per-slot scratch (scene of id 4,
+# its capacity: the context's two sorted working sets (position+volume and velocity+mass
+# 32, mass 4, density 4, flags 4, id 4: 2 x 48) and the gathered positions 16, its per-slot scratch (scene of id 4,
 # acceleration 16, alpha / rho_adv / kappa / strain rate / viscosity 20, slot of id 4,
 # sort key / rank / source 12), the neighbour counts 4 and 4 B per list entry, the CG
 # vectors (x, r, z, p, Ap and the matvec's positions: 6 x 16, coefficients 8,
@@ -50,7 +50,7 @@ class Request:
 # the batch's ParticleData fields (168: x, x_0, v, a 48; six scalars 24; four int32 16;
 # color 12; strain rate and viscosity 8; stress 24; rotations 36). A grid cell costs
 # CELL_BYTES (its count / start).
-CTX_BYTES_PER_PARTICLE = 96 + 56 + 4 + 128 + 4
+CTX_BYTES_PER_PARTICLE = 112 + 56 + 4 + 128 + 4
 PD_BYTES_PER_PARTICLE = 168
 CELL_BYTES = 4
 DEFAULT_RESERVE_BYTES = 4 << 30  # left free for torch, graphs and the repack's temporaries
