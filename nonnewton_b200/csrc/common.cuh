@@ -290,13 +290,19 @@ __device__ __forceinline__ void nb_sum(const int32_t* __restrict__ list, int str
     constexpr int P = 32 / L;
     const int p = (int)(threadIdx.x & (P - 1));
     const int cm = __reduce_max_sync(0xffffffffu, c);
-    int q0 = sub < c ? nb_list_load<false>(list + (size_t)sub * stride) : self;
-    int q1 = sub + L < c ? nb_list_load<false>(list + (size_t)(sub + L) * stride) : self;
+    // list entries are loaded three trips ahead of their use and the gathers two, so that a
+    // list of 26 entries at 8 lanes costs little more than one latency of each
+    auto entry = [&](int k) { return k < c ? nb_list_load<false>(list + (size_t)k * stride) : self; };
+    const int j0 = entry(sub), j1 = entry(sub + L);
+    int q = entry(sub + 2 * L);
+    auto g0 = load(j0), g1 = load(j1);
     for (int k = 0; k < cm; k += L) {
-      const int j = q0, kk = k + 2 * L + sub;
-      q0 = q1;
-      q1 = kk < c ? nb_list_load<false>(list + (size_t)kk * stride) : self;
-      const auto t = term(load(j));
+      const int j = q;
+      q = entry(k + 3 * L + sub);
+      const auto g = g0;
+      g0 = g1;
+      g1 = load(j);
+      const auto t = term(g);
 #pragma unroll
       for (int e = 0; e < L; ++e) {
         const auto u = shfl_reals(t, e * P + p);
@@ -393,17 +399,72 @@ __device__ __forceinline__ bool scene_implicit(const SceneDev& s) {
   return (s.flags & NN_F_IMPLICIT_VISCOSITY) && !(s.flags & NN_F_QUIRKS);
 }
 
-__device__ __forceinline__ double acc_sum(const double* acc, int scene, int quantity) {
-  const double* a = &acc[((size_t)scene * ACC_COUNT + quantity) * NN_STRIPES];
-  double s = 0.0;
+// A quantity's striped accumulators summed and cleared, by a whole warp (one lane per
+// stripe): every lane gets the sum.
+static_assert(NN_STRIPES == 32, "one lane per stripe");
+__device__ __forceinline__ double acc_take(double* acc, int scene, int quantity) {
+  double* a = &acc[((size_t)scene * ACC_COUNT + quantity) * NN_STRIPES + (threadIdx.x & 31)];
+  double v = __ldcg(a);  // written by atomics
+  *a = 0.0;
 #pragma unroll
-  for (int k = 0; k < NN_STRIPES; ++k) s += a[k];
-  return s;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
-__device__ __forceinline__ void acc_zero(double* acc, int scene, int quantity) {
-  double* a = &acc[((size_t)scene * ACC_COUNT + quantity) * NN_STRIPES];
-#pragma unroll
-  for (int k = 0; k < NN_STRIPES; ++k) a[k] = 0.0;
+
+// Barrier over the blocks of a cooperative launch (all resident). The last block to arrive
+// runs `last` before it lets the others go, so that the control of a solver loop costs no
+// barrier of its own. A wait that runs out (which a resident grid cannot cause) marks the
+// barrier failed; every block then leaves the kernel, and the step reports it.
+// The counter and the generation lie in lines of their own: the polls of a thousand waiting
+// blocks would queue up before the arrivals.
+struct GridBarrier { unsigned arrived, pad0[31], gen, pad1[31]; int fail, pad2[31]; };
+#define NN_BARRIER_POLLS (1u << 24)  // seconds
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned add_acq_rel(unsigned* p, unsigned v) {
+  unsigned old;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+// `gen`: the barrier's generation, read once by grid_gen before the block's first barrier
+// and counted on by each barrier (only thread 0's copy is used).
+__device__ __forceinline__ unsigned grid_gen(GridBarrier* b) { return threadIdx.x == 0 ? ld_acquire(&b->gen) : 0u; }
+template <typename F>
+__device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned& gen, F last) {
+  __shared__ int sh_last, sh_fail;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sh_last = add_acq_rel(&b->arrived, 1u) == gridDim.x - 1;
+    sh_fail = 0;
+  }
+  __syncthreads();
+  if (sh_last) {
+    last();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      b->arrived = 0u;
+      st_release(&b->gen, gen + 1u);
+    }
+  } else if (threadIdx.x == 0) {
+    unsigned polls = 0;
+    while (ld_acquire(&b->gen) == gen) {
+      if (++polls > NN_BARRIER_POLLS || ((polls & 1023u) == 0u && *(volatile int*)&b->fail)) {
+        atomicExch(&b->fail, 1);
+        sh_fail = 1;
+        break;
+      }
+      __nanosleep(40);
+    }
+  }
+  ++gen;
+  __syncthreads();
+  return sh_fail == 0;
 }
 
 // Rotation of the polar decomposition (semantics of ti.polar_decompose used at

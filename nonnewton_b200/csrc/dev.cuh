@@ -81,17 +81,32 @@ struct Dev {
   int32_t* any_active;         // host-visible flag of the last check
   unsigned long long loop_handle; // cudaGraphConditionalHandle (0 when not in a graph)
   int32_t* body_count;         // [4] executed loop bodies (div, pressure, cg, elastic)
+  GridBarrier* bar;            // barrier of the one-kernel loops
 };
 
 // The pair of float4 of a slot, position and velocity (or the matvec's), in one 256-bit
 // load (ld.global.nc.v8.f32): one request and one sector per neighbour, where two float4
 // gathers took two requests that each used half of theirs.
+// COH: coherently, where the same kernel writes the array on the other side of a grid barrier.
+template <bool COH, typename T>
+__device__ __forceinline__ T nb_load(const T* p) {
+  if constexpr (COH) return *p;
+  else return ldg(p);
+}
 struct GPV { real4 p, v; };
+template <bool COH = false>
 __device__ __forceinline__ GPV load_pv(const real4* pv, int j) {
   const real4* q = pv + 2 * (size_t)j;
 #ifdef NN_FP64
-  return GPV{ldg(q), ldg(q + 1)};
+  return GPV{nb_load<COH>(q), nb_load<COH>(q + 1)};
 #else
+  if constexpr (COH) {
+    GPV g;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(g.p.x), "=f"(g.p.y), "=f"(g.p.z), "=f"(g.p.w), "=f"(g.v.x), "=f"(g.v.y), "=f"(g.v.z), "=f"(g.v.w)
+        : "l"(q));  // volatile: stays on its side of the barriers' own asm
+    return g;
+  }
   GPV g;
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=f"(g.p.x), "=f"(g.p.y), "=f"(g.p.z), "=f"(g.p.w), "=f"(g.v.x), "=f"(g.v.y), "=f"(g.v.z), "=f"(g.v.w)

@@ -48,6 +48,8 @@ cudaError_t dalloc(T** p, size_t count) {
 #define NN_DEFAULT_UNROLL 0
 #define NN_DEFAULT_XSPLIT 2  // 2.4M scene: list build 0.66 -> 0.60 ms, step -0.7 % (x split 3 and 4: slower steps)
 
+#define NN_CG_LOOP_MAX 250000  // slots; see one_kernel_cg
+
 struct nn_ctx {
   int cap = 0, max_scenes = 0, max_nb = 0;
   int64_t max_cells = 0;
@@ -104,6 +106,7 @@ struct nn_ctx {
   int32_t* h_any = nullptr;            // pinned
   cudaEvent_t status_ev = nullptr;     // recorded after nn_status_async's copy
   int32_t* d_body = nullptr;
+  GridBarrier* d_bar = nullptr;
   int64_t fixed_nodes_per_step = 0;    // kernel nodes outside loop bodies (graph mode)
   int64_t graph_replays = 0;
   int64_t body_nodes[3] = {3, 3, 5};   // kernels per loop body: divergence, pressure, CG
@@ -121,7 +124,8 @@ static uint64_t feature_sig(const nn_ctx* c) {
   return (uint64_t)c->any_fluid | ((uint64_t)c->any_div << 1) | ((uint64_t)c->any_nonnewton << 2) |
          ((uint64_t)c->any_implicit << 3) | ((uint64_t)std::min(c->el_mult_max, 255) << 8) |
          ((uint64_t)(c->ne > 0) << 16) | ((uint64_t)c->block << 20) |
-         ((uint64_t)c->forces_feat << 40) | ((uint64_t)c->fold_np << 48) | ((uint64_t)c->lanes << 52);
+         ((uint64_t)c->forces_feat << 40) | ((uint64_t)c->fold_np << 48) | ((uint64_t)c->lanes << 52) |
+         ((uint64_t)(c->n <= NN_CG_LOOP_MAX) << 56);
 }
 
 // Lanes per particle of the neighbour passes (nb_sum), by the fluid particles they walk. A
@@ -196,6 +200,7 @@ static Dev make_dev(nn_ctx* c, int cur) {
   d.any_active = c->d_any;
   d.loop_handle = c->cur_handle;
   d.body_count = c->d_body;
+  d.bar = c->d_bar;
   return d;
 }
 
@@ -234,6 +239,31 @@ static int launch(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, int
 template <typename... KArgs, typename... Args>
 static int launch_nb(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, Args... args) {
   return launch_lanes(c, s, k, block, c->n, c->lanes, args...);
+}
+// A one-kernel loop: a cooperative launch, at most as many blocks as are resident at once
+// (capture records the launch attribute).
+template <typename... KArgs, typename... Args>
+static int launch_loop(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), Args... args) {
+  auto it = c->occ.find((const void*)k);
+  if (it == c->occ.end()) {
+    int per_sm = 1;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NN_SOLVE_BLOCK, 0));
+    it = c->occ.emplace((const void*)k, std::max(per_sm, 1)).first;
+  }
+  const int64_t want = ((int64_t)std::max(c->n, 1) * c->lanes + NN_SOLVE_BLOCK - 1) / NN_SOLVE_BLOCK;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)std::min<int64_t>(want, (int64_t)c->sms * it->second));
+  cfg.blockDim = dim3(NN_SOLVE_BLOCK);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, k, args...));
+  if (c->in_capture) c->capture_nodes++;
+  else c->launches++;
+  return NN_OK;
 }
 template <typename... KArgs, typename... Args>
 static int launch1(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), Args... args) {
@@ -398,6 +428,24 @@ static int enq_search(nn_ctx* c, cudaStream_t s, bool reset_step = false) {
   return NN_OK;
 }
 
+// The captured step runs a solver loop as one cooperative kernel (k_divergence_loop and its
+// neighbours) where its passes are short: the divergence and density loops in the scenes
+// that split a particle over lanes, the viscosity's, whose while-node costs most (19 us
+// before its first body), up to NN_CG_LOOP_MAX slots. Above, the passes run slower as parts
+// of such a kernel than the nodes cost. Step times, while-nodes / divergence loop / CG loop /
+// density loop / all in one kernel (us): 3,933 slots 178 / 163 / - / 162 / 152; 23,002 176 /
+// 170 / - / 170 / 165; 24k fluid at 4 lanes 315 / 311 / 298 / 303 / 281; 39k at 2 lanes 358 /
+// 365 / 352 / 360 / 349; 85,147 at 1 lane 441 / 457 / 434 / 453 / 451; 135,201 360 / 363 /
+// 347 / 361 / 343; 175,870 759 / 799 / 751 / 775 / 783; 616,732 1181 / 1239 / 1184 / 1223 /
+// 1282. Host-driven loops (one synchronisation per body) keep separate kernels.
+static bool one_kernel_loops(const nn_ctx* c) { return c->in_capture && c->lanes > 1; }
+static bool one_kernel_cg(const nn_ctx* c) {
+  return c->in_capture && c->unroll == 0 && (c->lanes > 1 || c->n <= NN_CG_LOOP_MAX);
+}
+#define KL_(k, ...) (c->lanes == 8 ? &k<8 __VA_ARGS__> : c->lanes == 4 ? &k<4 __VA_ARGS__> : &k<2 __VA_ARGS__>)
+#define KL(k) KL_(k)
+#define KL2(k, B) KL_(k, COMMA B)
+
 // DFSPHSolver.divergence_solve (SPH/main.py:1683-1713). In the fused step the first
 // density change and alpha *= 1/dt were done by k_density_factor<CHANGE> and the
 // closing alpha *= dt is folded into the pressure solve's first pass (fused = true);
@@ -406,6 +454,10 @@ static int enq_divergence(nn_ctx* c, cudaStream_t s, bool fused) {
   Dev d = make_dev(c, c->cur);
   const int B = c->block;
   const bool np = fused && c->fold_np;
+  if (fused && one_kernel_loops(c)) {
+    if (np) return launch_loop(c, s, KL2(k_divergence_loop, true), d);
+    return launch_loop(c, s, KL2(k_divergence_loop, false), d);
+  }
   if (!fused) RC(launch1(c, s, k_solver_begin, d, 0));
   RC(solver_loop(c, s, false,
                  [&](cudaStream_t q) {
@@ -428,6 +480,10 @@ static int enq_pressure(nn_ctx* c, cudaStream_t s, int init_mode, bool begun = f
   Dev d = make_dev(c, c->cur);
   const int B = c->block;
   if (!begun) RC(launch1(c, s, k_solver_begin, d, 1));
+  if (one_kernel_loops(c)) {
+    RC(launch_nb(c, s, KU(k_density_adv, U_DENSITY_ADV), B, d, init_mode));
+    return launch_loop(c, s, KL(k_pressure_loop), d);
+  }
   return solver_loop(c, s, false,
                      [&](cudaStream_t q) {
                        return launch_nb(c, q, KU(k_density_adv, U_DENSITY_ADV), B, make_dev(c, c->cur), init_mode);
@@ -450,15 +506,20 @@ static int enq_nonpressure(nn_ctx* c, cudaStream_t s, int advect, int clear) {
   RC(launch_nb(c, s, forces_kernel(c), B, d, clear));
   if (c->any_implicit) {
     RC(launch_nb(c, s, KU(k_cg_setup, U_CG_SETUP), B, d));
-    RC(solver_loop(c, s, true, [&](cudaStream_t q) { return launch1(c, q, k_cg_check0, make_dev(c, c->cur)); },
-                   [&](cudaStream_t q) {
-                     Dev e = make_dev(c, c->cur);
-                     RC(launch_nb(c, q, KU(k_cg_matvec, U_CG_MATVEC), B, e));
-                     RC(launch1(c, q, k_cg_alpha, e));
-                     RC(launch(c, q, k_cg_update, 256, c->n, e));
-                     RC(launch1(c, q, k_cg_check, e));
-                     return launch(c, q, k_cg_pupdate, 256, c->n, e);
-                   }));
+    if (one_kernel_cg(c)) {
+      RC(launch1(c, s, k_cg_check0, d));
+      RC(launch_loop(c, s, c->lanes == 1 ? &k_cg_loop<1> : KL(k_cg_loop), d));
+    } else {
+      RC(solver_loop(c, s, true, [&](cudaStream_t q) { return launch1(c, q, k_cg_check0, make_dev(c, c->cur)); },
+                     [&](cudaStream_t q) {
+                       Dev e = make_dev(c, c->cur);
+                       RC(launch_nb(c, q, KU(k_cg_matvec, U_CG_MATVEC), B, e));
+                       RC(launch1(c, q, k_cg_alpha, e));
+                       RC(launch(c, q, k_cg_update, 256, c->n, e));
+                       RC(launch1(c, q, k_cg_check, e));
+                       return launch(c, q, k_cg_pupdate, 256, c->n, e);
+                     }));
+    }
   }
   if (c->any_implicit || advect) RC(launch(c, s, k_cg_finish, 256, c->n, d, advect));
   return NN_OK;
@@ -738,12 +799,13 @@ int nn_ctx_create(int32_t max_particles, int32_t max_scenes, int32_t max_neighbo
   AL(c->cg_x, N); AL(c->cg_r, N); AL(c->cg_z, N); AL(c->cg_pp, 2 * N); AL(c->cg_Ap, N); AL(c->cg_aux, N);
   AL(c->cg_pinv, 6 * N);
   AL(c->e_of_id, N);
-  AL(c->d_any, 1); AL(c->d_body, 4);
+  AL(c->d_any, 1); AL(c->d_body, 4); AL(c->d_bar, 1);
 #undef AL
   if (cudaMallocHost((void**)&c->h_any, sizeof(int32_t)) != cudaSuccess)
     return bail(fail(nullptr, NN_ERR_OOM, "cudaMallocHost failed"));
   cudaMemset(c->d_acc, 0, (size_t)max_scenes * ACC_COUNT * NN_STRIPES * sizeof(double));
   cudaMemset(c->d_body, 0, 4 * sizeof(int32_t));
+  cudaMemset(c->d_bar, 0, sizeof(GridBarrier));
   cudaMemset(c->d_n, 0, 4 * sizeof(int32_t));
   cudaMemset(c->nbr_cnt, 0, N * sizeof(int32_t));
   if (cudaStreamCreateWithFlags(&c->side, cudaStreamDefault) != cudaSuccess ||
@@ -771,7 +833,7 @@ int nn_ctx_destroy(nn_ctx* c) {
   void* bufs[] = {c->set[0].pos, c->d_n, c->d_sc, c->d_dyn, c->d_acc, c->d_scene_of_id, c->d_src_flag, c->acc4, c->alpha,
                   c->rho_adv, c->kappa, c->srn, c->mu, c->slot_of_id, c->key, c->rank, c->src, c->nbr,
                   c->nbr_cnt, c->cg_x, c->cg_r, c->cg_z, c->cg_pp, c->cg_Ap, c->cg_aux, c->cg_pinv,
-                  c->e_of_id, c->d_any, c->d_body, c->cell_count, c->tile_sums};
+                  c->e_of_id, c->d_any, c->d_body, c->d_bar, c->cell_count, c->tile_sums};
   for (void* b : bufs) cudaFree(b);
   free_elastic(c);
   cudaFree(c->rb_of_id); cudaFree(c->rb_round); cudaFree(c->rb_acc); cudaFree(c->rb_rest); cudaFree(c->rb_cm);
@@ -995,6 +1057,7 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
   int32_t hn[4] = {n, nscenes, (int)cells, c->ne};
   CK(cudaMemcpy(c->d_n, hn, sizeof(hn), cudaMemcpyHostToDevice));
   CK(cudaMemset(c->d_acc, 0, (size_t)c->max_scenes * ACC_COUNT * NN_STRIPES * sizeof(double)));
+  CK(cudaMemset(c->d_bar, 0, sizeof(GridBarrier)));
   // rigid bodies ("r-space")
   cudaFree(c->rb_of_id); cudaFree(c->rb_round); cudaFree(c->rb_acc); cudaFree(c->rb_rest); cudaFree(c->rb_cm);
   cudaFree(c->rb_R);

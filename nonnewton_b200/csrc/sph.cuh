@@ -171,7 +171,7 @@ __device__ __forceinline__ void strain_term(real3 v, real3 g, real (&e)[6]) {
 struct TDiv { real V, dv; };  // volume, v_ij . grad W
 // with the non-pressure terms: surface tension (sx, sy, sz) * sw and strain rate e * m
 struct TDivNp { real V, dv, sx, sy, sz, sw, m, e[6]; };
-template <int U, int L, bool NP>
+template <int U, int L, bool NP, bool COH = false>
 __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int sel) {
   const int n = d.d_n[0];
   FOR_SPLIT(L, i, sub, valid, n) {
@@ -189,7 +189,7 @@ __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int 
       const int c = work ? d.nbr_cnt[i] : 0;
       real dd = 0.f;
       if constexpr (!NP) {
-        nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv(d.w.pv, j); },
+        nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv<COH>(d.w.pv, j); },
                      [&](const GPV& g) {
                        const real3 r = xi - f3(g.p);
                        return TDiv{fabs(g.p.w), dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s))};
@@ -201,7 +201,7 @@ __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int 
         const real mi = d.w.mass[self];
         real3 st = make_real3(0.f, 0.f, 0.f);
         real S[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // strain-rate sum: 00 11 22 01 02 12
-        auto load = [&](int j) { return load_pv(d.w.pv, j); };
+        auto load = [&](int j) { return load_pv<COH>(d.w.pv, j); };
         auto add_st = [&](real3 b, real sw) { st = make_real3(fma(-b.x, sw, st.x), fma(-b.y, sw, st.y), fma(-b.z, sw, st.z)); };
         auto add_sr = [&](const real (&e)[6], real m) {
 #pragma unroll
@@ -306,7 +306,7 @@ __device__ __forceinline__ TPush push_term(real3 xi, const GPK& g, real k_i, rea
 __device__ __forceinline__ void push_fold(real3& v, const TPush& t) {
   v = make_real3(fma(t.x, t.c, v.x), fma(t.y, t.c, v.y), fma(t.z, t.c, v.z));
 }
-template <int U, int L>
+template <int U, int L, bool COH = false>
 __device__ __forceinline__ void divergence_update_body(const Dev& d) {
   const int n = d.d_n[0];
   FOR_SPLIT(L, i, sub, valid, n) {
@@ -321,7 +321,7 @@ __device__ __forceinline__ void divergence_update_body(const Dev& d) {
     const real k_i = d.kappa[self];
     real3 dv = make_real3(0.f, 0.f, 0.f);
     nb_sum<U, L>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, self, sub,
-                 [&](int j) { return GPK{pos_of(d, j), ldg(&d.kappa[j])}; },
+                 [&](int j) { return GPK{pos_of(d, j), nb_load<COH>(&d.kappa[j])}; },
                  [&](const GPK& g) { return push_term(xi, g, k_i, dt, s); },
                  [&](const TPush& t) { push_fold(dv, t); });
     if (work && sub == 0) {
@@ -352,7 +352,7 @@ __global__ void k_alpha_times_dt(Dev d) {
 // (nb_batches<U, true>) and the list build writes them streaming: -2 % here and
 // -10 % in k_pressure_update, the step 3.475 -> 3.435 ms on the 2.4M scene (the other
 // passes measured flat or slower with it).
-template <int U, int L>
+template <int U, int L, bool COH = false>
 __device__ __forceinline__ void density_adv_body(const Dev& d, int mode) {
   const int n = d.d_n[0];
   LaneSums<1> sums;
@@ -370,7 +370,7 @@ __device__ __forceinline__ void density_adv_body(const Dev& d, int mode) {
       const real3 vi = f3(vel_of(d, self));
       real delta = 0.f;
       nb_sum<U, L, true>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, self, sub,
-                 [&](int j) { return load_pv(d.w.pv, j); },
+                 [&](int j) { return load_pv<COH>(d.w.pv, j); },
                  [&](const GPV& g) {
                    const real3 r = xi - f3(g.p);
                    return TDiv{fabs(g.p.w), dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s))};
@@ -401,7 +401,7 @@ __global__ void NN_PASS_REGS k_density_adv(Dev d, int mode) { density_adv_body<U
 // pressure_solve_iteration_kernel (SPH/main.py:1799-1841). Fluid slots update v in
 // place per neighbour; dynamic solid slots gather the two-way coupling acceleration
 // from their fluid neighbours (the reference scatters it with atomics, 1835-1841).
-template <int U, int L>
+template <int U, int L, bool COH = false>
 __device__ __forceinline__ void pressure_update_body(const Dev& d) {
   const int n = d.d_n[0];
   FOR_SPLIT(L, i, sub, valid, n) {
@@ -416,7 +416,7 @@ __device__ __forceinline__ void pressure_update_body(const Dev& d) {
     const real4 pi = d.w.pos[self];
     const real3 xi = f3(pi);
     const int c = work ? d.nbr_cnt[i] : 0;
-    auto load = [&](int j) { return GPK{pos_of(d, j), ldg(&d.kappa[j])}; };
+    auto load = [&](int j) { return GPK{pos_of(d, j), nb_load<COH>(&d.kappa[j])}; };
     if (L == 1 ? fluid : __any_sync(0xffffffffu, work && fluid)) {
       const real k_i = d.kappa[self];
       const real4 v4 = vel_of(d, self);
@@ -454,45 +454,55 @@ __global__ void NN_PASS_REGS k_pressure_update(Dev d) { pressure_update_body<U, 
 // CUDA graph while-condition (any scene still iterating).
 // `fold`: the divergence loop runs the non-pressure terms in body np_body (k_density_change
 // NP); when a scene stops, its terms are fresh if that body was its last.
-__global__ void k_solver_check(Dev d, int which /*0 div, 1 pressure*/, int fold) {
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
-  const int ns = d.d_n[1];
-  for (int sc = threadIdx.x; sc < ns; sc += blockDim.x) {
-    SceneDyn& y = d.dyn[sc];
-    const SceneDev& s = d.sc[sc];
+// One warp per scene; returns (to every thread of the block) whether a scene goes on.
+__device__ __forceinline__ int solver_check_scenes(const int32_t* d_n, const SceneDev* scenes, SceneDyn* dyn, double* acc,
+                                                   int which /*0 div, 1 pressure*/, int fold) {
+  const int ns = d_n[1];
+  int any = 0;
+  for (int sc = threadIdx.x >> 5; sc < ns; sc += blockDim.x >> 5) {
+    SceneDyn& y = dyn[sc];
+    const SceneDev& s = scenes[sc];
     int* act = which == 0 ? &y.act_v : &y.act_p;
     if (!*act) continue;
-    double err = acc_sum(d.acc, sc, ACC_ERR);
-    acc_zero(d.acc, sc, ACC_ERR);
-    double avg = err / (double)s.n_fluid;
-    double eta = which == 0 ? (1.0 / (double)y.dt) * s.eta_v_fac : s.eta_p;
-    int* it = which == 0 ? &y.it_v : &y.it_p;
-    const int body = *it;  // 0-based index of the body that just ran
-    int mx = which == 0 ? s.max_iter_v : s.max_iter;
-    if (which == 0) y.avg_v = avg; else y.avg_p = avg;
-    if (avg <= eta) {
-      *act = 0;
-    } else {
-      *it += 1;
-      if (*it >= max(mx, 1)) *act = 0;
+    const double err = acc_take(acc, sc, ACC_ERR);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+      const double avg = err / (double)s.n_fluid;
+      const double eta = which == 0 ? (1.0 / (double)y.dt) * s.eta_v_fac : s.eta_p;
+      int* it = which == 0 ? &y.it_v : &y.it_p;
+      const int body = *it;  // 0-based index of the body that just ran
+      const int mx = which == 0 ? s.max_iter_v : s.max_iter;
+      int on = 1;
+      if (which == 0) y.avg_v = avg; else y.avg_p = avg;
+      if (avg <= eta) {
+        on = 0;
+      } else {
+        *it += 1;
+        if (*it >= max(mx, 1)) on = 0;
+      }
+      if (!(avg == avg)) { set_status(&y, NN_ERR_NAN); on = 0; }
+      if (!on) *act = 0;
+      if (which == 0 && !on) {
+        y.np_last = body;
+        y.np_fresh = fold && body == y.np_body;
+      }
+      any |= on;
     }
-    if (!(avg == avg)) { set_status(&y, NN_ERR_NAN); *act = 0; }
-    if (which == 0 && !*act) {
-      y.np_last = body;
-      y.np_fresh = fold && body == y.np_body;
-    }
-    if (*act) any = 1;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *d.any_active = any;
-    atomicAdd(&d.body_count[which], 1);
+  return __syncthreads_or(any);
+}
+// The loop's condition: for the host (and the blocks of a one-kernel solve), the body
+// count, and the CUDA graph while-node's.
+__device__ __forceinline__ void loop_decide(const Dev& d, int any, int body) {
+  if (threadIdx.x != 0) return;
+  *d.any_active = any;
+  if (d.body_count && body >= 0) atomicAdd(&d.body_count[body], 1);
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
-    if (d.loop_handle) cudaGraphSetConditional((cudaGraphConditionalHandle)d.loop_handle, any ? 1u : 0u);
+  if (d.loop_handle) cudaGraphSetConditional((cudaGraphConditionalHandle)d.loop_handle, any ? 1u : 0u);
 #endif
-  }
+}
+__global__ void k_solver_check(Dev d, int which, int fold) {
+  loop_decide(d, solver_check_scenes(d.d_n, d.sc, d.dyn, d.acc, which, fold), which);
 }
 
 // Per-scene loop start: which scenes iterate, counters reset.
@@ -817,7 +827,7 @@ __device__ __forceinline__ bool cg_row(const Dev& d, int i, uint32_t fl) {
 struct GCG { real4 p, x; real2 a; };
 struct TMatvec { real x, y, z, c; };                             // grad W, c
 struct TSetup { real x, y, z, c, b, wx, wy, wz, rx, ry, rz; };   // and b of bcorr, c w grad W, r
-template <int U, int L, bool SETUP>
+template <int U, int L, bool SETUP, bool COH = false>
 __device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool work, real3 vi, const SceneDev& s, real dt, real* D, real3* bcorr) {
   const int self = work ? i : 0;
   const real3 xi = f3(d.w.pos[self]);
@@ -886,7 +896,7 @@ __device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool wor
     }
   } else {
     nb_sum<U, L>(d.nbr + i, d.cap, cnt, self, sub,
-                 [&](int j) { return load_pv(d.cg_pp, j); },
+                 [&](int j) { return load_pv<COH>(d.cg_pp, j); },
                  [&](const GPV& g) {  // fluid j: (mu_j, m_j / rho_j) in v.w, p.w
                    const real3 r = xi - f3(g.p);
                    const real r2 = dot3(r, r);
@@ -968,34 +978,28 @@ template <int U, int L>
 __global__ void NN_REGS64 k_cg_setup(Dev d) { cg_setup_body<U, L>(d); }
 
 // After setup: relative residual of the initial guess decides whether to iterate.
-__global__ void k_cg_check0(Dev d) {
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
+__device__ __forceinline__ int cg_check0_scenes(const Dev& d) {
   const int ns = d.d_n[1];
-  for (int sc = threadIdx.x; sc < ns; sc += blockDim.x) {
+  int any = 0;
+  for (int sc = threadIdx.x >> 5; sc < ns; sc += blockDim.x >> 5) {
     SceneDyn& y = d.dyn[sc];
     const SceneDev& s = d.sc[sc];
-    const bool on = s.n_fluid > 0 && scene_implicit(s);
-    double rr = acc_sum(d.acc, sc, ACC_RR), bb = acc_sum(d.acc, sc, ACC_BB), rz = acc_sum(d.acc, sc, ACC_RZ);
-    acc_zero(d.acc, sc, ACC_RR); acc_zero(d.acc, sc, ACC_BB); acc_zero(d.acc, sc, ACC_RZ);
-    y.it_cg = 0;
-    y.cg_bnorm2 = bb;
-    y.cg_rz = rz;
-    y.cg_rel = bb > 0 ? sqrt(rr / bb) : 0.0;
-    y.act_cg = on && (y.cg_rel > s.visco_tol) && s.visco_max_iter > 0;
-    if (y.act_cg) any = 1;
+    const double rr = acc_take(d.acc, sc, ACC_RR), bb = acc_take(d.acc, sc, ACC_BB), rz = acc_take(d.acc, sc, ACC_RZ);
+    if ((threadIdx.x & 31) == 0) {
+      const bool on = s.n_fluid > 0 && scene_implicit(s);
+      y.it_cg = 0;
+      y.cg_bnorm2 = bb;
+      y.cg_rz = rz;
+      y.cg_rel = bb > 0 ? sqrt(rr / bb) : 0.0;
+      y.act_cg = on && (y.cg_rel > s.visco_tol) && s.visco_max_iter > 0;
+      any |= y.act_cg;
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *d.any_active = any;
-#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
-    if (d.loop_handle) cudaGraphSetConditional((cudaGraphConditionalHandle)d.loop_handle, any ? 1u : 0u);
-#endif
-  }
+  return __syncthreads_or(any);
 }
+__global__ void k_cg_check0(Dev d) { loop_decide(d, cg_check0_scenes(d), -1); }
 
-template <int U, int L>
+template <int U, int L, bool COH = false>
 __device__ __forceinline__ void cg_matvec_body(const Dev& d) {
   const int n = d.d_n[0];
   LaneSums<1> sums;
@@ -1008,7 +1012,7 @@ __device__ __forceinline__ void cg_matvec_body(const Dev& d) {
     if (L == 1 ? work : __any_sync(0xffffffffu, work)) {
       const SceneDev& s = d.sc[scn];
       const real3 p = f3(d.cg_pp[2 * (size_t)(work ? i : 0) + 1]);
-      const real3 Ap = cg_apply<U, L, false>(d, i, sub, work, p, s, d.dyn[scn].dt, nullptr, nullptr);
+      const real3 Ap = cg_apply<U, L, false, COH>(d, i, sub, work, p, s, d.dyn[scn].dt, nullptr, nullptr);
       if (work && sub == 0) {
         d.cg_Ap[i] = make_real4(Ap.x, Ap.y, Ap.z, 0.f);
         pap = (double)p.x * Ap.x + (double)p.y * Ap.y + (double)p.z * Ap.z;
@@ -1021,7 +1025,7 @@ __device__ __forceinline__ void cg_matvec_body(const Dev& d) {
 template <int U, int L>
 __global__ void NN_REGS64 k_cg_matvec(Dev d) { cg_matvec_body<U, L>(d); }
 
-__global__ void k_cg_update(Dev d) {
+__device__ __forceinline__ void cg_update_body(const Dev& d) {
   const int n = d.d_n[0];
   LaneSums<2> sums;
   const int q[2] = {ACC_RR, ACC_RZ};
@@ -1050,62 +1054,57 @@ __global__ void k_cg_update(Dev d) {
   }
   sums.flush(d.acc, q);
 }
+__global__ void k_cg_update(Dev d) { cg_update_body(d); }
 
 // PCG step length per scene: alpha = (r.z) / (p.Ap).
-__global__ void k_cg_alpha(Dev d) {
+__device__ __forceinline__ void cg_alpha_scenes(const Dev& d) {
   const int ns = d.d_n[1];
-  for (int sc = threadIdx.x; sc < ns; sc += blockDim.x) {
+  for (int sc = threadIdx.x >> 5; sc < ns; sc += blockDim.x >> 5) {
     SceneDyn& y = d.dyn[sc];
     if (!y.act_cg) continue;
-    const double pap = acc_sum(d.acc, sc, ACC_PAP);
-    acc_zero(d.acc, sc, ACC_PAP);
-    y.cg_alpha = pap != 0.0 ? y.cg_rz / pap : 0.0;
+    const double pap = acc_take(d.acc, sc, ACC_PAP);
+    if ((threadIdx.x & 31) == 0) y.cg_alpha = pap != 0.0 ? y.cg_rz / pap : 0.0;
   }
 }
+__global__ void k_cg_alpha(Dev d) { cg_alpha_scenes(d); }
 
 // PCG convergence check per scene (relative residual, FP64) and beta.
-__global__ void k_cg_check(Dev d) {
-  __shared__ int any;
-  if (threadIdx.x == 0) any = 0;
-  __syncthreads();
+__device__ __forceinline__ int cg_check_scenes(const Dev& d) {
   const int ns = d.d_n[1];
-  for (int sc = threadIdx.x; sc < ns; sc += blockDim.x) {
+  int any = 0;
+  for (int sc = threadIdx.x >> 5; sc < ns; sc += blockDim.x >> 5) {
     SceneDyn& y = d.dyn[sc];
     const SceneDev& s = d.sc[sc];
     if (!y.act_cg) continue;
-    const double rr = acc_sum(d.acc, sc, ACC_RR), rz = acc_sum(d.acc, sc, ACC_RZ);
-    acc_zero(d.acc, sc, ACC_RR);
-    acc_zero(d.acc, sc, ACC_RZ);
-    y.it_cg += 1;
-    y.cg_rel = y.cg_bnorm2 > 0 ? sqrt(rr / y.cg_bnorm2) : 0.0;
-    y.cg_beta = y.cg_rz != 0.0 ? rz / y.cg_rz : 0.0;
-    y.cg_rz = rz;
-    if (y.cg_rel <= s.visco_tol || y.it_cg >= s.visco_max_iter || !(y.cg_rel == y.cg_rel)) y.act_cg = 0;
-    if (y.act_cg) any = 1;
+    const double rr = acc_take(d.acc, sc, ACC_RR), rz = acc_take(d.acc, sc, ACC_RZ);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+      y.it_cg += 1;
+      y.cg_rel = y.cg_bnorm2 > 0 ? sqrt(rr / y.cg_bnorm2) : 0.0;
+      y.cg_beta = y.cg_rz != 0.0 ? rz / y.cg_rz : 0.0;
+      y.cg_rz = rz;
+      if (y.cg_rel <= s.visco_tol || y.it_cg >= s.visco_max_iter || !(y.cg_rel == y.cg_rel)) y.act_cg = 0;
+      any |= y.act_cg;
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *d.any_active = any;
-    atomicAdd(&d.body_count[2], 1);
-#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
-    if (d.loop_handle) cudaGraphSetConditional((cudaGraphConditionalHandle)d.loop_handle, any ? 1u : 0u);
-#endif
-  }
+  return __syncthreads_or(any);
 }
+__global__ void k_cg_check(Dev d) { loop_decide(d, cg_check_scenes(d), 2); }
 
-__global__ void k_cg_pupdate(Dev d) {
+__device__ __forceinline__ void cg_pupdate_body(const Dev& d) {
   const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
-    const uint32_t fl = d.w.flags[i];
+  FOR_SLOTS_WARP(i, valid, n) {  // cg_update_body's slots, whose z it reads
+    const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const int scn = slot_scene(fl);
-    if (!cg_row(d, i, fl) || !d.dyn[scn].act_cg) continue;
+    if (!valid || !cg_row(d, i, fl) || !d.dyn[scn].act_cg) continue;
     const real be = (real)d.dyn[scn].cg_beta;
     const real3 z = f3(d.cg_z[i]);
-    const real4 p4 = d.cg_pp[2 * (size_t)(i) + 1];
+    const real4 p4 = d.cg_pp[2 * (size_t)i + 1];
     const real3 np = z + f3(p4) * be;
-    d.cg_pp[2 * (size_t)(i) + 1] = make_real4(np.x, np.y, np.z, p4.w);  // w: mu_i
+    d.cg_pp[2 * (size_t)i + 1] = make_real4(np.x, np.y, np.z, p4.w);  // w: mu_i
   }
 }
+__global__ void k_cg_pupdate(Dev d) { cg_pupdate_body(d); }
 
 // Implicit scenes: a_i += (x_i - v_i)/dt (the viscous acceleration of the CG
 // solution); then, for every scene, non_pressure_advect (SPH/main.py:1843-1848).
@@ -1131,6 +1130,56 @@ __global__ void k_cg_finish(Dev d, int advect) {
     }
     if (advect && (fl & NN_CLS_DYNAMIC)) vel_of(d, i) = make_real4(v4.x + dt * a.x, v4.y + dt * a.y, v4.z + dt * a.z, v4.w);
   }
+}
+
+// ---------------------------------------------------------------------------
+// The solver loops of a step as one cooperative kernel each. As graph nodes, a loop costs a
+// while-node (5-10 us a turn) and a one-block check (3 us) beside its two passes. The passes
+// are the same bodies; blocks meet at grid barriers (2.6 us), whose last arrival runs the
+// check. What a pass gathers of arrays that this kernel writes goes through coherent loads.
+#define NN_SOLVE_BLOCK 128
+__device__ __forceinline__ bool solve_failed(const Dev& d) {
+  if (threadIdx.x == 0) set_status(&d.dyn[0], NN_ERR_CUDA);
+  return true;
+}
+#define SOLVE_BARRIER(d, last) do { if (!grid_barrier((d).bar, gen, last) && solve_failed(d)) return; } while (0)
+#define SOLVE_GOES_ON(d) (*(volatile int32_t*)(d).any_active != 0)
+
+template <int L, bool FOLD>
+__global__ void NN_REGS64 k_divergence_loop(const __grid_constant__ Dev d) {
+  unsigned gen = grid_gen(d.bar);
+  do {
+    divergence_update_body<1, L, true>(d);
+    SOLVE_BARRIER(d, [] {});
+    density_change_body<1, L, false, true>(d, 1, FOLD ? 1 : 0);
+    if constexpr (FOLD) density_change_body<1, L, true, true>(d, 1, 1);
+    SOLVE_BARRIER(d, [&] { loop_decide(d, solver_check_scenes(d.d_n, d.sc, d.dyn, d.acc, 0, FOLD), -1); });
+  } while (SOLVE_GOES_ON(d));
+}
+
+template <int L>
+__global__ void NN_REGS64 k_cg_loop(const __grid_constant__ Dev d) {  // after k_cg_check0
+  unsigned gen = grid_gen(d.bar);
+  while (SOLVE_GOES_ON(d)) {
+    cg_matvec_body<1, L, true>(d);
+    SOLVE_BARRIER(d, [&] { cg_alpha_scenes(d); });
+    cg_update_body(d);
+    SOLVE_BARRIER(d, [&] { loop_decide(d, cg_check_scenes(d), -1); });
+    if (!SOLVE_GOES_ON(d)) return;
+    cg_pupdate_body(d);
+    SOLVE_BARRIER(d, [] {});
+  }
+}
+
+template <int L>
+__global__ void NN_REGS64 k_pressure_loop(const __grid_constant__ Dev d) {
+  unsigned gen = grid_gen(d.bar);
+  do {
+    pressure_update_body<1, L, true>(d);
+    SOLVE_BARRIER(d, [] {});
+    density_adv_body<1, L, true>(d, 1);
+    SOLVE_BARRIER(d, [&] { loop_decide(d, solver_check_scenes(d.d_n, d.sc, d.dyn, d.acc, 1, 0), -1); });
+  } while (SOLVE_GOES_ON(d));
 }
 
 // ---------------------------------------------------------------------------

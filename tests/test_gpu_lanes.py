@@ -55,6 +55,40 @@ def test_coupled_solids_do_not_depend_on_the_lanes(cuda_lib):
         assert np.array_equal(a[k].cpu().numpy(), b[k].cpu().numpy()), k
 
 
+@pytest.mark.parametrize("counts,kind", [((1, 1, 1), {}), ((9, 7, 8), CROSS), ((21, 20, 19), CROSS), ((26, 25, 24), CROSS),
+                                         ((35, 34, 33), CROSS), ((39, 40, 41), CROSS)])
+def test_one_kernel_loops_equal_the_host_driven_ones(cuda_lib, counts, kind):
+    """The captured step's loops, one cooperative kernel each where the scene splits a
+    particle over lanes (and the viscosity's below its own limit), against the separate
+    kernels that the host drives: the same fields and iteration counts, over steps in which
+    every loop runs several bodies."""
+    sc = S.dam_break(seed=5, n_side=counts, box=max(counts) * 0.02 + 0.1, **kind)
+    sc.config["Configuration"].update(maxError=0.002, maxErrorV=0.02)
+    sc.config["FluidParticles"][0].update(viscoMaxError=1e-6)
+    x = sc.particles.x
+    nf = sc.particles.n_fluid
+    x[:nf] = x[0] + (x[:nf] - x[0]) * 0.92  # above the rest density: the density solve iterates
+    out = []
+    for host in (False, True):
+        m = sph.initialize(SimConfig(config=sc.config), particles=sc.particles)
+        solver = sph.build_solver()
+        solver.host_loop = host
+        solver.initialize()
+        g = torch.Generator("cuda").manual_seed(2)
+        m.pd.v.copy_((torch.rand(m.pd.v.shape, generator=g, device="cuda") - 0.5) * m.pd.is_dynamic[:, None])
+        its = []
+        for _ in range(3):
+            solver.step()
+            st = solver.stats()
+            assert st["status"] == 0
+            its.append((st["iterations_v"], st["iterations"], st["cg_iterations"]))
+        out.append((its, *[getattr(m.pd, k).cpu().numpy() for k in ("x", "v", "acceleration")]))
+    assert out[0][0] == out[1][0]
+    assert nf < 100 or (max(i[0] for i in out[0][0]) > 0 and max(i[1] for i in out[0][0]) > 1), out[0][0]
+    for a, b in zip(out[0][1:], out[1][1:]):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("seed,counts,max_nb", [(1, (1, 1, 1), 64), (2, (3, 5, 7), 64), (3, (13, 13, 13), 64),
                                                 (4, (17, 9, 31), 40)])
 @pytest.mark.parametrize("cell_factor", [1, 2])
