@@ -63,12 +63,14 @@ struct Dev {
   int32_t* el_slot;            // [Ne] current slot
   int32_t* e_of_id;            // [cap] elastic index or -1
   real4* el_x0;                // [Ne] rest position, rest volume
+  real4* el_x;                 // [Ne] current position, mass
   int32_t* el_nb;              // [rest_cap][Ne] rest neighbours (elastic indices)
   int32_t* el_cnt;             // [Ne]
   int32_t el_cap;              // rest list capacity
   int32_t el_stride;           // Ne capacity
   real* el_R;                  // [9][Ne]
   real* el_S;                  // [6][Ne]
+  real* el_M;                  // [9][Ne] R S
   // rigid bodies ("r-space")
   int32_t n_rb;
   const int32_t* rb_of_id;     // [cap] body index or -1

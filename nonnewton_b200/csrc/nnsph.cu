@@ -97,8 +97,8 @@ struct nn_ctx {
   int el_cap = 64, el_stride = 0;
   bool el_stale = false;               // rest lists re-sized since the last nn_initialize
   int32_t *el_id = nullptr, *el_slot = nullptr, *e_of_id = nullptr, *el_nb = nullptr, *el_cnt = nullptr;
-  real4* el_x0 = nullptr;
-  real *el_R = nullptr, *el_S = nullptr;
+  real4 *el_x0 = nullptr, *el_x = nullptr;
+  real *el_R = nullptr, *el_S = nullptr, *el_M = nullptr;
   int n_rb = 0, rb_rounds = 0, coupling_max = 1;
   int32_t *rb_of_id = nullptr, *rb_round = nullptr;
   double *rb_acc = nullptr, *rb_rest = nullptr, *rb_cm = nullptr, *rb_R = nullptr;
@@ -192,9 +192,9 @@ static Dev make_dev(nn_ctx* c, int cur) {
   d.cg_x = c->cg_x; d.cg_r = c->cg_r; d.cg_z = c->cg_z; d.cg_pp = c->cg_pp; d.cg_Ap = c->cg_Ap;
   d.cg_aux = c->cg_aux;
   d.cg_pinv = c->cg_pinv;
-  d.el_id = c->el_id; d.el_slot = c->el_slot; d.e_of_id = c->e_of_id; d.el_x0 = c->el_x0;
+  d.el_id = c->el_id; d.el_slot = c->el_slot; d.e_of_id = c->e_of_id; d.el_x0 = c->el_x0; d.el_x = c->el_x;
   d.el_nb = c->el_nb; d.el_cnt = c->el_cnt; d.el_cap = c->el_cap; d.el_stride = c->el_stride;
-  d.el_R = c->el_R; d.el_S = c->el_S;
+  d.el_R = c->el_R; d.el_S = c->el_S; d.el_M = c->el_M;
   d.n_rb = c->n_rb; d.rb_of_id = c->rb_of_id; d.rb_round = c->rb_round; d.rb_acc = c->rb_acc;
   d.rb_rest = c->rb_rest; d.rb_cm = c->rb_cm; d.rb_R = c->rb_R;
   d.any_active = c->d_any;
@@ -528,11 +528,12 @@ static int enq_nonpressure(nn_ctx* c, cudaStream_t s, int advect, int clear) {
 static int enq_elastic(nn_ctx* c, cudaStream_t s) {
   if (c->el_mult_max <= 0 || c->ne == 0) return NN_OK;
   Dev d = make_dev(c, c->cur);
-  RC(launch(c, s, k_el_slots, 256, c->ne, d));
+  RC(launch(c, s, k_el_gather, 256, c->ne, d));
   for (int rep = 0; rep < c->el_mult_max; ++rep) {
-    RC(launch(c, s, k_el_rotations, 128, c->ne, d, rep));
-    RC(launch(c, s, k_el_stress, 128, c->ne, d, rep));
-    RC(launch(c, s, k_el_forces, 128, c->ne, d, rep));
+    RC(launch_lanes(c, s, k_el_deformation, EL_BLOCK, c->ne, EL_LANES, d, rep));
+    RC(launch(c, s, k_el_rotations, 64, c->ne, d, rep));
+    RC(launch_lanes(c, s, k_el_stress, EL_BLOCK, c->ne, EL_LANES, d, rep));
+    RC(launch_lanes(c, s, k_el_forces, EL_BLOCK, c->ne, EL_LANES, d, rep));
   }
   return NN_OK;
 }
@@ -749,10 +750,10 @@ static int ensure_cells(nn_ctx* c, int64_t cells) {
 
 static void free_elastic(nn_ctx* c) {
   cudaFree(c->el_id); cudaFree(c->el_slot); cudaFree(c->el_nb); cudaFree(c->el_cnt);
-  cudaFree(c->el_x0); cudaFree(c->el_R); cudaFree(c->el_S);
+  cudaFree(c->el_x0); cudaFree(c->el_x); cudaFree(c->el_R); cudaFree(c->el_S); cudaFree(c->el_M);
   c->el_id = c->el_slot = c->el_nb = c->el_cnt = nullptr;
-  c->el_x0 = nullptr;
-  c->el_R = c->el_S = nullptr;
+  c->el_x0 = c->el_x = nullptr;
+  c->el_R = c->el_S = c->el_M = nullptr;
   c->el_stride = 0;
 }
 
@@ -1038,7 +1039,8 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
     if (dalloc(&c->el_id, E) != cudaSuccess || dalloc(&c->el_slot, E) != cudaSuccess ||
         dalloc(&c->el_nb, E * c->el_cap) != cudaSuccess || dalloc(&c->el_cnt, E) != cudaSuccess ||
         dalloc(&c->el_x0, E) != cudaSuccess || dalloc(&c->el_R, 9 * E) != cudaSuccess ||
-        dalloc(&c->el_S, 6 * E) != cudaSuccess)
+        dalloc(&c->el_S, 6 * E) != cudaSuccess || dalloc(&c->el_x, E) != cudaSuccess ||
+        dalloc(&c->el_M, 9 * E) != cudaSuccess)
       return fail(c, NN_ERR_OOM, "elastic buffers");
     CK(cudaMemcpy(c->el_id, el_id.data(), E * sizeof(int32_t), cudaMemcpyHostToDevice));
     CK(cudaMemset(c->el_cnt, 0, E * sizeof(int32_t)));
