@@ -542,6 +542,9 @@ static int enq_elastic(nn_ctx* c, cudaStream_t s) {
 static int enq_rigid(nn_ctx* c, cudaStream_t s) {
   if (c->n_rb == 0) return NN_OK;
   Dev d = make_dev(c, c->cur);
+  if (std::max(c->n, c->in_capture ? c->cap : 0) <= NN_RIGID_BLOCK_MAX) {  // a capture serves up to the capacity
+    return launch_g(c, s, k_rigid_block, 1, 1024, d, c->rb_rounds, c->coupling_max);
+  }
   for (int rep = 0; rep < c->coupling_max; ++rep)
     for (int r = 0; r < c->rb_rounds; ++r) {
       RC(launch(c, s, k_rigid_ground, 256, c->n, d, r, rep));

@@ -1545,107 +1545,154 @@ __device__ __forceinline__ int rigid_body_of_slot(const Dev& d, int i, int round
   return (b >= 0 && d.rb_round[b] == round) ? b : -1;
 }
 
+// The steps of a body's substep, per slot or per body; kernels of their own below, and one
+// block's loop over all of them in a small scene (k_rigid_block).
+
 // ground_collision (SPH/main.py:1113-1118): every solid particle of a scene with
 // rigid bodies is lifted to y >= padding (once per body substep, like the reference).
-__global__ void k_rigid_ground(Dev d, int round, int rep) {
-  const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
-    const uint32_t fl = d.w.flags[i];
-    if (!cls_solid(fl)) continue;
-    const SceneDev& s = d.sc[slot_scene(fl)];
-    if (!(s.flags & NN_F_RIGID) || round >= s.n_rigid || rep >= s.coupling) continue;
-    real4 p = xyz_of(d, i);
-    if (p.y < s.padding) { p.y = s.padding; xyz_of(d, i) = p; }
+__device__ __forceinline__ void rigid_ground_slot(const Dev& d, int i, int round, int rep) {
+  const uint32_t fl = d.w.flags[i];
+  if (!cls_solid(fl)) return;
+  const SceneDev& s = d.sc[slot_scene(fl)];
+  if (!(s.flags & NN_F_RIGID) || round >= s.n_rigid || rep >= s.coupling) return;
+  real4 p = xyz_of(d, i);
+  if (p.y < s.padding) { p.y = s.padding; xyz_of(d, i) = p; }
+}
+// compute_com (SPH/main.py:1120-1130) over the current (rest = 0) or rest positions.
+__device__ __forceinline__ void rigid_com_slot(const Dev& d, int i, int rest, double (&v)[4]) {
+  const SceneDev& s = d.sc[slot_scene(d.w.flags[i])];
+  const double m = (double)(s.V0 * d.w.dens[i]);
+  real3 x;
+  if (rest) {
+    const int id = d.w.id[i];
+    x = make_real3(d.t.x_0[3 * id], d.t.x_0[3 * id + 1], d.t.x_0[3 * id + 2]);
+  } else {
+    x = f3(xyz_of(d, i));
   }
+  v[0] = m * x.x; v[1] = m * x.y; v[2] = m * x.z; v[3] = m;
+}
+// Centre of mass of a body (into rb_rest for the rest state, rb_cm otherwise).
+__device__ __forceinline__ void rigid_cm_body(const Dev& d, int b, int rest) {
+  double* a = &d.rb_acc[(size_t)b * RB_ACC];
+  double* out = rest ? &d.rb_rest[3 * b] : &d.rb_cm[3 * b];
+  const double m = __ldcg(&a[3]);  // written by atomics, like the rest of the accumulators
+  for (int k = 0; k < 3; ++k) out[k] = m > 0 ? __ldcg(&a[k]) / m : 0.0;
+  for (int k = 0; k < RB_ACC; ++k) a[k] = 0.0;
+}
+// A = sum m (x - cm) (x) (x0 - rest_cm) (SPH/main.py:1141-1146).
+__device__ __forceinline__ void rigid_A_slot(const Dev& d, int i, int b, double (&v)[9]) {
+  const SceneDev& s = d.sc[slot_scene(d.w.flags[i])];
+  const double m = (double)(s.V0 * d.w.dens[i]);
+  const int id = d.w.id[i];
+  const real4 x = xyz_of(d, i);
+  const double p[3] = {(double)x.x - d.rb_cm[3 * b], (double)x.y - d.rb_cm[3 * b + 1],
+                       (double)x.z - d.rb_cm[3 * b + 2]};
+  const double q[3] = {(double)d.t.x_0[3 * id] - d.rb_rest[3 * b], (double)d.t.x_0[3 * id + 1] - d.rb_rest[3 * b + 1],
+                       (double)d.t.x_0[3 * id + 2] - d.rb_rest[3 * b + 2]};
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[3 * r + c] = m * p[r] * q[c];
+}
+// R = polar(A) (SPH/main.py:1148-1151), identity if every entry is below 1e-6.
+__device__ __forceinline__ void rigid_R_body(const Dev& d, int b) {
+  double* a = &d.rb_acc[(size_t)b * RB_ACC + 4];
+  double A[3][3], R[3][3];
+  for (int k = 0; k < 9; ++k) A[k / 3][k % 3] = __ldcg(&a[k]);
+  closest_rotation(A, R);
+  bool small = true;
+  for (int k = 0; k < 9; ++k) small = small && fabs(R[k / 3][k % 3]) < 1e-6;
+  for (int k = 0; k < 9; ++k) d.rb_R[9 * b + k] = small ? ((k % 4 == 0) ? 1.0 : 0.0) : R[k / 3][k % 3];
+  for (int k = 0; k < RB_ACC; ++k) d.rb_acc[(size_t)b * RB_ACC + k] = 0.0;
+}
+// x = cm + R (x0 - rest_cm) (SPH/main.py:1153-1157).
+__device__ __forceinline__ void rigid_apply_slot(const Dev& d, int i, int b) {
+  const int id = d.w.id[i];
+  const double q[3] = {(double)d.t.x_0[3 * id] - d.rb_rest[3 * b], (double)d.t.x_0[3 * id + 1] - d.rb_rest[3 * b + 1],
+                       (double)d.t.x_0[3 * id + 2] - d.rb_rest[3 * b + 2]};
+  const double* R = &d.rb_R[9 * b];
+  real4 p = xyz_of(d, i);
+  p.x = (real)(d.rb_cm[3 * b] + R[0] * q[0] + R[1] * q[1] + R[2] * q[2]);
+  p.y = (real)(d.rb_cm[3 * b + 1] + R[3] * q[0] + R[4] * q[1] + R[5] * q[2]);
+  p.z = (real)(d.rb_cm[3 * b + 2] + R[6] * q[0] + R[7] * q[1] + R[8] * q[2]);
+  xyz_of(d, i) = p;
 }
 
-// compute_com (SPH/main.py:1120-1130) over the current (rest = 0) or rest positions.
+__global__ void k_rigid_ground(Dev d, int round, int rep) {
+  GRID_STRIDE(i, d.d_n[0]) rigid_ground_slot(d, i, round, rep);
+}
 __global__ void k_rigid_com(Dev d, int round, int rest) {
   const int n = d.d_n[0];
   FOR_SLOTS_WARP(i, valid, n) {
-    int b = valid ? rigid_body_of_slot(d, i, round) : -1;
+    const int b = valid ? rigid_body_of_slot(d, i, round) : -1;
     double v[4] = {0, 0, 0, 0};
-    if (b >= 0) {
-      const SceneDev& s = d.sc[slot_scene(d.w.flags[i])];
-      const double m = (double)(s.V0 * d.w.dens[i]);
-      real3 x;
-      if (rest) {
-        const int id = d.w.id[i];
-        x = make_real3(d.t.x_0[3 * id], d.t.x_0[3 * id + 1], d.t.x_0[3 * id + 2]);
-      } else {
-        x = f3(xyz_of(d, i));
-      }
-      v[0] = m * x.x; v[1] = m * x.y; v[2] = m * x.z; v[3] = m;
-    }
+    if (b >= 0) rigid_com_slot(d, i, rest, v);
     body_add<4>(d.rb_acc, b, v);
   }
 }
-
-// Per body: centre of mass (into rb_rest for the rest state, rb_cm otherwise).
 __global__ void k_rigid_cm(Dev d, int round, int rest) {
-  for (int b = threadIdx.x; b < d.n_rb; b += blockDim.x) {
-    if (d.rb_round[b] != round) continue;
-    double* a = &d.rb_acc[(size_t)b * RB_ACC];
-    double* out = rest ? &d.rb_rest[3 * b] : &d.rb_cm[3 * b];
-    for (int k = 0; k < 3; ++k) out[k] = a[3] > 0 ? a[k] / a[3] : 0.0;
-    for (int k = 0; k < RB_ACC; ++k) a[k] = 0.0;
-  }
+  for (int b = threadIdx.x; b < d.n_rb; b += blockDim.x)
+    if (d.rb_round[b] == round) rigid_cm_body(d, b, rest);
 }
-
-// A = sum m (x - cm) (x) (x0 - rest_cm) (SPH/main.py:1141-1146).
 __global__ void k_rigid_A(Dev d, int round) {
   const int n = d.d_n[0];
   FOR_SLOTS_WARP(i, valid, n) {
-    int b = valid ? rigid_body_of_slot(d, i, round) : -1;
+    const int b = valid ? rigid_body_of_slot(d, i, round) : -1;
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (b >= 0) {
-      const SceneDev& s = d.sc[slot_scene(d.w.flags[i])];
-      const double m = (double)(s.V0 * d.w.dens[i]);
-      const int id = d.w.id[i];
-      const real4 x = xyz_of(d, i);
-      const double p[3] = {(double)x.x - d.rb_cm[3 * b], (double)x.y - d.rb_cm[3 * b + 1],
-                           (double)x.z - d.rb_cm[3 * b + 2]};
-      const double q[3] = {(double)d.t.x_0[3 * id] - d.rb_rest[3 * b], (double)d.t.x_0[3 * id + 1] - d.rb_rest[3 * b + 1],
-                           (double)d.t.x_0[3 * id + 2] - d.rb_rest[3 * b + 2]};
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) v[3 * r + c] = m * p[r] * q[c];
-    }
-    double* acc = d.rb_acc + 4;  // the A block of each body's accumulator
-    body_add<9>(acc, b, v);
+    if (b >= 0) rigid_A_slot(d, i, b, v);
+    body_add<9>(d.rb_acc + 4, b, v);  // the A block of each body's accumulator
   }
 }
-
-// R = polar(A) (SPH/main.py:1148-1151), identity if every entry is below 1e-6.
 __global__ void k_rigid_R(Dev d, int round) {
-  for (int b = threadIdx.x; b < d.n_rb; b += blockDim.x) {
-    if (d.rb_round[b] != round) continue;
-    double* a = &d.rb_acc[(size_t)b * RB_ACC + 4];
-    double A[3][3], R[3][3];
-    for (int k = 0; k < 9; ++k) A[k / 3][k % 3] = a[k];
-    closest_rotation(A, R);
-    bool small = true;
-    for (int k = 0; k < 9; ++k) small = small && fabs(R[k / 3][k % 3]) < 1e-6;
-    for (int k = 0; k < 9; ++k) d.rb_R[9 * b + k] = small ? ((k % 4 == 0) ? 1.0 : 0.0) : R[k / 3][k % 3];
-    for (int k = 0; k < RB_ACC; ++k) d.rb_acc[(size_t)b * RB_ACC + k] = 0.0;
+  for (int b = threadIdx.x; b < d.n_rb; b += blockDim.x)
+    if (d.rb_round[b] == round) rigid_R_body(d, b);
+}
+__global__ void k_rigid_apply(Dev d, int round) {
+  GRID_STRIDE(i, d.d_n[0]) {
+    const int b = rigid_body_of_slot(d, i, round);
+    if (b >= 0) rigid_apply_slot(d, i, b);
   }
 }
 
-// x = cm + R (x0 - rest_cm) (SPH/main.py:1153-1157).
-__global__ void k_rigid_apply(Dev d, int round) {
+// All rounds and coupling substeps in one block, for up to NN_RIGID_BLOCK_MAX slots: the six
+// launches of a body's substep, 2-4 us each, are barriers of the block, and after the ground
+// pass only the round's own slots are walked. 2,966 slots, two substeps: 33 -> 18 us.
+#define NN_RIGID_BLOCK_MAX 8192
+__global__ void __launch_bounds__(1024) k_rigid_block(Dev d, int rounds, int reps) {
+  __shared__ int slots[NN_RIGID_BLOCK_MAX];
+  __shared__ int count;
   const int n = d.d_n[0];
-  GRID_STRIDE(i, n) {
-    const int b = rigid_body_of_slot(d, i, round);
-    if (b < 0) continue;
-    const int id = d.w.id[i];
-    const double q[3] = {(double)d.t.x_0[3 * id] - d.rb_rest[3 * b], (double)d.t.x_0[3 * id + 1] - d.rb_rest[3 * b + 1],
-                         (double)d.t.x_0[3 * id + 2] - d.rb_rest[3 * b + 2]};
-    const double* R = &d.rb_R[9 * b];
-    real4 p = xyz_of(d, i);
-    p.x = (real)(d.rb_cm[3 * b] + R[0] * q[0] + R[1] * q[1] + R[2] * q[2]);
-    p.y = (real)(d.rb_cm[3 * b + 1] + R[3] * q[0] + R[4] * q[1] + R[5] * q[2]);
-    p.z = (real)(d.rb_cm[3 * b + 2] + R[6] * q[0] + R[7] * q[1] + R[8] * q[2]);
-    xyz_of(d, i) = p;
-  }
+  for (int rep = 0; rep < reps; ++rep)
+    for (int r = 0; r < rounds; ++r) {
+      if (threadIdx.x == 0) count = 0;
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        rigid_ground_slot(d, i, r, rep);
+        if (rigid_body_of_slot(d, i, r) >= 0) slots[atomicAdd(&count, 1)] = i;
+      }
+      __syncthreads();
+      const int m = count, warps_end = (m + 31) & ~31;
+      for (int k = threadIdx.x; k < warps_end; k += blockDim.x) {
+        const int b = k < m ? rigid_body_of_slot(d, slots[k], r) : -1;
+        double v[4] = {0, 0, 0, 0};
+        if (b >= 0) rigid_com_slot(d, slots[k], 0, v);
+        body_add<4>(d.rb_acc, b, v);
+      }
+      __syncthreads();
+      for (int b = threadIdx.x; b < d.n_rb; b += blockDim.x)
+        if (d.rb_round[b] == r) rigid_cm_body(d, b, 0);
+      __syncthreads();
+      for (int k = threadIdx.x; k < warps_end; k += blockDim.x) {
+        const int b = k < m ? rigid_body_of_slot(d, slots[k], r) : -1;
+        double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+        if (b >= 0) rigid_A_slot(d, slots[k], b, v);
+        body_add<9>(d.rb_acc + 4, b, v);
+      }
+      __syncthreads();
+      for (int b = threadIdx.x; b < d.n_rb; b += blockDim.x)
+        if (d.rb_round[b] == r) rigid_R_body(d, b);
+      __syncthreads();
+      for (int k = threadIdx.x; k < m; k += blockDim.x) rigid_apply_slot(d, slots[k], rigid_body_of_slot(d, slots[k], r));
+      __syncthreads();
+    }
 }

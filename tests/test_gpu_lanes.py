@@ -124,3 +124,23 @@ def test_list_build_per_row(cuda_lib, seed, counts, max_nb, cell_factor):
         m.engine.run_pass(_abi.NN_PASS_SEARCH)
         st = m.engine.stats(0)
         assert st["status"] == _abi.NN_ERR_NEIGHBOR_OVERFLOW and st["max_neighbors_seen"] == int(num.max())
+
+
+@pytest.mark.parametrize("n_body,coupling", [((4, 4, 4), 1), ((3, 5, 2), 3)])
+def test_rigid_substeps_in_one_block(cuda_lib, n_body, coupling):
+    """The rigid bodies' substeps run in one block up to a slot capacity, as separate kernels
+    above it: a batch of each capacity over the same scene. The sums are FP64 atomics in
+    both, so positions agree to the last bits of f32."""
+    from nonnewton_b200.batch import Batch
+
+    sc = S.rigid_drop(seed=6, n_body=n_body, coupling=coupling)
+    sc.particles.x[sc.particles.phase_id >= 2000, 1] -= 0.05
+    out = []
+    for capacity in (sc.particles.n, 8193):
+        b = Batch(capacity, 1)
+        b.set([sc])
+        b.step(3)
+        assert b.stats(0)["status"] == 0
+        out.append(b.scene_view(0, "x").cpu().numpy())
+    assert sc.particles.n <= 8192
+    assert np.abs(out[0] - out[1]).max() <= 2e-7  # an ulp or two at the domain's size
