@@ -348,14 +348,18 @@ __device__ __forceinline__ uint64_t splat_x2(float v) {
   const uint64_t u = __float_as_uint(v);
   return u | (u << 32);
 }
-__device__ __forceinline__ uint32_t pair_hits(const float* sx, const float* sy, const float* sz, uint32_t t,
-                                              uint64_t nx, uint64_t ny, uint64_t nz, float thr) {
+// The candidates t and t + 1 pushed into a hit mask from the right: the test r2 < h2_thr is
+// the sign of r2 - h2_thr (one packed add; the sign of a correctly rounded difference is
+// exact, and a NaN result is the positive canonical one), which a funnel shift moves into
+// the mask, one instruction per candidate instead of compare, select and insert.
+__device__ __forceinline__ void pair_push(const float* sx, const float* sy, const float* sz, uint32_t t, uint64_t nx,
+                                          uint64_t ny, uint64_t nz, uint64_t nthr, uint32_t& m) {
   const uint64_t dx = add_rn_x2(*reinterpret_cast<const uint64_t*>(sx + t), nx);
   const uint64_t dy = add_rn_x2(*reinterpret_cast<const uint64_t*>(sy + t), ny);
   const uint64_t dz = add_rn_x2(*reinterpret_cast<const uint64_t*>(sz + t), nz);
-  const uint64_t r2 = add_rn_x2(add_rn_x2(sq_rn_x2(dx), sq_rn_x2(dy)), sq_rn_x2(dz));
-  return (uint32_t)(__uint_as_float((uint32_t)r2) < thr) |
-         ((uint32_t)(__uint_as_float((uint32_t)(r2 >> 32)) < thr) << 1);
+  const uint64_t d = add_rn_x2(add_rn_x2(add_rn_x2(sq_rn_x2(dx), sq_rn_x2(dy)), sq_rn_x2(dz)), nthr);
+  m = __funnelshift_l((uint32_t)d, m, 1);
+  m = __funnelshift_l((uint32_t)(d >> 32), m, 1);
 }
 #endif
 
@@ -384,7 +388,7 @@ __global__ void __launch_bounds__(NS_WARPS * 32) k_build_lists(Dev d) {
     const real3 xi = f3(pi);
     const real thr = s.h2_thr;
 #ifdef NS_PACKED
-    const uint64_t nx = splat_x2(-xi.x), ny = splat_x2(-xi.y), nz = splat_x2(-xi.z);
+    const uint64_t nx = splat_x2(-xi.x), ny = splat_x2(-xi.y), nz = splat_x2(-xi.z), nthr = splat_x2(-thr);
 #endif
     const int x0 = max(cx - s.nfx, 0), x1 = min(cx + s.nfx, s.gx - 1);
     // lane 0 is always valid (the warp's first slot is below n)
@@ -425,21 +429,23 @@ __global__ void __launch_bounds__(NS_WARPS * 32) k_build_lists(Dev d) {
             // groups of up to 32 candidates from an even stage index (one below lo when
             // lo - c0 is odd; that bit is cleared), tested in pairs
             for (uint32_t g = (lo - c0) & ~1u; lo < hi && g < hi - c0; g += 32) {
+              // candidate c0 + g + t ends up in bit 31 - t
               const uint32_t len = min(32u, hi - c0 - g);
               uint32_t m = 0u, k = 0u;
               for (; k + 4 <= len; k += 4) {  // two independent pairs
-                const uint32_t p0 = pair_hits(sx, sy, sz, g + k, nx, ny, nz, thr);
-                const uint32_t p1 = pair_hits(sx, sy, sz, g + k + 2, nx, ny, nz, thr);
-                m |= (p0 | (p1 << 2)) << k;
+                pair_push(sx, sy, sz, g + k, nx, ny, nz, nthr, m);
+                pair_push(sx, sy, sz, g + k + 2, nx, ny, nz, nthr, m);
               }
-              for (; k < len; k += 2) m |= pair_hits(sx, sy, sz, g + k, nx, ny, nz, thr) << k;
-              if (len < 32u) m &= (1u << len) - 1u;
-              if (c0 + g < lo) m &= ~1u;
+              for (; k < len; k += 2) pair_push(sx, sy, sz, g + k, nx, ny, nz, nthr, m);
+              m <<= 32u - k;
+              m &= 0xffffffffu << (32u - len);
+              if (c0 + g < lo) m &= 0x7fffffffu;
               const uint32_t self = (uint32_t)i - (c0 + g);
-              if (self < 32u) m &= ~(1u << self);
+              if (self < 32u) m &= ~(0x80000000u >> self);
               while (m) {
-                append((int)(c0 + g + __ffs(m) - 1));
-                m &= m - 1u;
+                const uint32_t t = (uint32_t)__clz((int)m);
+                append((int)(c0 + g + t));
+                m &= 0x7fffffffu >> t;
               }
             }
 #else
@@ -562,11 +568,18 @@ __global__ void __launch_bounds__(NSR_WARPS * 32) k_build_lists_rows(Dev d) {
           if (lane == 0 && ((re - rb) & 1u)) { sx[re - rb] = 0.f; sy[re - rb] = 0.f; sz[re - rb] = 0.f; }
           __syncwarp();
           if (e > b) {
-            const uint64_t nx = splat_x2(-xi.x), ny = splat_x2(-xi.y), nz = splat_x2(-xi.z);
+            const uint64_t nx = splat_x2(-xi.x), ny = splat_x2(-xi.y), nz = splat_x2(-xi.z), nthr = splat_x2(-thr);
             const uint32_t g = (b - rb) & ~1u, len = e - rb - g;  // from an even stage index, at most 63
             from = rb + g;
-            for (uint32_t k = 0; k < len; k += 2)
-              hits |= (unsigned long long)pair_hits(sx, sy, sz, g + k, nx, ny, nz, thr) << k;
+            // two words of up to 32 candidates, the first in bit 63 of hits
+            uint32_t m0 = 0u, m1 = 0u, k = 0u;
+            for (; k < min(len, 32u); k += 2) pair_push(sx, sy, sz, g + k, nx, ny, nz, nthr, m0);
+            m0 <<= 32u - k;
+            if (len > 32u) {
+              for (; k < len; k += 2) pair_push(sx, sy, sz, g + k, nx, ny, nz, nthr, m1);
+              m1 <<= 64u - k;
+            }
+            hits = __brevll(((unsigned long long)m0 << 32) | m1);
             hits &= (1ull << len) - 1ull;
             if (from < b) hits &= ~1ull;
             const uint32_t self = (uint32_t)i - from;
