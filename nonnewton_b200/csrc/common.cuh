@@ -215,7 +215,13 @@ __device__ __forceinline__ int nb_list_load(const int32_t* p) {
   else return ldg(p);
 }
 
-template <int NB_U, bool STREAM = false, typename Load, typename Use>
+// WALK walks the queue of list entries in place, PD batches per turn of the loop, instead of
+// moving it up by PD * NB_U moves per batch. The passes that gain from it name it
+// (k_pressure_update 167 -> 155 us, k_cg_setup 315 -> 304, k_density_factor 258 -> 248,
+// k_density_change_np 390 -> 385, k_divergence_update 208 -> 205 on the 2.4M scene);
+// k_density_adv (218 -> 240) and k_cg_matvec (92 -> 102 on 900,000) keep the short loop.
+enum NbLoop { NB_SHIFT = 0, NB_WALK = 1 };
+template <int NB_U, bool STREAM = false, int LOOP = NB_SHIFT, typename Load, typename Use>
 __device__ __forceinline__ void nb_batches(const int32_t* __restrict__ list, int stride, int c, int self, Load load,
                                            Use use) {
   // software pipeline: list entries are loaded PD batches (8 entries) ahead of the
@@ -226,6 +232,29 @@ __device__ __forceinline__ void nb_batches(const int32_t* __restrict__ list, int
   for (int p = 0; p < PD; ++p)
 #pragma unroll
     for (int u = 0; u < NB_U; ++u) q[p][u] = (p * NB_U + u < c) ? nb_list_load<STREAM>(list + (size_t)(p * NB_U + u) * stride) : self;
+  if constexpr (LOOP == NB_WALK) {
+    for (int k = 0;;) {
+#pragma unroll
+      for (int p = 0; p < PD; ++p) {
+        if (k >= c) return;
+        int j[NB_U];
+#pragma unroll
+        for (int u = 0; u < NB_U; ++u) j[u] = q[p][u];
+#pragma unroll
+        for (int u = 0; u < NB_U; ++u) {
+          const int kk = k + PD * NB_U + u;
+          q[p][u] = (kk < c) ? nb_list_load<STREAM>(list + (size_t)kk * stride) : self;
+        }
+        decltype(load(0)) g[NB_U];
+#pragma unroll
+        for (int u = 0; u < NB_U; ++u) g[u] = load(j[u]);
+#pragma unroll
+        for (int u = 0; u < NB_U; ++u)
+          if (k + u < c) use(j[u], g[u]);
+        k += NB_U;
+      }
+    }
+  }
   for (int k = 0; k < c; k += NB_U) {
     int j[NB_U];
 #pragma unroll
@@ -281,11 +310,11 @@ __device__ __forceinline__ T shfl_reals(const T& t, int src) {
 // order (shuffles): the sums are the same operations in the same order for every L, so
 // results do not depend on it, nor on what a scene is batched with. All 32 lanes call
 // this; lanes without work pass c = 0.
-template <int U, int L, bool STREAM = false, typename Load, typename Term, typename Fold>
+template <int U, int L, bool STREAM = false, int LOOP = NB_SHIFT, typename Load, typename Term, typename Fold>
 __device__ __forceinline__ void nb_sum(const int32_t* __restrict__ list, int stride, int c, int self, int sub,
                                        Load load, Term term, Fold fold) {
   if constexpr (L == 1) {
-    if (c > 0) nb_batches<U, STREAM>(list, stride, c, self, load, [&](int, const auto& g) { fold(term(g)); });
+    if (c > 0) nb_batches<U, STREAM, LOOP>(list, stride, c, self, load, [&](int, const auto& g) { fold(term(g)); });
   } else {
     constexpr int P = 32 / L;
     const int p = (int)(threadIdx.x & (P - 1));

@@ -111,10 +111,10 @@ __global__ void k_density_factor(Dev d, int do_density, int do_factor) {
       if (CHANGE) dd = fma(t.V, t.dv, dd);
     };
     if constexpr (CHANGE) {
-      nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv(d.w.pv, j); },
+      nb_sum<U, L, false, NB_WALK>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv(d.w.pv, j); },
                    [&](const GPV& g) { return term(g.p, g.v); }, fold);
     } else {
-      nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return pos_of(d, j); },
+      nb_sum<U, L, false, NB_WALK>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return pos_of(d, j); },
                    [&](real4 pj) { return term(pj, pj); }, fold);
     }
     if (work) {
@@ -189,7 +189,7 @@ __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int 
       const int c = work ? d.nbr_cnt[i] : 0;
       real dd = 0.f;
       if constexpr (!NP) {
-        nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv<COH>(d.w.pv, j); },
+        nb_sum<U, L, false, NB_WALK>(d.nbr + i, d.cap, c, self, sub, [&](int j) { return load_pv<COH>(d.w.pv, j); },
                      [&](const GPV& g) {
                        const real3 r = xi - f3(g.p);
                        return TDiv{fabs(g.p.w), dot3(vi - f3(g.v), kgrad_r2(r, dot3(r, r), s))};
@@ -210,7 +210,7 @@ __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int 
         // a term struct with the lanes' common operands costs registers that one lane per
         // particle does not have at its cap (40 B spilled): it adds each sum where it is made
         if constexpr (L == 1) {
-          nb_batches<U>(d.nbr + i, d.cap, c, self, load, [&](int, const GPV& g) {
+          nb_batches<U, false, NB_WALK>(d.nbr + i, d.cap, c, self, load, [&](int, const GPV& g) {
             const real3 r = xi - f3(g.p);
             const real r2 = dot3(r, r);
             real w;
@@ -226,7 +226,7 @@ __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int 
             }
           });
         } else {
-          nb_sum<U, L>(d.nbr + i, d.cap, c, self, sub, load,
+          nb_sum<U, L, false, NB_WALK>(d.nbr + i, d.cap, c, self, sub, load,
                        [&](const GPV& g) {
                          TDivNp t;
                          const real3 r = xi - f3(g.p);
@@ -320,7 +320,7 @@ __device__ __forceinline__ void divergence_update_body(const Dev& d) {
     const real3 xi = f3(d.w.pos[self]);
     const real k_i = d.kappa[self];
     real3 dv = make_real3(0.f, 0.f, 0.f);
-    nb_sum<U, L>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, self, sub,
+    nb_sum<U, L, false, NB_WALK>(d.nbr + i, d.cap, work ? d.nbr_cnt[i] : 0, self, sub,
                  [&](int j) { return GPK{pos_of(d, j), nb_load<COH>(&d.kappa[j])}; },
                  [&](const GPK& g) { return push_term(xi, g, k_i, dt, s); },
                  [&](const TPush& t) { push_fold(dv, t); });
@@ -421,7 +421,7 @@ __device__ __forceinline__ void pressure_update_body(const Dev& d) {
       const real k_i = d.kappa[self];
       const real4 v4 = vel_of(d, self);
       real3 vi = f3(v4);
-      nb_sum<U, L, true>(d.nbr + i, d.cap, fluid ? c : 0, self, sub, load,
+      nb_sum<U, L, true, NB_WALK>(d.nbr + i, d.cap, fluid ? c : 0, self, sub, load,
                          [&](const GPK& g) { return push_term(xi, g, k_i, dt, s); },
                          [&](const TPush& t) { push_fold(vi, t); });
       if (work && fluid && sub == 0) vel_of(d, i) = make_real4(vi.x, vi.y, vi.z, v4.w);
@@ -430,7 +430,7 @@ __device__ __forceinline__ void pressure_update_body(const Dev& d) {
       const real Vi = fabs(pi.w);
       const real inv_dt = 1.f / dt;
       real3 ai = make_real3(0.f, 0.f, 0.f);
-      nb_sum<U, L, true>(d.nbr + i, d.cap, fluid ? 0 : c, self, sub, load,
+      nb_sum<U, L, true, NB_WALK>(d.nbr + i, d.cap, fluid ? 0 : c, self, sub, load,
                          [&](const GPK& g) {
                            const real3 r = f3(g.p) - xi;  // x_fluid - x_solid, as the fluid computes it
                            const real3 a = kgrad_r2(r, dot3(r, r), s) * -Vi * (dt * g.k);
@@ -849,7 +849,7 @@ __device__ __forceinline__ real3 cg_apply(const Dev& d, int i, int sub, bool wor
       D[3] = fma(-wg.x, r.y, D[3]); D[4] = fma(-wg.x, r.z, D[4]); D[5] = fma(-wg.y, r.z, D[5]);
     };
     if constexpr (L == 1) {  // each sum added where its term is made, as in density_change_body
-      nb_batches<U>(d.nbr + i, d.cap, cnt, self, load, [&](int, const GCG& g) {
+      nb_batches<U, false, NB_WALK>(d.nbr + i, d.cap, cnt, self, load, [&](int, const GCG& g) {
         const real3 r = xi - f3(g.p);
         const real r2 = dot3(r, r);
         const real3 gw = kgrad_r2(r, r2, s);
