@@ -30,6 +30,7 @@ __device__ __forceinline__ real add_rn(real a, real b) { return __dadd_rn(a, b);
 __device__ __forceinline__ real sqrt_rn(real a) { return __dsqrt_rn(a); }
 __device__ __forceinline__ real fast_div(real a, real b) { return a / b; }
 #define NN_REGS64                         // no register caps: double registers come in pairs
+#define NN_REGS(n)
 #else
 typedef float real;
 typedef float2 real2;
@@ -43,6 +44,7 @@ __device__ __forceinline__ real add_rn(real a, real b) { return __fadd_rn(a, b);
 __device__ __forceinline__ real sqrt_rn(real a) { return __fsqrt_rn(a); }
 __device__ __forceinline__ real fast_div(real a, real b) { return __fdividef(a, b); }
 #define NN_REGS64 __maxnreg__(64)
+#define NN_REGS(n) __maxnreg__(n)
 #endif
 
 // Read-only loads through the texture path (__ldg), double4 as two double2 loads.
