@@ -86,6 +86,8 @@ struct nn_ctx {
   double* d_acc = nullptr;
   int32_t* d_scene_of_id = nullptr;
   int32_t* d_src_flag = nullptr;
+  int src_flag = -1;                   // its value once the stream gets there, -1 unknown
+  bool src_tracked = true;
   real4* acc4 = nullptr;
   real *alpha = nullptr, *rho_adv = nullptr, *kappa = nullptr, *srn = nullptr, *mu = nullptr;
   int32_t* slot_of_id = nullptr;
@@ -404,6 +406,21 @@ static int solver_loop(nn_ctx* c, cudaStream_t s, bool check_first, Pre pre, Bod
 static int enq_build_lists(nn_ctx* c, cudaStream_t s, const Dev& d) {
   if (c->n <= NN_BUILD_ROWS_MAX) return launch_lanes(c, s, k_build_lists_rows, NSR_WARPS * 32, c->n, NSR_WARPS, d);
   return launch(c, s, k_build_lists, NS_WARPS * 32, c->n, d);
+}
+
+// What the next search reads (Dev::src_from_truth): 0 the previous slots, 1 the caller's state,
+// 2 the caller's rest positions. Enqueued only where it changes: before every step it was a
+// launch of its own on the stream. A caller who captures the stream replays the launch at
+// times of their own: from then on it is enqueued every time.
+static int set_src(nn_ctx* c, cudaStream_t s, int v) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(s, &st));
+  if (st != cudaStreamCaptureStatusNone) c->src_tracked = false;
+  if (c->src_tracked && c->src_flag == v) return NN_OK;
+  c->src_flag = -1;
+  RC(launch1(c, s, k_set_int, c->d_src_flag, (int32_t)v));
+  c->src_flag = v;
+  return NN_OK;
 }
 
 // ---- pass sequences ---------------------------------------------------------------
@@ -854,6 +871,7 @@ int nn_ctx_set_stream(nn_ctx* c, void* stream) {
   if (!c) return fail(nullptr, NN_ERR_INVALID_ARG, "null context");
   if ((cudaStream_t)stream != c->stream) drop_graphs(c);
   c->stream = (cudaStream_t)stream;
+  c->src_flag = -1;  // set again on the new stream
   return NN_OK;
 }
 
@@ -1118,14 +1136,13 @@ int nn_initialize(nn_ctx* c) {
   // Their rest neighbourhoods come from a search over the rest positions x_0 (equal to
   // x at t = 0, as in the reference; after a checkpoint restore they differ).
   if (c->ne > 0) {
-    CK(cudaMemsetAsync(c->d_src_flag, 0, sizeof(int32_t), s));
-    RC(launch1(c, s, k_set_int, c->d_src_flag, 2));
+    RC(set_src(c, s, 2));
     RC(enq_search(c, s));
     Dev dr = make_dev(c, c->cur);
     RC(launch1(c, s, k_step_dt, dr, 0));
     RC(launch(c, s, k_el_init, 256, c->n, dr));
   }
-  CK(cudaMemsetAsync(c->d_src_flag, 1, sizeof(int32_t), s));
+  RC(set_src(c, s, 1));
   RC(enq_search(c, s));
   Dev d = make_dev(c, c->cur);
   RC(launch1(c, s, k_step_dt, d, 0));
@@ -1154,7 +1171,7 @@ int nn_step(nn_ctx* c, int32_t nsteps, uint32_t flags) {
     return fail(c, NN_ERR_STATE, "NN_STEP_RESUME: no state left resident by a previous nn_step");
   for (int k = 0; k < nsteps; ++k) {
     // the first step reads the caller's state, unless it resumes from the resident slots
-    CK(cudaMemsetAsync(c->d_src_flag, (k == 0 && !resume) ? 1 : 0, sizeof(int32_t), s));
+    RC(set_src(c, s, (k == 0 && !resume) ? 1 : 0));
     if (host) {
       RC(enq_step(c, s));
     } else {
@@ -1179,7 +1196,7 @@ int nn_run_pass(nn_ctx* c, int32_t pass) {
   c->resident_ok = false;
   cudaStream_t s = run_stream(c);
   if (pass == NN_PASS_SEARCH) {
-    CK(cudaMemsetAsync(c->d_src_flag, 1, sizeof(int32_t), s));
+    RC(set_src(c, s, 1));
     RC(launch1(c, s, k_step_reset, make_dev(c, c->cur)));
     RC(enq_search(c, s));
     CK(cudaStreamSynchronize(s));
@@ -1232,7 +1249,7 @@ int nn_time_kernel(nn_ctx* c, int32_t kernel, int32_t reps, float* ms_out) {
     // the slots of the last search are sorted by the positions before its step's
     // advection: sort the current ones again (from the slots), so the timed builds see
     // the cell ranges a step's build sees
-    CK(cudaMemsetAsync(c->d_src_flag, 0, sizeof(int32_t), s));
+    RC(set_src(c, s, 0));
     RC(launch1(c, s, k_step_reset, make_dev(c, c->cur)));
     RC(enq_search(c, s));
   }
