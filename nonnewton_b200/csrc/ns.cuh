@@ -77,51 +77,49 @@ __global__ void k_keys(Dev d) {
   }
 }
 
-// Exclusive scan of cell_count[0 .. cells] in place (two phases over tiles).
-#define SCAN_TILE 4096
+// Exclusive scan of cell_count[0 .. cells] in place (two phases over tiles). A warp takes
+// SCAN_PER * 32 consecutive counts as 16-byte loads, and a block, one tile with one barrier
+// between its warps' scans; 16,384 counts a tile give the blocks of a 3M-cell grid one tile
+// each (4,096 with a 4-byte load per count and six barriers a tile: 32 us for both kernels at
+// 900,000 particles, 14 so; 33 and 16 at 2.4M).
+#define SCAN_TILE 16384
 #define SCAN_THREADS 1024
-__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* sh, uint32_t* total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t x = v;
+#define SCAN_ROUNDS (SCAN_TILE / SCAN_THREADS / 4)
+__device__ __forceinline__ int scan_at(int t, int r) {  // this thread's 4 counts of round r
+  return t * SCAN_TILE + (int)(threadIdx.x >> 5) * (SCAN_ROUNDS * 128) + r * 128 + (int)(threadIdx.x & 31) * 4;
+}
+__device__ __forceinline__ uint4 scan_load(const uint32_t* a, int i, int len) {
+  if (i + 4 <= len) return *reinterpret_cast<const uint4*>(a + i);
+  return make_uint4(i < len ? a[i] : 0u, i + 1 < len ? a[i + 1] : 0u, i + 2 < len ? a[i + 2] : 0u, 0u);
+}
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+    const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
   }
-  if (lane == 31) sh[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    uint32_t w = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0u;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    sh[lane] = w;
-  }
-  __syncthreads();
-  uint32_t base = wid > 0 ? sh[wid - 1] : 0u;
-  uint32_t incl = base + x;
-  if (total) *total = sh[(blockDim.x >> 5) - 1];
-  __syncthreads();
-  return incl - v;
+  return v;
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(Dev d) {
   __shared__ uint32_t sh[32];
   const int len = d.d_n[2] + 1;
   const int ntiles = (len + SCAN_TILE - 1) / SCAN_TILE;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     uint32_t s = 0;
-    for (int k = threadIdx.x; k < SCAN_TILE; k += blockDim.x) {
-      int i = t * SCAN_TILE + k;
-      if (i < len) s += d.cell_count[i];
+#pragma unroll
+    for (int r = 0; r < SCAN_ROUNDS; ++r) {
+      const uint4 v = scan_load(d.cell_count, scan_at(t, r), len);
+      s += v.x + v.y + v.z + v.w;
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    s = __reduce_add_sync(0xffffffffu, s);
+    if (lane == 0) sh[wid] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t tot = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += sh[w];
-      d.tile_sums[t] = tot;
+    if (wid == 0) {
+      const uint32_t tot = __reduce_add_sync(0xffffffffu, sh[lane]);
+      if (lane == 0) d.tile_sums[t] = tot;
     }
     __syncthreads();
   }
@@ -131,32 +129,51 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(Dev d) {
 // walk the tiles in order, so each reads about as many tile sums as there are tiles),
 // then scans its tile. A separate one-block scan of the tile sums would cost a launch.
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(Dev d) {
-  __shared__ uint32_t sh[32];
+  static_assert(SCAN_THREADS == 1024, "32 warps, one lane each");
+  __shared__ uint32_t sh[32], sh_part[32];
   const int len = d.d_n[2] + 1;
   const int ntiles = (len + SCAN_TILE - 1) / SCAN_TILE;
-  constexpr int PER = SCAN_TILE / SCAN_THREADS;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint32_t before = 0;  // sum of tile_sums[0 .. done)
   int done = 0;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    uint32_t part = 0, tot = 0;
+    uint32_t part = 0;
     for (int k = done + (int)threadIdx.x; k < t; k += blockDim.x) part += d.tile_sums[k];
-    block_excl_scan(part, sh, &tot);
-    before += tot;
-    done = t;
-    uint32_t v[PER];
-    uint32_t s = 0;
+    uint4 v[SCAN_ROUNDS];
+    uint32_t ex[SCAN_ROUNDS], tot = 0;
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      int i = t * SCAN_TILE + threadIdx.x * PER + k;
-      v[k] = i < len ? d.cell_count[i] : 0u;
-      s += v[k];
+    for (int r = 0; r < SCAN_ROUNDS; ++r) v[r] = scan_load(d.cell_count, scan_at(t, r), len);
+#pragma unroll
+    for (int r = 0; r < SCAN_ROUNDS; ++r) {
+      const uint32_t s = v[r].x + v[r].y + v[r].z + v[r].w, incl = warp_incl_scan(s);
+      ex[r] = tot + incl - s;
+      tot += __shfl_sync(0xffffffffu, incl, 31);
     }
-    uint32_t ex = block_excl_scan(s, sh, nullptr) + before;
+    part = __reduce_add_sync(0xffffffffu, part);
+    if (lane == 0) {
+      sh[wid] = tot;
+      sh_part[wid] = part;
+    }
+    __syncthreads();
+    const uint32_t w = sh[lane];
+    const uint32_t base = __shfl_sync(0xffffffffu, warp_incl_scan(w) - w, wid);
+    before += __reduce_add_sync(0xffffffffu, sh_part[lane]);
+    done = t;
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      int i = t * SCAN_TILE + threadIdx.x * PER + k;
-      if (i < len) d.cell_count[i] = ex;
-      ex += v[k];
+    for (int r = 0; r < SCAN_ROUNDS; ++r) {
+      const int i = scan_at(t, r);
+      uint4 o;
+      o.x = before + base + ex[r];
+      o.y = o.x + v[r].x;
+      o.z = o.y + v[r].y;
+      o.w = o.z + v[r].z;
+      if (i + 4 <= len) {
+        *reinterpret_cast<uint4*>(d.cell_count + i) = o;
+      } else {
+        if (i < len) d.cell_count[i] = o.x;
+        if (i + 1 < len) d.cell_count[i + 1] = o.y;
+        if (i + 2 < len) d.cell_count[i + 2] = o.z;
+      }
     }
     __syncthreads();
   }
