@@ -185,15 +185,42 @@ __global__ void k_scatter(Dev d) {
 }
 
 // In-cell order by particle id, so that the slot order (and every neighbour sum)
-// does not depend on the atomics of k_keys. A cell of up to NS_SORT_REG particles is
-// sorted by its own thread in registers, one of up to NS_SORT_SMALL by its own thread
-// in place (insertion sort); a crowded cell (a cluster) by the
+// does not depend on the atomics of k_keys. A cell of up to 16 particles is sorted by its
+// own thread in registers, one of up to NS_SORT_SMALL by its own thread in place (insertion
+// sort, a chain of dependent loads: 17.5 us of an 85,147-slot pool's step when it took
+// the cells of 9 to 16 too, 4 now); a crowded cell (a cluster) by the
 // whole warp: each lane ranks some of its particles by counting the smaller ids, so
 // a cell of n particles takes n^2 / 32 steps per lane instead of about n^2 / 4 on one
 // thread. Particle ids are distinct, so the ranks are a permutation. The scratch of
 // the warp path is the key array, which nothing reads after k_scatter.
 #define NS_SORT_SMALL 24
-#define NS_SORT_REG 8
+#define NS_SORT_REG 16
+// The sources and their ids load together (no chain of dependent loads per comparison), a
+// bitonic network sorts N slots whose unused tail holds the largest key, and the sources go
+// back in id order.
+template <int N>
+__device__ __forceinline__ void sort_cell(int* src, const int* ids, uint32_t n, bool truth) {
+  int sv[N], kv[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) sv[q] = (uint32_t)q < n ? src[q] : 0;
+#pragma unroll
+  for (int q = 0; q < N; ++q) kv[q] = (uint32_t)q < n ? (truth ? sv[q] : ids[sv[q]]) : INT_MAX;
+#pragma unroll
+  for (int k = 2; k <= N; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const int l = i ^ j;
+        if (l > i && ((i & k) == 0 ? kv[i] > kv[l] : kv[i] < kv[l])) {
+          const int tk = kv[i]; kv[i] = kv[l]; kv[l] = tk;
+          const int ts = sv[i]; sv[i] = sv[l]; sv[l] = ts;
+        }
+      }
+#pragma unroll
+  for (int q = 0; q < N; ++q)
+    if ((uint32_t)q < n) src[q] = sv[q];
+}
 __global__ void k_cell_sort(Dev d) {
   const int nc = d.d_n[2];
   const bool truth = *d.src_from_truth != 0;
@@ -203,26 +230,10 @@ __global__ void k_cell_sort(Dev d) {
     uint32_t b = 0, e = 0;
     if (valid) { b = d.cell_count[c]; e = d.cell_count[c + 1]; }
     const uint32_t n = e - b;
-    if (n >= 2 && n <= NS_SORT_REG) {
-      // in registers: the sources and their ids load together (no chain of dependent
-      // loads per comparison), an odd-even transposition network sorts NS_SORT_REG slots
-      // whose unused tail holds the largest key, and the sources go back in id order
-      int sv[NS_SORT_REG], kv[NS_SORT_REG];
-#pragma unroll
-      for (int q = 0; q < NS_SORT_REG; ++q) sv[q] = (uint32_t)q < n ? d.src[b + q] : 0;
-#pragma unroll
-      for (int q = 0; q < NS_SORT_REG; ++q) kv[q] = (uint32_t)q < n ? (truth ? sv[q] : d.wo.id[sv[q]]) : INT_MAX;
-#pragma unroll
-      for (int r = 0; r < NS_SORT_REG; ++r)
-#pragma unroll
-        for (int q = r & 1; q + 1 < NS_SORT_REG; q += 2)
-          if (kv[q] > kv[q + 1]) {
-            const int tk = kv[q]; kv[q] = kv[q + 1]; kv[q + 1] = tk;
-            const int ts = sv[q]; sv[q] = sv[q + 1]; sv[q + 1] = ts;
-          }
-#pragma unroll
-      for (int q = 0; q < NS_SORT_REG; ++q)
-        if ((uint32_t)q < n) d.src[b + q] = sv[q];
+    if (n >= 2 && n <= 8) {
+      sort_cell<8>(d.src + b, d.wo.id, n, truth);
+    } else if (n > 8 && n <= NS_SORT_REG) {
+      sort_cell<NS_SORT_REG>(d.src + b, d.wo.id, n, truth);
     } else if (n > NS_SORT_REG && n <= NS_SORT_SMALL) {
       for (uint32_t i = b + 1; i < e; ++i) {
         int s = d.src[i];

@@ -1,5 +1,7 @@
-"""The search's scan (16,384 counts a tile, 16-byte loads, a ragged end): lists against brute
-force over grids on both sides of a tile."""
+"""The search's scan (16,384 counts a tile, 16-byte loads, a ragged end) and its in-cell sort
+(registers up to 16 particles, in place up to 24, a warp above): lists against brute force
+over grids on both sides of a tile, and slot orders that do not depend on the atomics."""
+import numpy as np
 import pytest
 import torch
 
@@ -28,3 +30,25 @@ def test_lists_over_grid_sizes(cuda_lib, box):
     i, j = near.nonzero(as_tuple=True)
     want[i, torch.arange(len(i), device="cuda") - (near.sum(1).cumsum(0) - near.sum(1))[i]] = j.int()
     assert torch.equal(num, near.sum(1).int()) and torch.equal(lists, want)
+
+
+def test_slot_order_of_crowded_cells(cuda_lib):
+    """Cells of 1 to 34 particles: three steps (the first sorts the caller's order, the others
+    the previous slots) give the same bits every time, so the order in a cell is the ids'."""
+    sc = S.dam_break(seed=2, n_side=(14, 11, 9), box=0.5)
+    x, nf, rng = sc.particles.x, sc.particles.n_fluid, np.random.default_rng(4)
+    ids, at = rng.permutation(nf), 0
+    for k in range(1, 35):
+        c = np.array([3 + k % 7, 2 + k // 7, 8], np.float32) * 0.04  # a cell's lower corner
+        x[ids[at:at + k]] = c + rng.uniform(0.005, 0.035, (k, 3)).astype(np.float32)
+        at += k
+    out = []
+    for _ in range(4):
+        m = sph.initialize(SimConfig(config=sc.config), particles=sc.particles, max_neighbors=256)
+        solver = sph.build_solver()
+        solver.initialize()
+        m.engine.step(3)
+        out.append([m.pd.x.clone(), m.pd.v.clone(), m.pd.density.clone()])
+    for o in out[1:]:
+        for a, b in zip(o, out[0]):
+            assert torch.equal(a, b)
