@@ -115,7 +115,7 @@ struct SceneDyn {
   int32_t np_last;                // index of the last divergence loop body of the last step
   double max_avg_p;               // largest avg_p at the end of a step since the scene was set
   int32_t np_fresh;               // this step's non-pressure terms came from body np_body, the last
-  int32_t pad;
+  int32_t dyn_solids;             // the step's search met a dynamic solid
 };
 
 // Accumulator slots per scene (each NN_STRIPES doubles).

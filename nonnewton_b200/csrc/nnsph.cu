@@ -426,7 +426,7 @@ static int set_src(nn_ctx* c, cudaStream_t s, int v) {
 // ---- pass sequences ---------------------------------------------------------------
 // NeighborhoodSearchSparse.run_search (SPH/main.py:822-829): the new slots go into the
 // other working set; the source (caller state or previous slots) is a device flag.
-// `reset_step`: the step's first launch (k_zero_cells) also resets its per-scene counters.
+// `reset_step`: in a step, whose first launch (k_zero_cells) also resets its per-scene counters.
 static int enq_search(nn_ctx* c, cudaStream_t s, bool reset_step = false) {
   c->cur = 1 - c->cur;
   Dev d = make_dev(c, c->cur);
@@ -439,7 +439,7 @@ static int enq_search(nn_ctx* c, cudaStream_t s, bool reset_step = false) {
   RC(launch_g(c, s, k_scan_apply, std::min(tiles, c->sms * 2), SCAN_THREADS, d));
   RC(launch(c, s, k_scatter, B, c->n, d));
   RC(launch(c, s, k_cell_sort, B, (int)std::min<int64_t>(cells, INT32_MAX), d));
-  RC(launch(c, s, k_gather, B, c->n, d));
+  RC(launch(c, s, k_gather, B, c->n, d, !reset_step ? 0 : c->fold_np ? 2 : 1));
   RC(enq_build_lists(c, s, d));
   c->searched = true;
   return NN_OK;
@@ -492,7 +492,7 @@ static int enq_divergence(nn_ctx* c, cudaStream_t s, bool fused) {
 
 // DFSPHSolver.pressure_solve (SPH/main.py:1762-1791); init_mode 2 also folds the
 // divergence solve's alpha *= dt.
-// `begun`: the loop start is done (k_clear_acc at the start of the step).
+// `begun`: the loop start is done (k_boundary_volume at the start of the step).
 static int enq_pressure(nn_ctx* c, cudaStream_t s, int init_mode, bool begun = false) {
   Dev d = make_dev(c, c->cur);
   const int B = c->block;
@@ -575,7 +575,7 @@ static int enq_rigid(nn_ctx* c, cudaStream_t s) {
 }
 
 // DFSPHSolver.substep (SPH/main.py:1546-1555) with the fused passes.
-// `begun`: the loops' start is done (k_clear_acc at the start of the step).
+// `begun`: the loops' start is done (k_boundary_volume at the start of the step).
 static int enq_substep(nn_ctx* c, cudaStream_t s, bool begun = false) {
   if (!c->any_fluid) return NN_OK;
   Dev d = make_dev(c, c->cur);
@@ -593,11 +593,10 @@ static int enq_substep(nn_ctx* c, cudaStream_t s, bool begun = false) {
 // SPHBase.step (SPH/main.py:915-937)
 static int enq_step(nn_ctx* c, cudaStream_t s) {
   // k_step_reset rides in the search's first launch, k_step_dt and the solves' loop
-  // start in k_clear_acc's first block: one-block kernels cost a graph node each
+  // start in k_boundary_volume's first block: one-block kernels cost a graph node each
   RC(enq_search(c, s, true));
   Dev d = make_dev(c, c->cur);
-  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1));
-  RC(launch(c, s, k_clear_acc, 256, c->n, d, c->fold_np ? 1 : 0, 1));
+  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1, 1));
   RC(enq_substep(c, s, true));
   RC(enq_elastic(c, s));
   RC(enq_rigid(c, s));
@@ -1151,8 +1150,8 @@ int nn_initialize(nn_ctx* c) {
     RC(launch(c, s, k_rigid_com, 256, c->n, d, r, 1));
     RC(launch1(c, s, k_rigid_cm, d, r, 1));
   }
-  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 0));
-  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1));
+  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 0, 0));
+  RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1, 0));
   RC(enq_sync_out(c, s, SM_VOL));
   CK(cudaStreamSynchronize(s));
   c->el_stale = false;
@@ -1208,9 +1207,9 @@ int nn_run_pass(nn_ctx* c, int32_t pass) {
   RC(launch(c, s, k_sync_in, 256, c->n, d, (uint32_t)SM_ALL));
   RC(launch1(c, s, k_step_dt, d, 0));
   switch (pass) {
-    case NN_PASS_STATIC_BOUNDARY_VOLUME: RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 0)); break;
-    case NN_PASS_MOVING_BOUNDARY_VOLUME: RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1)); break;
-    case NN_PASS_CLEAR_ACCELERATIONS: RC(launch(c, s, k_clear_acc, 256, c->n, d, 0, 0)); break;
+    case NN_PASS_STATIC_BOUNDARY_VOLUME: RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 0, 0)); break;
+    case NN_PASS_MOVING_BOUNDARY_VOLUME: RC(launch_nb(c, s, KU(k_boundary_volume, U_BOUNDARY_VOLUME), c->block, d, 1, 0)); break;
+    case NN_PASS_CLEAR_ACCELERATIONS: RC(launch(c, s, k_clear_acc, 256, c->n, d)); break;
     case NN_PASS_DENSITIES: RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 1, 0)); break;
     case NN_PASS_DFSPH_FACTOR: RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 0, 1)); break;
     case NN_PASS_DIVERGENCE_SOLVE: if (c->any_div) RC(enq_divergence(c, s, false)); break;

@@ -43,6 +43,7 @@ __device__ __forceinline__ void step_reset_scenes(const Dev& d) {
     y.it_v = y.it_p = y.it_cg = 0;
     y.div_ran = 0;
     y.np_fresh = 0;
+    y.dyn_solids = 0;
   }
 }
 
@@ -282,8 +283,13 @@ __device__ __forceinline__ uint32_t class_bits(int material, int dynamic, int ph
 }
 
 // Gather the state into the new slot order (from Truth by id, or from the previous
-// slots), and record max |v| per scene for the CFL step.
-__global__ void k_gather(Dev d) {
+// slots), and record max |v| per scene for the CFL step. `step`, in a step: also which scenes
+// have dynamic solids, and the accelerations that the force pass will not clear: those of
+// scenes without fluid and, when the divergence loop's last density change carries the fluid's
+// non-pressure terms (step 2), what the force pass would write for the solids of the others
+// (strain rate and viscosity 0, CG coefficients (0, 1 if dynamic)). A clear pass of its own
+// took 12 us on 2.4M slots.
+__global__ void k_gather(Dev d, int step) {
   const int n = d.d_n[0];
   const int mode = *d.src_from_truth;
   const bool truth = mode != 0;
@@ -325,6 +331,15 @@ __global__ void k_gather(Dev d) {
       d.w.id[i] = id;
       d.slot_of_id[id] = i;
       vm = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
+      const SceneDev& sc = d.sc[slot_scene(fl)];
+      if (step && (sc.n_fluid == 0 || (step == 2 && !cls_fluid(fl)))) {
+        d.acc4[i] = cls_static_solid(fl) ? make_real4(0.f, 0.f, 0.f, 0.f) : make_real4(sc.g[0], sc.g[1], sc.g[2], 0.f);
+        if (step == 2 && sc.n_fluid > 0 && !cls_fluid(fl)) {
+          if (sc.flags & NN_F_NONNEWTON) { d.srn[i] = 0.f; d.mu[i] = 0.f; }
+          if (scene_implicit(sc)) d.cg_aux[i] = make_real2(0.f, cls_dyn_solid(fl) ? 1.f : 0.f);
+        }
+      }
+      if (cls_dyn_solid(fl)) d.dyn[slot_scene(fl)].dyn_solids = 1;  // every writer the same value
     }
     const bool cfl = valid && (fl & NN_CLS_DYNAMIC) && (d.sc[slot_scene(fl)].flags & NN_F_CFL);
     warp_max_to(&d.dyn[slot_scene(fl)].vmax_bits, __float_as_uint((float)vm), cfl);

@@ -17,11 +17,32 @@
     for (int j = (d).nbr[(size_t)_k * (d).cap + (i)], _o = 1; _o; _o = 0)
 
 
+// A one-lane launch that no scene has work for (`need`) ends before it reads the slots' flags
+// (9-12 us on 2.4M slots, 2-3 so): a body's other instance, terms that are fresh, scenes
+// without dynamic solids. Batches of more than a warp's scenes always go on.
+template <typename F>
+__device__ __forceinline__ bool no_scene(const Dev& d, F need) {
+  const int ns = d.d_n[1], lane = threadIdx.x & 31;
+  return ns <= 32 && !__any_sync(0xffffffffu, lane < ns && need(d.sc[lane], d.dyn[lane]));
+}
+
 // ---------------------------------------------------------------------------
 // compute_static_boundary_volume / compute_moving_boundary_volume (SPH/main.py:1010-1035)
+// `step_start`: block 0 also takes the step's time step (k_step_dt with the CFL rule)
+// and the divergence and pressure solves' loop start, which nothing reads before this pass.
+__device__ __forceinline__ void step_dt_scenes(const Dev& d, int do_cfl);
+__device__ __forceinline__ void solver_begin_scene(SceneDyn& y, const SceneDev& s, int which);
 template <int U, int L>
-__global__ void k_boundary_volume(Dev d, int moving) {
+__global__ void k_boundary_volume(Dev d, int moving, int step_start) {
+  if (step_start && blockIdx.x == 0) {
+    step_dt_scenes(d, 1);
+    for (int sc = threadIdx.x; sc < d.d_n[1]; sc += blockDim.x) {
+      solver_begin_scene(d.dyn[sc], d.sc[sc], 0);
+      solver_begin_scene(d.dyn[sc], d.sc[sc], 1);
+    }
+  }
   const int n = d.d_n[0];
+  if (L == 1 && moving && no_scene(d, [](const SceneDev&, const SceneDyn& y) { return y.dyn_solids != 0; })) return;
   FOR_SPLIT(L, i, sub, valid, n) {
     const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const bool work = valid && (moving ? cls_dyn_solid(fl) : cls_static_solid(fl));
@@ -40,31 +61,14 @@ __global__ void k_boundary_volume(Dev d, int moving) {
   }
 }
 
-// clear_accelerations_kernel (SPH/main.py:945-951). With `solid_terms` also what the
-// force pass would write for the solid slots of scenes with fluid (strain rate and
-// viscosity 0, CG coefficients (0, 1 if dynamic)): the step sets it when the fluid's
-// non-pressure terms come from the divergence loop's last density change instead.
-// `step_start`: block 0 also takes the step's time step (k_step_dt with the CFL rule)
-// and the divergence and pressure solves' loop start, which nothing reads before them.
-__device__ __forceinline__ void step_dt_scenes(const Dev& d, int do_cfl);
-__device__ __forceinline__ void solver_begin_scene(SceneDyn& y, const SceneDev& s, int which);
-__global__ void k_clear_acc(Dev d, int solid_terms, int step_start) {
-  if (step_start && blockIdx.x == 0) {
-    step_dt_scenes(d, 1);
-    for (int sc = threadIdx.x; sc < d.d_n[1]; sc += blockDim.x) {
-      solver_begin_scene(d.dyn[sc], d.sc[sc], 0);
-      solver_begin_scene(d.dyn[sc], d.sc[sc], 1);
-    }
-  }
+// clear_accelerations_kernel (SPH/main.py:945-951) as a pass of its own; the step's clear is
+// k_gather's and the force pass's.
+__global__ void k_clear_acc(Dev d) {
   const int n = d.d_n[0];
   GRID_STRIDE(i, n) {
     const uint32_t fl = d.w.flags[i];
     const SceneDev& s = d.sc[slot_scene(fl)];
     d.acc4[i] = cls_static_solid(fl) ? make_real4(0.f, 0.f, 0.f, 0.f) : make_real4(s.g[0], s.g[1], s.g[2], 0.f);
-    if (solid_terms && !cls_fluid(fl) && s.n_fluid > 0) {
-      if (s.flags & NN_F_NONNEWTON) { d.srn[i] = 0.f; d.mu[i] = 0.f; }
-      if (scene_implicit(s)) d.cg_aux[i] = make_real2(0.f, cls_dyn_solid(fl) ? 1.f : 0.f);
-    }
   }
 }
 
@@ -165,7 +169,7 @@ __device__ __forceinline__ void strain_term(real3 v, real3 g, real (&e)[6]) {
 // last body of its previous step) runs this instance; when the prediction holds,
 // k_solver_check marks the terms fresh and the force pass skips the scene. The step
 // uses it when no scene needs the force pass's other terms (explicit viscosity, quirk
-// mode); the solids' outputs come from k_clear_acc.
+// mode); the solids' outputs come from k_gather.
 // `sel` = 1 in such a loop: the plain instance skips, and the NP instance takes, the
 // scenes whose np_body this body is; 0: every scene.
 struct TDiv { real V, dv; };  // volume, v_ij . grad W
@@ -174,6 +178,10 @@ struct TDivNp { real V, dv, sx, sy, sz, sw, m, e[6]; };
 template <int U, int L, bool NP, bool COH = false>
 __device__ __forceinline__ void density_change_body(const Dev& d, int mode, int sel) {
   const int n = d.d_n[0];
+  if (L == 1 && no_scene(d, [&](const SceneDev&, const SceneDyn& y) {
+        return y.act_v && (!sel || NP == (y.it_v == y.np_body));
+      }))
+    return;
   FOR_SPLIT(L, i, sub, valid, n) {
     uint32_t fl = valid ? d.w.flags[i] : 0u;
     const int scn = slot_scene(fl);
@@ -661,6 +669,7 @@ template <int U, int L, int FF>
 __device__ __forceinline__ void forces_body(const Dev& d, int clear) {
   static_assert(!(FF & FF_Q) || L == 1, "quirk mode keeps one lane per particle");
   const int n = d.d_n[0];
+  if (L == 1 && no_scene(d, [](const SceneDev& s, const SceneDyn& y) { return s.n_fluid != 0 && !y.np_fresh; })) return;
   FOR_SPLIT(L, i, sub, valid, n) {
     const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const bool fluid = cls_fluid(fl);
