@@ -3,7 +3,8 @@
 // One step (SPHBase.step, SPH/main.py:915-940) is a fixed sequence of kernels; the
 // three data-dependent solver loops (divergence, implicit-viscosity CG, pressure)
 // become CUDA-graph while-nodes whose condition is set on the device by the loop's
-// check kernel, so a step runs without a host round-trip. A host-driven mode (one
+// check kernel, or, in small scenes, one cooperative kernel each (one_kernel_loops), so a
+// step runs without a host round-trip. A host-driven mode (one
 // stream sync per iteration, like the reference's Python loops) is kept for the
 // per-pass API and as a fallback.
 #include <cuda_runtime.h>

@@ -42,7 +42,8 @@ __global__ void k_boundary_volume(Dev d, int moving, int step_start) {
     }
   }
   const int n = d.d_n[0];
-  if (L == 1 && moving && no_scene(d, [](const SceneDev&, const SceneDyn& y) { return y.dyn_solids != 0; })) return;
+  // (dyn_solids is this step's: the gather of its search set it)
+  if (L == 1 && step_start && no_scene(d, [](const SceneDev&, const SceneDyn& y) { return y.dyn_solids != 0; })) return;
   FOR_SPLIT(L, i, sub, valid, n) {
     const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const bool work = valid && (moving ? cls_dyn_solid(fl) : cls_static_solid(fl));
