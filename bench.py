@@ -55,29 +55,31 @@ ALG_BYTES = {
 # loop's predicted last body) reads mass and density besides and writes acc4, srn, mu, aux2
 ALG_BYTES["density_change_np"] = ALG_BYTES["density_change"] + 4 + 4 + 16 + 4 + 4 + 8
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch on the
-# 2.4M-particle dam break, from `ncu --set full` captures of the current kernels.
-# list entries of the captured k_build_lists launch (step 5 of the 2.4M scene); the line
+# 2.4M-particle dam break, from ncu captures of the current kernels; "nonpressure" and
+# "density_change", which have no work in that step, from captures with positions and
+# velocities in separate arrays.
+# list entries of the captured k_build_lists launch (an early step of the 2.4M scene); the line
 # scales that launch's traffic to the timed launch's entries, which the bytes follow
 NCU_ENTRIES_2M = 62_580_972
-NCU_TRAFFIC_2M = {"build_lists": 477530368, "density_adv": 372967680,
-                  "nonpressure": 431172096, "density_factor": 365270272,
-                  "density_change": 366368512, "divergence_update": 376274432,
-                  "pressure_update": 383854080, "cg_matvec": 433442816, "density_change_np": 430826240,
-                  "cg_setup": 567003648}
+NCU_TRAFFIC_2M = {"build_lists": 505586688, "density_adv": 414270976,
+                  "nonpressure": 431172096, "density_factor": 398540800,
+                  "density_change": 366368512, "divergence_update": 425979136,
+                  "pressure_update": 414269952, "cg_matvec": 431102976, "density_change_np": 464528128,
+                  "cg_setup": 610421248}
 # what bounds each kernel instead of DRAM, from its ncu capture on the 2.4M scene:
 # the HBM fraction above is low because none is DRAM-bound
 LIMITER_2M = {
-    "build_lists": "instruction issue: 72 % issue active, ~160 exact f32 distance tests per particle, two per packed f32x2 instruction; DRAM 13 %",
-    "density_adv": "L1 data pipe: LSU wavefronts at 78 % of peak (neighbour gathers); DRAM 19 %",
+    "build_lists": "instruction issue: 68 % issue active, ~160 exact f32 distance tests per particle, two per packed f32x2 instruction; LSU wavefronts 60 %; DRAM 15 %",
+    "density_adv": "L1 data pipe: LSU wavefronts at 78 % of peak (256-bit neighbour gathers), 47 % warps active; DRAM 23 %",
     "nonpressure": "L1 data pipe and gather latency: LSU wavefronts 62 %, 46 % warps active; DRAM 13 %",
-    "density_factor": "gather latency: LSU wavefronts 64 %, issue 64 %, 53 % warps active; DRAM 15 %",
+    "density_factor": "L1 data pipe: LSU wavefronts 75 %, issue 65 %, 52 % warps active; DRAM 19 %",
     "density_change": "L1 data pipe: LSU wavefronts 85 % of peak; DRAM 18 %",
-    "divergence_update": "L1 data pipe: LSU wavefronts 65 % of peak, 64 % issue active; DRAM 20 %",
-    "pressure_update": "L1 data pipe: LSU wavefronts 72 % of peak; DRAM 24 %",
-    "cg_matvec": "gather latency: LSU wavefronts 66 %, issue 63 %, 46 % warps active at 64 registers; DRAM 20 %",
-    "cg_setup": "L1 data pipe and gather latency: LSU wavefronts 72 %, issue 64 %, 46 % warps active; DRAM 21 %",
-    "density_change_np": "gather latency with the folded force terms: LSU wavefronts 55 %, issue 68 %, "
-                         "46 % warps active at 64 registers; DRAM 13 %",
+    "divergence_update": "gather latency and issue: LSU wavefronts 59 %, 66 % issue active, 50 % warps active; DRAM 24 %",
+    "pressure_update": "L1 data pipe: LSU wavefronts 74 % of peak, 43 % issue active; DRAM 32 %",
+    "cg_matvec": "L1 data pipe: LSU wavefronts 75 %, issue 63 %, 53 % warps active at 56 registers; DRAM 22 %",
+    "cg_setup": "L1 data pipe: LSU wavefronts 80 %, issue 63 %, 47 % warps active at 64 registers; DRAM 24 %",
+    "density_change_np": "issue and gather latency with the folded force terms: LSU wavefronts 59 %, issue 67 %, "
+                         "46 % warps active at 64 registers; DRAM 14 %",
 }
 KERNEL_IDS = {"pressure_update": 0, "density_adv": 1, "divergence_update": 2, "density_change": 3,
               "density_factor": 4, "build_lists": 5, "cg_matvec": 6, "nonpressure": 7, "density_change_np": 8,
