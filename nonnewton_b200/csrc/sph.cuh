@@ -593,6 +593,14 @@ __global__ void k_set_int(int32_t* p, int32_t v) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *const_cast<int32_t*>(p) = v;
 }
 
+// A scene's (status, max_nb) into the caller's mapped pinned memory.
+__global__ void k_status_out(Dev d, int scene, int32_t* out) {
+  if (threadIdx.x == 0) {
+    out[0] = d.dyn[scene].status;
+    out[1] = d.dyn[scene].max_nb;
+  }
+}
+
 __global__ void k_step_end(Dev d) {
   const int ns = d.d_n[1];
   for (int sc = threadIdx.x; sc < ns; sc += blockDim.x) {

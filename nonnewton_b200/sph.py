@@ -134,8 +134,7 @@ class SPHBase:
         self.host_loop = False
         # re-run a step whose neighbour lists overflowed, with a larger cap
         self.grow_neighbors = True
-        self._snap = None          # x and v that the last call started from
-        self._spare = None         # ... and where the next call keeps its own
+        self._snap = None
         self._status = None
         self._pending = None       # the last call's unchecked status copy
         self._last_max = None      # largest neighbour count last seen
@@ -182,42 +181,31 @@ class SPHBase:
         A call whose last known neighbour count is within a quarter of the capacity
         reads the scene's status right after its steps (one host synchronisation).
         Otherwise the status is copied to pinned memory without waiting and checked
-        when the next call has enqueued its own steps (or by stats()), so that the device
-        does not wait for the host between two calls (a step of 3,933 particles 139 ->
-        136 us, 23,002 157 -> 153, 85,147 427 -> 421); in the rare case that it overflowed, the state it started from is restored, its
-        steps run again, checked, and the new call's after them. Until then meta.pd
-        holds that call's unverified result."""
+        when the next call (or stats()) begins; in the rare case that it overflowed,
+        the state it started from is restored and its steps run again, checked, before
+        the new work. Until then meta.pd holds that call's unverified result."""
         eng = self.engine
         if not self.grow_neighbors:
             if displacement is not None:
                 eng.set_animation(0, displacement)
             eng.step(nsteps, sync=True, host_loop=self.host_loop)
             return
+        self._settle()
         pd = meta.pd
         if self._snap is None or self._snap[0].shape != pd.x.shape:
-            self._settle()
-            n = pd.x.shape[0]  # one allocation (a call's first pays for it), 16-byte aligned parts
-            buf = pd.x.new_empty((4, (n + 3) // 4 * 4, pd.x.shape[1]))
-            self._snap, self._spare = (buf[0, :n], buf[1, :n]), (buf[2, :n], buf[3, :n])
+            self._snap = (torch.empty_like(pd.x), torch.empty_like(pd.v))
             self._status = torch.zeros(2, dtype=torch.int32, pin_memory=torch.cuda.is_available())
-        self._start(nsteps, displacement)
-        if self._settle():  # ran the previous call again: this one starts from its new state
-            self._start(nsteps, displacement)
-        self._snap, self._spare = self._spare, self._snap
-        if self._last_max is None or 4 * self._last_max >= 3 * eng.max_neighbors:
+        self._snap[0].copy_(pd.x)
+        self._snap[1].copy_(pd.v)
+        near = self._last_max is None or 4 * self._last_max >= 3 * eng.max_neighbors
+        if displacement is not None:
+            eng.set_animation(0, displacement)
+        eng.step(nsteps, sync=True, host_loop=self.host_loop)
+        if near:
             self._check(nsteps, displacement)
         else:
             eng.status_async(self._status)
             self._pending = (nsteps, displacement)
-
-    def _start(self, nsteps, displacement):
-        """Enqueue steps, with the state they start from kept in the spare buffers (the
-        pending call's own start is needed until its status is known)."""
-        self._spare[0].copy_(meta.pd.x)
-        self._spare[1].copy_(meta.pd.v)
-        if displacement is not None:
-            self.engine.set_animation(0, displacement)
-        self.engine.step(nsteps, sync=True, host_loop=self.host_loop)
 
     def _check(self, nsteps, displacement):
         """Status after the steps just enqueued: on overflow, grow and run them again."""
@@ -241,10 +229,10 @@ class SPHBase:
             eng.set_animation(0, displacement)
         eng.step(nsteps, sync=True, host_loop=self.host_loop)
 
-    def _settle(self) -> bool:
-        """Check the previous call's status copy (see _advance); whether its steps ran again."""
+    def _settle(self):
+        """Check the previous call's status copy (see _advance)."""
         if self._pending is None:
-            return False
+            return
         nsteps, displacement = self._pending
         self._pending = None
         self.engine.status_wait()
@@ -253,8 +241,6 @@ class SPHBase:
         if status == _abi.NN_ERR_NEIGHBOR_OVERFLOW:
             self._rerun(nsteps, displacement, seen)
             self._check(nsteps, displacement)
-            return True
-        return False
 
     def _grow_cap(self, st):
         cap = max(st["max_neighbors_seen"], self.engine.max_neighbors) * 5 // 4
