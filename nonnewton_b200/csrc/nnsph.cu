@@ -1044,9 +1044,11 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
   c->n_fluid = 0;
   for (int k = 0; k < nscenes; ++k) c->n_fluid += scenes[k].n_fluid;
   c->lanes = lanes_for(c, c->n_fluid);
-  // elastic buffers are reallocated below (their pointers and stride are graph arguments)
-  if (feature_sig(c) != c->graph_sig || c->ne > 0) drop_graphs(c);
-  c->scenes.assign(scenes, scenes + nscenes);
+  // elastic and rigid-body buffers are freed and reallocated below: their pointers, strides and
+  // counts are graph arguments, those of the old set as well (a set without bodies after one with
+  // bodies has the same features)
+  if (feature_sig(c) != c->graph_sig || c->ne > 0 || c->n_rb > 0 || !rb_list.empty()) drop_graphs(c);
+  c->scenes.clear();  // no step until every buffer is there again
   c->sdev = sdev;
   c->n = n;
   c->ncells = (int)cells;
@@ -1107,12 +1109,12 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
     CK(cudaMemcpy(c->rb_of_id, rb_of.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c->rb_round, rounds.data(), B * sizeof(int32_t), cudaMemcpyHostToDevice));
     CK(cudaMemset(c->rb_acc, 0, B * 13 * sizeof(double)));
-    drop_graphs(c);  // body buffers and counts are graph arguments
   }
   if (nscenes > 0 && n > 0) {  // scene of every particle id, filled from the scene table on the device
     k_scene_of_id<<<std::min(nscenes, 65535), 256>>>(make_dev(c, c->cur));
     CK(cudaGetLastError());
   }
+  c->scenes.assign(scenes, scenes + nscenes);
   c->searched = false;
   c->resident_ok = false;
   return NN_OK;
