@@ -12,6 +12,11 @@
 
 #define GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
+// Over grid cells, up to 2^31 - 1 of them: an int counter within a stride (up to 600,000) of
+// that wraps negative, passes the test and indexes below the array.
+#define FOR_CELLS(c, n) \
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < (uint32_t)(n); c += gridDim.x * blockDim.x)
+
 // Grid-stride loop whose trip count is uniform across a warp (for warp collectives):
 // `valid` is false on the lanes past the end.
 #define FOR_SLOTS_WARP(i, valid, n)                                                        \

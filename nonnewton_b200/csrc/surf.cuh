@@ -702,7 +702,7 @@ __device__ __forceinline__ void sr_block_add(double a, double b, double* dst, bo
 __global__ void k_sr_fix_to_field(SrDev s, int32_t cells) {
   if (blockIdx.x == 0 && threadIdx.x == 0) s.scan_n[2] = cells;
   double a = 0.0, b = 0.0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
+  FOR_CELLS(c, cells) {
     const float v = (float)((double)(long long)s.fix[c] / SR_FIX);
     s.splat[c] = v;
     s.field[c] = v;
@@ -832,9 +832,9 @@ __device__ void sr_normal_at(const SrDev& s, const double p[3], double n[3]) {
 
 // The crossing cubes in vertex-id order, so that the QEF kernel runs on dense work.
 __global__ void k_sr_dc_list(SrDev s, int32_t cells) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
+  FOR_CELLS(c, cells) {
     const uint32_t id = s.vflag[c];
-    if (s.vflag[c + 1] != id && (int64_t)id < s.max_v) s.cube_of[id] = (uint32_t)c;
+    if (s.vflag[c + 1] != id && (int64_t)id < s.max_v) s.cube_of[id] = c;
   }
 }
 

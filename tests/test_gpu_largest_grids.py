@@ -1,0 +1,36 @@
+"""Grids of almost 2^31 cells, the largest that are accepted: loops over cells and the scan of
+their counts end at the last cell, so a small set of particles has there what it has in a
+grid that just holds it."""
+import numpy as np
+import pytest
+import torch
+
+from nonnewton_b200.surface import SRTool
+
+from .surf_cases import ball
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(dims, pos, voxel=0.01, smooth=0.03):
+    reach = 11  # vertices that the tool adds to the box at this smoothing radius
+    sr = SRTool([[0.0] * 3, [(d - reach - 0.5) * voxel for d in dims]], voxel_size=voxel, particle_radius=0.02,
+                record_normals=True, max_num_vertices=100000, max_num_indices=600000, max_num_particles=len(pos))
+    assert sr.grid_dims(smooth) == list(dims)
+    sr.dual_contouring(0.0, smooth, len(pos), torch.from_numpy(pos).cuda())
+    out = [t.cpu().numpy() for t in (sr.mesh_vertex, sr.mesh_index, sr.mesh_normal)]
+    sr.close()
+    return out
+
+
+@pytest.mark.parametrize("dims", [(1263, 1291, 1317)])  # 32 bytes a vertex
+def test_surface_of_the_largest_grid(cuda_lib, dims):
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 90e9:
+        pytest.skip("needs 69 GB of device memory")
+    pos = ball(seed=5, radius=0.1)
+    want = _mesh((111, 110, 109), pos)
+    got = _mesh(dims, pos)
+    assert len(want[1]) > 0
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
