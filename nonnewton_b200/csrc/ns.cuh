@@ -57,7 +57,7 @@ __device__ __forceinline__ void step_reset_scenes(const Dev& d) {
 __global__ void k_zero_cells(Dev d, int reset_step) {
   if (reset_step && blockIdx.x == 0) step_reset_scenes(d);
   const int nc = d.d_n[2];
-  GRID_STRIDE(i, nc + 1) d.cell_count[i] = 0u;
+  FOR_CELLS(i, nc + 1) d.cell_count[i] = 0u;
 }
 
 // Keys and in-cell ranks of every source particle (truth id order or previous slots).
@@ -228,11 +228,14 @@ __device__ __forceinline__ void sort_cell(int* src, const int* ids, uint32_t n, 
     if ((uint32_t)q < n) src[q] = sv[q];
 }
 __global__ void k_cell_sort(Dev d) {
-  const int nc = d.d_n[2];
+  const uint32_t nc = (uint32_t)d.d_n[2];
   const bool truth = *d.src_from_truth != 0;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  FOR_SLOTS_WARP(c, valid, nc) {
+  // (unsigned like FOR_CELLS, with a trip count that is uniform across the warp)
+  for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < nc; base += gridDim.x * blockDim.x) {
+    const uint32_t c = base + lane;
+    const bool valid = c < nc;
     uint32_t b = 0, e = 0;
     if (valid) { b = d.cell_count[c]; e = d.cell_count[c + 1]; }
     const uint32_t n = e - b;

@@ -5,6 +5,9 @@ import numpy as np
 import pytest
 import torch
 
+from nonnewton_b200 import _abi
+from nonnewton_b200 import scene as S
+from nonnewton_b200.batch import Batch, scene_grid_cells
 from nonnewton_b200.surface import SRTool
 
 from .surf_cases import ball
@@ -34,3 +37,30 @@ def test_surface_of_the_largest_grid(cuda_lib, dims):
     assert len(want[1]) > 0
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+def _dam(extra=(0, 0, 0)):
+    """A dam break whose domain goes on past its box by `extra` cells of the search grid."""
+    sc = S.dam_break(seed=4, n_side=(9, 7, 8), box=0.4)
+    edge = np.array([0.5, 1, 1]) * sc.param.support_radius * (1 + 1e-3)  # x cells are half as long
+    sc.param.domain_end = np.asarray(sc.param.domain_end) + np.asarray(extra) * edge
+    return sc
+
+
+def _lists(scenes):
+    b = Batch(sum(sc.particles.n for sc in scenes), len(scenes))
+    b.set(scenes)
+    b.engine.run_pass(_abi.NN_PASS_SEARCH)
+    assert all(b.stats(k)["status"] == 0 for k in range(len(scenes)))
+    out = b.engine.neighbors(b.n, 64)
+    b.engine.close()
+    return out
+
+
+def test_lists_in_the_largest_search_grid(cuda_lib):
+    """32,767 cells of 256 x 256 rows, a channel of 656 m: lists as in the box alone."""
+    nx = scene_grid_cells(_dam(), x_split=2) // 1024  # 32 x 32 rows in the box's own grid
+    far = _dam((32767 - nx, 200, 200))
+    assert scene_grid_cells(far, x_split=2) == 32767 * 65536
+    for a, b in zip(_lists([far]), _lists([_dam()])):
+        assert torch.equal(a, b)
