@@ -95,7 +95,7 @@ __device__ __forceinline__ int scan_at(int t, int r) {  // this thread's 4 count
   return t * SCAN_TILE + (int)(threadIdx.x >> 5) * (SCAN_ROUNDS * 128) + r * 128 + (int)(threadIdx.x & 31) * 4;
 }
 __device__ __forceinline__ uint4 scan_load(const uint32_t* a, int i, int len) {
-  if (i + 4 <= len) return *reinterpret_cast<const uint4*>(a + i);
+  if (len - i >= 4) return *reinterpret_cast<const uint4*>(a + i);
   return make_uint4(i < len ? a[i] : 0u, i + 1 < len ? a[i + 1] : 0u, i + 2 < len ? a[i + 2] : 0u, 0u);
 }
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(Dev d) {
   __shared__ uint32_t sh[32];
   const int len = d.d_n[2] + 1;
-  const int ntiles = (len + SCAN_TILE - 1) / SCAN_TILE;
+  const int ntiles = (len - 1) / SCAN_TILE + 1;  // len up to 2^31 - 1: nothing is added to it
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     uint32_t s = 0;
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(Dev d) {
   static_assert(SCAN_THREADS == 1024, "32 warps, one lane each");
   __shared__ uint32_t sh[32], sh_part[32];
   const int len = d.d_n[2] + 1;
-  const int ntiles = (len + SCAN_TILE - 1) / SCAN_TILE;
+  const int ntiles = (len - 1) / SCAN_TILE + 1;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint32_t before = 0;  // sum of tile_sums[0 .. done)
   int done = 0;
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(Dev d) {
       o.y = o.x + v[r].x;
       o.z = o.y + v[r].y;
       o.w = o.z + v[r].z;
-      if (i + 4 <= len) {
+      if (len - i >= 4) {
         *reinterpret_cast<uint4*>(d.cell_count + i) = o;
       } else {
         if (i < len) d.cell_count[i] = o.x;

@@ -64,3 +64,7 @@ def test_lists_in_the_largest_search_grid(cuda_lib):
     assert scene_grid_cells(far, x_split=2) == 32767 * 65536
     for a, b in zip(_lists([far]), _lists([_dam()])):
         assert torch.equal(a, b)
+    # with a second scene the cells are 2^31 - 6,144: a scan tile (16,384) more would not fit an int
+    assert scene_grid_cells(_dam((25, 0, 0)), x_split=2) == 58 * 1024
+    for a, b in zip(_lists([far, _dam((25, 0, 0))]), _lists([_dam(), _dam()])):
+        assert torch.equal(a, b)
