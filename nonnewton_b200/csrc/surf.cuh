@@ -1188,11 +1188,14 @@ static int sr_scan(nn_sr_ctx* c, uint32_t* a, int64_t len, cudaStream_t st) {
 
 extern "C" {
 
+// Vertices of a grid stay this far below 2^31 - 1 (indices are int32; the scans need no margin).
+#define NN_SR_CELL_MARGIN 4096
+
 int nn_sr_create(int32_t max_particles, int64_t max_cells, int32_t max_vertices, int32_t max_indices,
                  int32_t options, nn_sr_ctx** out) {
   if (!out) return NN_ERR_INVALID_ARG;
   *out = nullptr;
-  if (max_particles <= 0 || max_cells <= 0 || max_cells >= (int64_t)INT32_MAX - SCAN_TILE || max_vertices <= 0 ||
+  if (max_particles <= 0 || max_cells <= 0 || max_cells >= (int64_t)INT32_MAX - NN_SR_CELL_MARGIN || max_vertices <= 0 ||
       max_indices <= 0 || (options & ~NN_SR_VELOCITY))
     return NN_ERR_INVALID_ARG;
   nn_sr_ctx* c = new nn_sr_ctx();

@@ -26,7 +26,7 @@ def _mesh(dims, pos, voxel=0.01, smooth=0.03):
     return out
 
 
-@pytest.mark.parametrize("dims", [(1263, 1291, 1317)])  # 32 bytes a vertex
+@pytest.mark.parametrize("dims", [(1263, 1291, 1317), (1263, 1293, 1315)])  # 32 bytes a vertex
 def test_surface_of_the_largest_grid(cuda_lib, dims):
     torch.cuda.empty_cache()
     if torch.cuda.mem_get_info()[0] < 90e9:
