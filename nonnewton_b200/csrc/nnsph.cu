@@ -50,6 +50,16 @@ cudaError_t dalloc(T** p, size_t count) {
 #define NN_DEFAULT_XSPLIT 2  // 2.4M scene: list build 0.66 -> 0.60 ms, step -0.7 % (x split 3 and 4: slower steps)
 
 #define NN_CG_LOOP_MAX 250000  // slots; see one_kernel_cg
+#define NN_BUILD_ROWS_MAX 110000  // slots; see enq_build_lists
+
+// How a composition's steps are launched, chosen in one place (plan_for) when the scenes are
+// set. A captured step holds these choices, so all of them are in its key (feature_sig).
+struct StepPlan {
+  int lanes = 1;          // lanes per particle of the neighbour passes (lanes_for)
+  bool rows = true;       // the list build takes one cell row per warp (enq_build_lists)
+  bool cg_loop = false;   // the viscosity loop is one kernel (one_kernel_cg)
+  int loop_slots = 0;     // slots that the grids of the one-kernel loops are laid out for, 0 without loops
+};
 
 struct nn_ctx {
   int cap = 0, max_scenes = 0, max_nb = 0;
@@ -64,7 +74,7 @@ struct nn_ctx {
   int unroll = NN_DEFAULT_UNROLL;      // neighbour chains in flight per thread (1, 2, 4; 0: per pass)
   int cell_factor = 1;                 // cells of edge h / cell_factor
   int x_split = NN_DEFAULT_XSPLIT;     // x cells per cell edge
-  int lanes = 1;                       // lanes per particle of the neighbour passes (lanes_for)
+  StepPlan plan;
   // state binding and scenes
   nn_state state{};
   bool bound = false;
@@ -122,15 +132,6 @@ struct nn_ctx {
   uint64_t graph_sig = 0;              // features the captured graphs were built for
 };
 
-// The kernels and loops a captured step contains depend only on these features.
-static uint64_t feature_sig(const nn_ctx* c) {
-  return (uint64_t)c->any_fluid | ((uint64_t)c->any_div << 1) | ((uint64_t)c->any_nonnewton << 2) |
-         ((uint64_t)c->any_implicit << 3) | ((uint64_t)std::min(c->el_mult_max, 255) << 8) |
-         ((uint64_t)(c->ne > 0) << 16) | ((uint64_t)c->block << 20) |
-         ((uint64_t)c->forces_feat << 40) | ((uint64_t)c->fold_np << 48) | ((uint64_t)c->lanes << 52) |
-         ((uint64_t)(c->n <= NN_CG_LOOP_MAX) << 56);
-}
-
 // Lanes per particle of the neighbour passes (nb_sum), by the fluid particles they walk. A
 // thread's pass over its 26-odd neighbours is one chain of dependent loads and arithmetic,
 // 10-20 us however few particles there are; splitting it over L lanes shortens it until the
@@ -142,6 +143,36 @@ static uint64_t feature_sig(const nn_ctx* c) {
 static int lanes_for(const nn_ctx* c, int n_fluid) {
   if (c->unroll) return 1;
   return n_fluid <= 10000 ? 8 : n_fluid <= 28000 ? 4 : n_fluid <= 56000 ? 2 : 1;
+}
+
+// The one-kernel loops' grids are laid out for the slots rounded up to a power of two (at most
+// the capacity): compositions of the same class share a captured step, and neither a small one
+// gets the blocks of the largest (each block more is an arrival at every barrier) nor a large one
+// those of the smallest that was captured first.
+static int log2_up(int n) {
+  int b = 0;
+  while (((int64_t)1 << b) < n) ++b;
+  return b;
+}
+static StepPlan plan_for(const nn_ctx* c) {
+  StepPlan p;
+  p.lanes = lanes_for(c, c->n_fluid);
+  p.rows = c->n <= NN_BUILD_ROWS_MAX;
+  p.cg_loop = c->unroll == 0 && (p.lanes > 1 || c->n <= NN_CG_LOOP_MAX);
+  if (p.lanes > 1 || (p.cg_loop && c->any_implicit))
+    p.loop_slots = (int)std::min<int64_t>((int64_t)1 << log2_up(c->n), c->cap);
+  return p;
+}
+
+// The kernels and loops a captured step contains, and their grids, depend only on these features
+// (and on buffers whose change drops the captured steps).
+static uint64_t feature_sig(const nn_ctx* c) {
+  return (uint64_t)c->any_fluid | ((uint64_t)c->any_div << 1) | ((uint64_t)c->any_nonnewton << 2) |
+         ((uint64_t)c->any_implicit << 3) | ((uint64_t)std::min(c->el_mult_max, 255) << 8) |
+         ((uint64_t)(c->ne > 0) << 16) | ((uint64_t)c->block << 20) |
+         ((uint64_t)c->forces_feat << 40) | ((uint64_t)c->fold_np << 48) | ((uint64_t)c->plan.lanes << 52) |
+         ((uint64_t)c->plan.cg_loop << 56) | ((uint64_t)c->plan.rows << 57) |
+         ((uint64_t)(c->plan.loop_slots ? 1 + log2_up(c->plan.loop_slots) : 0) << 58);
 }
 
 static thread_local char g_err[512];
@@ -238,10 +269,10 @@ template <typename... KArgs, typename... Args>
 static int launch(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, int work, Args... args) {
   return launch_lanes(c, s, k, block, work, 1, args...);
 }
-// A neighbour pass: c->lanes threads per particle.
+// A neighbour pass: c->plan.lanes threads per particle.
 template <typename... KArgs, typename... Args>
 static int launch_nb(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), int block, Args... args) {
-  return launch_lanes(c, s, k, block, c->n, c->lanes, args...);
+  return launch_lanes(c, s, k, block, c->n, c->plan.lanes, args...);
 }
 // A one-kernel loop: a cooperative launch, at most as many blocks as are resident at once
 // (capture records the launch attribute).
@@ -253,7 +284,7 @@ static int launch_loop(nn_ctx* c, cudaStream_t s, void (*k)(KArgs...), Args... a
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NN_SOLVE_BLOCK, 0));
     it = c->occ.emplace((const void*)k, std::max(per_sm, 1)).first;
   }
-  const int64_t want = ((int64_t)std::max(c->n, 1) * c->lanes + NN_SOLVE_BLOCK - 1) / NN_SOLVE_BLOCK;
+  const int64_t want = ((int64_t)std::max(c->plan.loop_slots, 1) * c->plan.lanes + NN_SOLVE_BLOCK - 1) / NN_SOLVE_BLOCK;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeCooperative;
   at.val.cooperative = 1;
@@ -291,9 +322,9 @@ enum : int {
 static inline int ku(const nn_ctx* c, int pass_default) { return c->unroll ? c->unroll : pass_default; }
 // The instantiation of a neighbour kernel for the context's (or the pass's) batch depth.
 #define KU_(k, def, ...)                                                                        \
-  (c->lanes == 8   ? &k<1, 8 __VA_ARGS__>                                                       \
-   : c->lanes == 4 ? &k<1, 4 __VA_ARGS__>                                                       \
-   : c->lanes == 2 ? &k<1, 2 __VA_ARGS__>                                                       \
+  (c->plan.lanes == 8   ? &k<1, 8 __VA_ARGS__>                                                       \
+   : c->plan.lanes == 4 ? &k<1, 4 __VA_ARGS__>                                                       \
+   : c->plan.lanes == 2 ? &k<1, 2 __VA_ARGS__>                                                       \
    : ku(c, def) == 4 ? &k<4, 1 __VA_ARGS__>                                                     \
    : ku(c, def) == 2 ? &k<2, 1 __VA_ARGS__>                                                     \
                      : &k<1, 1 __VA_ARGS__>)
@@ -311,9 +342,9 @@ static void (*forces_kernel(const nn_ctx* c))(Dev, int) {
   using All = std::make_integer_sequence<int, 16>;
   const int f = c->forces_feat & 15;
   const int u = ku(c, U_FORCES);
-  if (c->lanes == 8) return forces_pick<1, 8>(f, All{});
-  if (c->lanes == 4) return forces_pick<1, 4>(f, All{});
-  if (c->lanes == 2) return forces_pick<1, 2>(f, All{});
+  if (c->plan.lanes == 8) return forces_pick<1, 8>(f, All{});
+  if (c->plan.lanes == 4) return forces_pick<1, 4>(f, All{});
+  if (c->plan.lanes == 2) return forces_pick<1, 2>(f, All{});
   return u == 4 ? forces_pick<4, 1>(f, All{}) : u == 2 ? forces_pick<2, 1>(f, All{}) : forces_pick<1, 1>(f, All{});
 }
 
@@ -403,9 +434,8 @@ static int solver_loop(nn_ctx* c, cudaStream_t s, bool check_first, Pre pre, Bod
 // warp for all rows of its slots (rows / whole, us: 3,933 slots 9 / 36; 23,002 13 / 35;
 // 85,147 40 / 51; 135,201 46 / 44; 900,002 265 / 200; 2,400,002 694 / 470). Both write the
 // same lists.
-#define NN_BUILD_ROWS_MAX 110000
 static int enq_build_lists(nn_ctx* c, cudaStream_t s, const Dev& d) {
-  if (c->n <= NN_BUILD_ROWS_MAX) return launch_lanes(c, s, k_build_lists_rows, NSR_WARPS * 32, c->n, NSR_WARPS, d);
+  if (c->plan.rows) return launch_lanes(c, s, k_build_lists_rows, NSR_WARPS * 32, c->n, NSR_WARPS, d);
   return launch(c, s, k_build_lists, NS_WARPS * 32, c->n, d);
 }
 
@@ -456,11 +486,9 @@ static int enq_search(nn_ctx* c, cudaStream_t s, bool reset_step = false) {
 // 365 / 352 / 360 / 349; 85,147 at 1 lane 441 / 457 / 434 / 453 / 451; 135,201 360 / 363 /
 // 347 / 361 / 343; 175,870 759 / 799 / 751 / 775 / 783; 616,732 1181 / 1239 / 1184 / 1223 /
 // 1282. Host-driven loops (one synchronisation per body) keep separate kernels.
-static bool one_kernel_loops(const nn_ctx* c) { return c->in_capture && c->lanes > 1; }
-static bool one_kernel_cg(const nn_ctx* c) {
-  return c->in_capture && c->unroll == 0 && (c->lanes > 1 || c->n <= NN_CG_LOOP_MAX);
-}
-#define KL_(k, ...) (c->lanes == 8 ? &k<8 __VA_ARGS__> : c->lanes == 4 ? &k<4 __VA_ARGS__> : &k<2 __VA_ARGS__>)
+static bool one_kernel_loops(const nn_ctx* c) { return c->in_capture && c->plan.lanes > 1; }
+static bool one_kernel_cg(const nn_ctx* c) { return c->in_capture && c->plan.cg_loop; }
+#define KL_(k, ...) (c->plan.lanes == 8 ? &k<8 __VA_ARGS__> : c->plan.lanes == 4 ? &k<4 __VA_ARGS__> : &k<2 __VA_ARGS__>)
 #define KL(k) KL_(k)
 #define KL2(k, B) KL_(k, COMMA B)
 
@@ -526,7 +554,7 @@ static int enq_nonpressure(nn_ctx* c, cudaStream_t s, int advect, int clear) {
     RC(launch_nb(c, s, KU(k_cg_setup, U_CG_SETUP), B, d));
     if (one_kernel_cg(c)) {
       RC(launch1(c, s, k_cg_check0, d));
-      RC(launch_loop(c, s, c->lanes == 1 ? &k_cg_loop<1> : KL(k_cg_loop), d));
+      RC(launch_loop(c, s, c->plan.lanes == 1 ? &k_cg_loop<1> : KL(k_cg_loop), d));
     } else {
       RC(solver_loop(c, s, true, [&](cudaStream_t q) { return launch1(c, q, k_cg_check0, make_dev(c, c->cur)); },
                      [&](cudaStream_t q) {
@@ -896,7 +924,7 @@ int nn_set_tuning(nn_ctx* c, int32_t block, int32_t unroll, int32_t cell_factor)
   if (cell_factor != c->cell_factor) c->scenes.clear();  // cell layout changes: set the scenes again
   c->block = block;
   c->unroll = unroll;
-  c->lanes = lanes_for(c, c->n_fluid);
+  c->plan = plan_for(c);
   c->cell_factor = cell_factor;
   c->occ.clear();
   return NN_OK;
@@ -1043,14 +1071,14 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
   c->ne = (int)el_id.size();
   c->n_fluid = 0;
   for (int k = 0; k < nscenes; ++k) c->n_fluid += scenes[k].n_fluid;
-  c->lanes = lanes_for(c, c->n_fluid);
+  c->n = n;
+  c->plan = plan_for(c);
   // elastic and rigid-body buffers are freed and reallocated below: their pointers, strides and
   // counts are graph arguments, those of the old set as well (a set without bodies after one with
   // bodies has the same features)
   if (feature_sig(c) != c->graph_sig || c->ne > 0 || c->n_rb > 0 || !rb_list.empty()) drop_graphs(c);
   c->scenes.clear();  // no step until every buffer is there again
   c->sdev = sdev;
-  c->n = n;
   c->ncells = (int)cells;
   c->ne = (int)el_id.size();
   free_elastic(c);

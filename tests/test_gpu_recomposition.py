@@ -1,10 +1,13 @@
 """A batch whose composition changes between steps: the step that follows launches what a
 fresh batch of the same composition launches, and gives its bits."""
+import json
+
 import pytest
 import torch
+from torch.profiler import ProfilerActivity, profile
 
 from nonnewton_b200 import scene as S
-from nonnewton_b200.batch import Batch
+from nonnewton_b200.batch import Batch, scene_grid_cells
 
 pytestmark = pytest.mark.gpu
 FIELDS = ("x", "v", "acceleration", "density", "volume")
@@ -65,3 +68,42 @@ def test_rigid_scene_is_repacked_away(cuda_lib):
     _steps(fresh)
     fresh.repack([0], [])
     _same(_steps(b), _steps(fresh))
+
+
+def _kernels(b, path):
+    """Names and grids of the kernels of a step, in time order (none without a profiler)."""
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        b.step(1)
+        torch.cuda.synchronize()
+    p.export_chrome_trace(str(path))
+    ev = [e for e in json.loads(path.read_text())["traceEvents"] if e.get("cat") == "kernel"]
+    return [(e["name"], e["args"]["grid"]) for e in sorted(ev, key=lambda e: e["ts"])]
+
+
+# fluid on both sides of every line of the choices: lanes (10,000, 28,000, 56,000 fluid), the list
+# build (110,000 slots), the viscosity's one-kernel loop (250,000), its grid (powers of two)
+@pytest.mark.parametrize("implicit", [False, True])
+def test_choices_follow_the_composition(cuda_lib, tmp_path, implicit):
+    """Up and down through the sizes: the launch choices of a captured step (lanes, list build,
+    loops in one kernel or as while-nodes, their grids) are those of the present composition,
+    not of the one before it or of the one that was captured first."""
+    kind = dict(extra_cfg={"useNonNewtonianModel": True},
+                fluid_cfg={"nonNewtonMethod": "CROSS_", "viscosity0": 5.0, "viscosity_inf": 0.01,
+                           "consistency_index": 1.0, "power_index": 0.7, "viscosityMethod": 13,
+                           "viscoMaxError": 1e-5}) if implicit else {}
+    scenes = [S.dam_break(seed=k, n_side=(side,) * 3, box=(side + 4) * 0.02, **kind)
+              for k, side in enumerate((9, 24, 33, 45, 50, 62))]
+    sizes = [sc.particles.n for sc in scenes]
+    assert sizes[0] < 2000 and sizes[3] < 110000 < sizes[4] < 250000 < sizes[5]
+    cells = max(scene_grid_cells(sc, x_split=2) for sc in scenes)
+    b = Batch(sizes[-1], 1, max_cells=cells)
+    want = []
+    for sc in scenes:
+        fresh = Batch(sizes[-1], 1, max_cells=cells)
+        fresh.set([sc])
+        want.append((_steps(fresh), _kernels(fresh, tmp_path / "trace.json")))
+        fresh.engine.close()
+    for k in (0, 1, 2, 3, 4, 5, 4, 5, 3, 2, 0, 4, 1):
+        b.set([scenes[k]])
+        _same(_steps(b), want[k][0])
+        assert _kernels(b, tmp_path / "trace.json") == want[k][1]
