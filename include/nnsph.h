@@ -268,6 +268,13 @@ int nn_set_neighbor_cap(nn_ctx* ctx, int32_t max_neighbors);
 int nn_status_async(nn_ctx* ctx, int32_t scene, int32_t* host_out);
 int nn_status_wait(nn_ctx* ctx);
 
+/* How long a block of a solver loop that runs as one kernel waits for the others, in polls of
+   about half a microsecond; negative: the default (seconds). The blocks are resident together,
+   so the wait does not run out by itself; where it does, the loop ends, the step goes on with
+   an unfinished solve and every scene of the batch gets the status NN_ERR_CUDA, which stays
+   until the scenes are set again. 0 makes every wait run out. */
+int nn_set_wait_limit(nn_ctx* ctx, int32_t polls);
+
 /* Statistics of scene `scene` (copies from the device; synchronises the stream). */
 int nn_get_stats(nn_ctx* ctx, int32_t scene, nn_stats* out);
 

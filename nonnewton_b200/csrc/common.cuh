@@ -445,11 +445,12 @@ __device__ __forceinline__ double acc_take(double* acc, int scene, int quantity)
 // Barrier over the blocks of a cooperative launch (all resident). The last block to arrive
 // runs `last` before it lets the others go, so that the control of a solver loop costs no
 // barrier of its own. A wait that runs out (which a resident grid cannot cause) marks the
-// barrier failed; every block then leaves the kernel, and the step reports it.
+// barrier failed: every block then leaves the kernel, every scene of the step reports it, and
+// the next step starts with the barrier at rest (k_zero_cells).
 // The counter and the generation lie in lines of their own: the polls of a thousand waiting
 // blocks would queue up before the arrivals.
 struct GridBarrier { unsigned arrived, pad0[31], gen, pad1[31]; int fail, pad2[31]; };
-#define NN_BARRIER_POLLS (1u << 24)  // seconds
+#define NN_BARRIER_POLLS (1u << 24)  // seconds (nn_set_wait_limit)
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -464,10 +465,11 @@ __device__ __forceinline__ unsigned add_acq_rel(unsigned* p, unsigned v) {
   return old;
 }
 // `gen`: the barrier's generation, read once by grid_gen before the block's first barrier
-// and counted on by each barrier (only thread 0's copy is used).
+// and counted on by each barrier (only thread 0's copy is used). `limit`: polls of a wait; at 0
+// a block that is not the last to arrive gives up at once.
 __device__ __forceinline__ unsigned grid_gen(GridBarrier* b) { return threadIdx.x == 0 ? ld_acquire(&b->gen) : 0u; }
 template <typename F>
-__device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned& gen, F last) {
+__device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned limit, unsigned& gen, F last) {
   __shared__ int sh_last, sh_fail;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -484,8 +486,8 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned& gen, F la
     }
   } else if (threadIdx.x == 0) {
     unsigned polls = 0;
-    while (ld_acquire(&b->gen) == gen) {
-      if (++polls > NN_BARRIER_POLLS || ((polls & 1023u) == 0u && *(volatile int*)&b->fail)) {
+    while (limit == 0u || ld_acquire(&b->gen) == gen) {
+      if (++polls > limit || ((polls & 1023u) == 0u && *(volatile int*)&b->fail)) {
         atomicExch(&b->fail, 1);
         sh_fail = 1;
         break;

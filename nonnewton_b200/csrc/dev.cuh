@@ -84,6 +84,7 @@ struct Dev {
   unsigned long long loop_handle; // cudaGraphConditionalHandle (0 when not in a graph)
   int32_t* body_count;         // [4] executed loop bodies (div, pressure, cg, elastic)
   GridBarrier* bar;            // barrier of the one-kernel loops
+  uint32_t bar_polls;          // polls of a wait at it
 };
 
 // The pair of float4 of a slot, position and velocity (or the matvec's), in one 256-bit

@@ -120,6 +120,7 @@ struct nn_ctx {
   cudaEvent_t status_ev = nullptr;     // recorded after nn_status_async's copy
   int32_t* d_body = nullptr;
   GridBarrier* d_bar = nullptr;
+  uint32_t bar_polls = NN_BARRIER_POLLS;
   int64_t fixed_nodes_per_step = 0;    // kernel nodes outside loop bodies (graph mode)
   int64_t graph_replays = 0;
   int64_t body_nodes[3] = {3, 3, 5};   // kernels per loop body: divergence, pressure, CG
@@ -235,6 +236,7 @@ static Dev make_dev(nn_ctx* c, int cur) {
   d.loop_handle = c->cur_handle;
   d.body_count = c->d_body;
   d.bar = c->d_bar;
+  d.bar_polls = c->bar_polls;
   return d;
 }
 
@@ -942,6 +944,14 @@ int nn_set_x_split(nn_ctx* c, int32_t x_split) {
   return NN_OK;
 }
 
+int nn_set_wait_limit(nn_ctx* c, int32_t polls) {
+  if (!c) return fail(nullptr, NN_ERR_INVALID_ARG, "null context");
+  const uint32_t limit = polls < 0 ? NN_BARRIER_POLLS : (uint32_t)polls;
+  if (limit != c->bar_polls) drop_graphs(c);  // a kernel argument
+  c->bar_polls = limit;
+  return NN_OK;
+}
+
 int64_t nn_launch_count(const nn_ctx* cc) {
   nn_ctx* c = const_cast<nn_ctx*>(cc);
   if (!c) return -1;
@@ -1110,7 +1120,6 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
   int32_t hn[4] = {n, nscenes, (int)cells, c->ne};
   CK(cudaMemcpy(c->d_n, hn, sizeof(hn), cudaMemcpyHostToDevice));
   CK(cudaMemset(c->d_acc, 0, (size_t)c->max_scenes * ACC_COUNT * NN_STRIPES * sizeof(double)));
-  CK(cudaMemset(c->d_bar, 0, sizeof(GridBarrier)));
   // rigid bodies ("r-space")
   cudaFree(c->rb_of_id); cudaFree(c->rb_round); cudaFree(c->rb_acc); cudaFree(c->rb_rest); cudaFree(c->rb_cm);
   cudaFree(c->rb_R);

@@ -53,9 +53,20 @@ __device__ __forceinline__ void step_reset_scenes(const Dev& d) {
 }
 
 // `reset_step`: block 0 also resets the step's per-scene counters (the step's first
-// launch; nothing before the list build reads them).
+// launch; nothing before the list build reads them) and, after a wait at the loops' barrier
+// that ran out, the arrivals and the sums that it left behind.
 __global__ void k_zero_cells(Dev d, int reset_step) {
-  if (reset_step && blockIdx.x == 0) step_reset_scenes(d);
+  if (reset_step && blockIdx.x == 0) {
+    step_reset_scenes(d);
+    if (*(volatile int*)&d.bar->fail) {
+      for (int t = threadIdx.x; t < d.d_n[1] * ACC_COUNT * NN_STRIPES; t += blockDim.x) d.acc[t] = 0.0;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        d.bar->arrived = d.bar->gen = 0u;
+        d.bar->fail = 0;
+      }
+    }
+  }
   const int nc = d.d_n[2];
   FOR_CELLS(i, nc + 1) d.cell_count[i] = 0u;
 }

@@ -1158,11 +1158,12 @@ __global__ void k_cg_finish(Dev d, int advect) {
 // are the same bodies; blocks meet at grid barriers (2.6 us), whose last arrival runs the
 // check. What a pass gathers of arrays that this kernel writes goes through coherent loads.
 #define NN_SOLVE_BLOCK 128
-__device__ __forceinline__ bool solve_failed(const Dev& d) {
-  if (threadIdx.x == 0) set_status(&d.dyn[0], NN_ERR_CUDA);
+__device__ __forceinline__ bool solve_failed(const Dev& d) {  // the loop ends for all scenes
+  for (int sc = threadIdx.x; sc < d.d_n[1]; sc += blockDim.x) set_status(&d.dyn[sc], NN_ERR_CUDA);
   return true;
 }
-#define SOLVE_BARRIER(d, last) do { if (!grid_barrier((d).bar, gen, last) && solve_failed(d)) return; } while (0)
+#define SOLVE_BARRIER(d, last) \
+  do { if (!grid_barrier((d).bar, (d).bar_polls, gen, last) && solve_failed(d)) return; } while (0)
 #define SOLVE_GOES_ON(d) (*(volatile int32_t*)(d).any_active != 0)
 
 template <int L, bool FOLD>

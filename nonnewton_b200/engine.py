@@ -212,6 +212,13 @@ class Engine:
         f.restype = C.c_int
         self._rc(f(self.h))
 
+    def set_wait_limit(self, polls: int | None = None):
+        """Polls of a wait inside a one-kernel solver loop (see nn_set_wait_limit); None: the default."""
+        f = self.L.nn_set_wait_limit
+        f.argtypes = [C.c_void_p, C.c_int32]
+        f.restype = C.c_int
+        self._rc(f(self.h, -1 if polls is None else int(polls)))
+
     def stats(self, scene: int = 0) -> dict:
         s = _abi.nn_stats()
         self._rc(self.L.nn_get_stats(self.h, int(scene), C.byref(s)))

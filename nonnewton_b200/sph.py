@@ -16,7 +16,7 @@ import torch
 
 from . import _abi
 from .config import Parameter, SimConfig
-from .engine import Engine
+from .engine import Engine, NNError
 from .scene import ParticleSet, export_ply_particles, geometry_path, load_particles, read_animation
 
 FLUID, SOLID = _abi.NN_FLUID, _abi.NN_SOLID
@@ -213,6 +213,7 @@ class SPHBase:
         while True:
             st = eng.stats(0)
             self._last_max = st["max_neighbors_seen"]
+            self._raise_unfinished(st["status"])
             if st["status"] != _abi.NN_ERR_NEIGHBOR_OVERFLOW or eng.max_neighbors >= 1024:
                 return
             self._rerun(nsteps, displacement, st["max_neighbors_seen"])
@@ -229,8 +230,15 @@ class SPHBase:
             eng.set_animation(0, displacement)
         eng.step(nsteps, sync=True, host_loop=self.host_loop)
 
-    def _settle(self):
-        """Check the previous call's status copy (see _advance)."""
+    @staticmethod
+    def _raise_unfinished(status):
+        """A wait inside a solver loop ran out: the state that the step left is no result."""
+        if status == _abi.NN_ERR_CUDA:
+            raise NNError(status, "a solver loop of the step ended before its solve")
+
+    def _settle(self, report=True):
+        """Check the previous call's status copy (see _advance); `report`: raise if its
+        solver loops did not finish."""
         if self._pending is None:
             return
         nsteps, displacement = self._pending
@@ -241,6 +249,8 @@ class SPHBase:
         if status == _abi.NN_ERR_NEIGHBOR_OVERFLOW:
             self._rerun(nsteps, displacement, seen)
             self._check(nsteps, displacement)
+        elif report:
+            self._raise_unfinished(status)
 
     def _grow_cap(self, st):
         cap = max(st["max_neighbors_seen"], self.engine.max_neighbors) * 5 // 4
@@ -283,7 +293,7 @@ class SPHBase:
         self._pass(_abi.NN_PASS_ADVECT)
 
     def stats(self) -> dict:
-        self._settle()
+        self._settle(report=False)  # the statistics carry the status
         return self.engine.stats(0)
 
 
