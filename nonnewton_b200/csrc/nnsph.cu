@@ -497,11 +497,12 @@ static bool one_kernel_cg(const nn_ctx* c) { return c->in_capture && c->plan.cg_
 // DFSPHSolver.divergence_solve (SPH/main.py:1683-1713). In the fused step the first
 // density change and alpha *= 1/dt were done by k_density_factor<CHANGE> and the
 // closing alpha *= dt is folded into the pressure solve's first pass (fused = true);
-// with c->fold_np the loop's density change also computes the fluid's non-pressure terms.
-static int enq_divergence(nn_ctx* c, cudaStream_t s, bool fused) {
+// with c->fold_np the loop's density change also computes the fluid's non-pressure terms, in a
+// step (`fold`), whose gather writes the solids'.
+static int enq_divergence(nn_ctx* c, cudaStream_t s, bool fused, bool fold) {
   Dev d = make_dev(c, c->cur);
   const int B = c->block;
-  const bool np = fused && c->fold_np;
+  const bool np = fold && c->fold_np;
   if (fused && one_kernel_loops(c)) {
     if (np) return launch_loop(c, s, KL2(k_divergence_loop, true), d);
     return launch_loop(c, s, KL2(k_divergence_loop, false), d);
@@ -606,14 +607,15 @@ static int enq_rigid(nn_ctx* c, cudaStream_t s) {
 }
 
 // DFSPHSolver.substep (SPH/main.py:1546-1555) with the fused passes.
-// `begun`: the loops' start is done (k_boundary_volume at the start of the step).
+// `begun`: in a step, where the loops' start is done (k_boundary_volume) and the solids'
+// non-pressure terms are (k_gather); as a pass of its own the force pass writes all of them.
 static int enq_substep(nn_ctx* c, cudaStream_t s, bool begun = false) {
   if (!c->any_fluid) return NN_OK;
   Dev d = make_dev(c, c->cur);
   if (c->any_div) {
     if (!begun) RC(launch1(c, s, k_solver_begin, d, 0));
     RC(launch_nb(c, s, KU2(k_density_factor, true, U_DENSITY_FACTOR), c->block, d, 1, 1));
-    RC(enq_divergence(c, s, true));
+    RC(enq_divergence(c, s, true, begun));
   } else {
     RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 1, 1));
   }
@@ -1252,7 +1254,7 @@ int nn_run_pass(nn_ctx* c, int32_t pass) {
     case NN_PASS_CLEAR_ACCELERATIONS: RC(launch(c, s, k_clear_acc, 256, c->n, d)); break;
     case NN_PASS_DENSITIES: RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 1, 0)); break;
     case NN_PASS_DFSPH_FACTOR: RC(launch_nb(c, s, KU2(k_density_factor, false, U_DENSITY_FACTOR), c->block, d, 0, 1)); break;
-    case NN_PASS_DIVERGENCE_SOLVE: if (c->any_div) RC(enq_divergence(c, s, false)); break;
+    case NN_PASS_DIVERGENCE_SOLVE: if (c->any_div) RC(enq_divergence(c, s, false, false)); break;
     case NN_PASS_NON_PRESSURE_FORCES: if (c->any_fluid) RC(enq_nonpressure(c, s, 0, 0)); break;
     case NN_PASS_NON_PRESSURE_ADVECT: RC(launch(c, s, k_np_advect, 256, c->n, d)); break;
     case NN_PASS_PRESSURE_SOLVE: if (c->any_fluid) RC(enq_pressure(c, s, 0)); break;

@@ -678,15 +678,16 @@ template <int U, int L, int FF>
 __device__ __forceinline__ void forces_body(const Dev& d, int clear) {
   static_assert(!(FF & FF_Q) || L == 1, "quirk mode keeps one lane per particle");
   const int n = d.d_n[0];
-  if (L == 1 && no_scene(d, [](const SceneDev& s, const SceneDyn& y) { return s.n_fluid != 0 && !y.np_fresh; })) return;
+  if (L == 1 && no_scene(d, [&](const SceneDev& s, const SceneDyn& y) { return s.n_fluid != 0 && !(clear && y.np_fresh); })) return;
   FOR_SPLIT(L, i, sub, valid, n) {
     const uint32_t fl = valid ? d.w.flags[i] : 0u;
     const bool fluid = cls_fluid(fl);
     const int scn = slot_scene(fl);
     const SceneDev& s = d.sc[scn];
     // the reference runs the substep only with fluid; np_fresh: computed by the divergence
-    // loop's last density change
-    const bool work = valid && s.n_fluid != 0 && !d.dyn[scn].np_fresh;
+    // loop's last density change (of this substep; a force pass of its own, without `clear`,
+    // takes nothing over from a step before it)
+    const bool work = valid && s.n_fluid != 0 && !(clear && d.dyn[scn].np_fresh);
     if (L == 1 ? !work : !__any_sync(0xffffffffu, work)) continue;
     const bool implicit = scene_implicit(s);
     const bool quirks = (FF & FF_Q) && (s.flags & NN_F_QUIRKS);
