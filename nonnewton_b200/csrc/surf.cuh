@@ -951,6 +951,20 @@ __device__ __forceinline__ int64_t sr_vid(const SrDev& s, int x, int y, int z) {
   return s.vflag[c + 1] != s.vflag[c] ? (int64_t)s.vflag[c] : -1;
 }
 
+// The cubes around edge w (2, 3 or 11) of cube (x, y, z), as vertex ids; false where
+// the edge has no crossing or a cube no vertex.
+__device__ __forceinline__ bool sr_quad(const SrDev& s, int x, int y, int z, int ci, int w, int64_t id[4]) {
+  if (!sr_edge_cross(ci, w)) return false;
+  int d[4][3];
+  sr_edge_cubes(w, d);
+  bool ok = true;
+  for (int q = 0; q < 4; ++q) {
+    id[q] = sr_vid(s, x + d[q][0], y + d[q][1], z + d[q][2]);
+    ok = ok && id[q] >= 0;
+  }
+  return ok;
+}
+
 // pass 0 counts the indices each crossing cube emits (into tcount, by vertex id, which
 // follows the cube order), pass 1 writes them at the scanned offsets
 __global__ void k_sr_tris(SrDev s, int64_t cells, int pass) {
@@ -964,16 +978,8 @@ __global__ void k_sr_tris(SrDev s, int64_t cells, int pass) {
     int64_t o = pass ? (int64_t)s.tcount[v] : 0;
     for (int k = 0; k < 3; ++k) {
       const int w = k == 0 ? 2 : k == 1 ? 3 : 11;
-      if (!sr_edge_cross(ci, w)) continue;
-      int d[4][3];
-      sr_edge_cubes(w, d);
       int64_t id[4];
-      bool ok = true;
-      for (int q = 0; q < 4; ++q) {
-        id[q] = sr_vid(s, x + d[q][0], y + d[q][1], z + d[q][2]);
-        ok = ok && id[q] >= 0;
-      }
-      if (!ok) continue;
+      if (!sr_quad(s, x, y, z, ci, w, id)) continue;
       cnt += 6;
       if (pass) {
         if (o + 6 > s.max_i) { sr_fail(s, NN_ERR_CAPACITY); continue; }
@@ -987,6 +993,21 @@ __global__ void k_sr_tris(SrDev s, int64_t cells, int pass) {
     }
     if (!pass) s.tcount[v] = cnt;
   }
+}
+
+// All the indices of a mesh whose vertices overflow, for the error message: k_sr_tris has walked
+// the cubes of the first max_v vertices only. result->ni is zero.
+__global__ void k_sr_tris_total(SrDev s, int32_t cells) {
+  uint32_t cnt = 0;
+  FOR_CELLS(c, cells) {
+    if (s.vflag[c + 1] == s.vflag[c]) continue;
+    const int x = (int)c % s.g.nx, y = ((int)c / s.g.nx) % s.g.ny, z = (int)c / (s.g.nx * s.g.ny);
+    const int ci = sr_cube_mask(s, x, y, z);
+    int64_t id[4];
+    for (int k = 0; k < 3; ++k) cnt += sr_quad(s, x, y, z, ci, k == 0 ? 2 : k == 1 ? 3 : 11, id) ? 6u : 0u;
+  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&s.result->ni, cnt);
 }
 
 // What the host reads back, in one copy.
@@ -1375,6 +1396,13 @@ static int sr_run(nn_sr_ctx* c, const nn_sr_params* p, const float* pos, const f
   SRCK(cudaGetLastError());
   SRCK(cudaMemcpyAsync(c->h_result, c->result, sizeof(SrResult), cudaMemcpyDeviceToHost, st));
   SRCK(cudaStreamSynchronize(st));
+  if (!marching_cubes && c->h_result->nv > (uint32_t)c->max_v) {
+    SRCK(cudaMemsetAsync(&c->result->ni, 0, sizeof(uint32_t), st));
+    k_sr_tris_total<<<grid_c, B, 0, st>>>(s, (int32_t)cells);
+    SRCK(cudaGetLastError());
+    SRCK(cudaMemcpyAsync(c->h_result, c->result, sizeof(SrResult), cudaMemcpyDeviceToHost, st));
+    SRCK(cudaStreamSynchronize(st));
+  }
   int32_t status = c->h_result->status;
   c->nv = (int32_t)c->h_result->nv;
   c->ni = (int32_t)c->h_result->ni;
