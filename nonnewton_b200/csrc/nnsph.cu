@@ -737,6 +737,8 @@ static SceneDev make_scene(const nn_scene_desc& sd, int64_t cell_base, int el_mu
   s.k_w = (real)k;
   s.k2_w = (real)(k * 2.0);
   s.k_grad = (real)(6.0 * (8.0 / kPi) / (h * h * h));
+  s.k_grad_h = (real)(6.0 * k / h);
+  s.k_grad_h2 = (real)(6.0 * k / (h * h));
   s.W0 = host_kernel_w(0.f, s.h, s.k_w, s.k2_w);
   s.rho0 = (real)p.density0;
   s.inv_rho0 = (real)(1.0 / p.density0);

@@ -1217,7 +1217,12 @@ __global__ void NN_REGS64 k_pressure_loop(const __grid_constant__ Dev d) {
 // gradient, R_j S_j (gw V_i) (-V_j) - R_i S_i (-gw V_j) (-V_i) =
 // -V_i V_j (R_i S_i + R_j S_j) gw. On the fluid-elastic scene (64,000 elastic particles)
 // rotations 38 + stress 37 + forces 62 us became gather 3 +
-// deformation 16 + rotations 12 + stress 13 + forces 20 us.
+// deformation 16 + rotations 12 + stress 15 + forces 22 us.
+// The kernel and its gradient are those with a correctly rounded root and divisions (kernel_w,
+// kernel_grad): from rsqrt (kw_r2, kgrad_r2) the stress took 12.5 and the forces 20.2 us, but in a
+// strained block, whose terms do not cancel, the accelerations were 1.7 times as far from 64
+// bits (deformed by 10 %: 7.2e-7 against 3.7e-7 of their root mean square, the stress 3.9e-7
+// against 2.8e-7).
 #define EL_LANES 4
 #define EL_U 2
 #define EL_BLOCK 128
@@ -1271,7 +1276,7 @@ __global__ void __launch_bounds__(EL_BLOCK) k_el_deformation(Dev d, int rep) {
     el_walk(d, e, sub, work ? d.el_cnt[e] : 0, [&](int j) { return ElPair{ldg(&d.el_x[j]), ldg(&d.el_x0[j])}; },
             [&](const ElPair& g) {
               const real3 a = f3(g.x) - xi, b = f3(g.x0) - x0i;
-              const real w = xi4.w * kw_r2(dot3(b, b), s);
+              const real w = xi4.w * kernel_w(sqrt(dot3(b, b)), s);
               A[0] += a.x * b.x * w; A[1] += a.x * b.y * w; A[2] += a.x * b.z * w;
               A[3] += a.y * b.x * w; A[4] += a.y * b.y * w; A[5] += a.y * b.z * w;
               A[6] += a.z * b.x * w; A[7] += a.z * b.y * w; A[8] += a.z * b.z * w;
@@ -1316,7 +1321,7 @@ __global__ void __launch_bounds__(EL_BLOCK) k_el_stress(Dev d, int rep) {
                                      R[1] * xji.x + R[4] * xji.y + R[7] * xji.z - xji0.y,
                                      R[2] * xji.x + R[5] * xji.y + R[8] * xji.z - xji0.z);
               u = u * g.x0.w;
-              const real3 gw = kgrad_r2(xji0, dot3(xji0, xji0), s);
+              const real3 gw = kernel_grad(xji0, sqrt(dot3(xji0, xji0)), s);
               G[0] -= u.x * gw.x; G[1] -= u.x * gw.y; G[2] -= u.x * gw.z;
               G[3] -= u.y * gw.x; G[4] -= u.y * gw.y; G[5] -= u.y * gw.z;
               G[6] -= u.z * gw.x; G[7] -= u.z * gw.y; G[8] -= u.z * gw.z;
@@ -1365,7 +1370,7 @@ __global__ void __launch_bounds__(EL_BLOCK) k_el_forces(Dev d, int rep) {
             },
             [&](const ElForce& g) {
               const real3 xji0 = f3(g.x0) - f3(x0i);
-              const real3 gw = kgrad_r2(xji0, dot3(xji0, xji0), s) * g.x0.w;
+              const real3 gw = kernel_grad(xji0, sqrt(dot3(xji0, xji0)), s) * g.x0.w;
 #pragma unroll
               for (int q = 0; q < 3; ++q)
                 f[q] -= (Mi[3 * q] + g.M[3 * q]) * gw.x + (Mi[3 * q + 1] + g.M[3 * q + 1]) * gw.y +
