@@ -182,13 +182,16 @@ class Engine:
         self._rc(self.L.nn_run_pass(self.h, int(p)))
 
     def neighbors(self, n: int, width: int = 60):
-        whole = self._state is not None and n == self._state.n  # every row is then written
-        num = (torch.empty if whole else torch.zeros)(n, dtype=torch.int32, device=self.device)
-        lists = torch.empty((n, width), dtype=torch.int32, device=self.device)
-        if not whole:
-            lists.fill_(-1)
+        """Counts and id-sorted lists of the first `n` particles (rows past the bound state: none)."""
+        bound = self._state.n if self._state is not None else 0
+        rows = max(int(n), bound)  # the export writes every bound particle's
+        num = torch.empty(rows, dtype=torch.int32, device=self.device)
+        lists = torch.empty((rows, width), dtype=torch.int32, device=self.device)
+        if rows > bound:
+            num[bound:] = 0
+            lists[bound:] = -1
         self._rc(self.L.nn_get_neighbors(self.h, _ptr(num), _ptr(lists), int(width)))
-        return num, lists
+        return num[:n], lists[:n]
 
     def set_neighbor_cap(self, max_neighbors: int):
         """Re-size the neighbour lists (see nn_set_neighbor_cap); clears overflow statuses."""
