@@ -116,6 +116,10 @@ __constant__ int8_t c_sr_edge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {3, 0}, {4, 5}, 
         for (bool act = (s).active[(s).g.bidx(x, y, z)]; _once; _once = 0)
 static_assert(NN_SR_BLOCK == 32, "a warp covers a block's row");
 
+// Where particle (or vertex) i starts in an array of 3 words each; in int, the 9 words of G would
+// end at 238 million particles.
+__device__ __forceinline__ size_t at3(int i) { return 3 * (size_t)i; }
+
 __device__ __forceinline__ void sr_fail(const SrDev& s, int code) { atomicCAS(s.status, 0, code); }
 
 __device__ __forceinline__ void sr_add(const SrDev& s, int64_t c, double val) {
@@ -129,7 +133,7 @@ __global__ void k_sr_keys(SrDev s, int32_t cells) {
   if (blockIdx.x == 0 && threadIdx.x == 0) s.scan_n[2] = cells;
   GRID_STRIDE(i, s.n) {
     int x, y, z;
-    s.g.voxel_of(s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2], x, y, z);
+    s.g.voxel_of(s.pos[at3(i)], s.pos[at3(i) + 1], s.pos[at3(i) + 2], x, y, z);
     if (!s.g.in(x, y, z)) { sr_fail(s, NN_ERR_INVALID_ARG); s.vkey[i] = 0xffffffffu; continue; }
     const uint32_t k = (uint32_t)s.g.idx(x, y, z);
     s.vkey[i] = k;
@@ -163,14 +167,14 @@ __global__ void k_sr_sorted_pos(SrDev s, int64_t cells) {
   GRID_STRIDE(k, nb) {
     const int i = s.vsrc[k];
     if (i < 0 || i >= s.n) continue;
-    s.spos[k] = make_float4(s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2], 0.f);
+    s.spos[k] = make_float4(s.pos[at3(i)], s.pos[at3(i) + 1], s.pos[at3(i) + 2], 0.f);
   }
 }
 
 // ---- 2. isotropic splat (generate_fluid_field) --------------------------------------
 __global__ void k_sr_iso(SrDev s) {
   GRID_STRIDE(i, s.n) {
-    const float px = s.pos[3 * i], py = s.pos[3 * i + 1], pz = s.pos[3 * i + 2];
+    const float px = s.pos[at3(i)], py = s.pos[at3(i) + 1], pz = s.pos[at3(i) + 2];
     int cx, cy, cz;
     s.g.voxel_of(px, py, pz, cx, cy, cz);
     if (!s.g.in(cx, cy, cz)) continue;
@@ -302,7 +306,7 @@ __device__ __forceinline__ void sr_range_particles(const SrDev& s, int cx, int c
 struct SrMoments { double tw, m1[3], m2[6]; int nnb; };
 
 __device__ __forceinline__ void sr_aniso_kernel_of(const SrDev& s, int i, const SrMoments& a) {
-  const float px = s.pos[3 * i], py = s.pos[3 * i + 1], pz = s.pos[3 * i + 2];
+  const float px = s.pos[at3(i)], py = s.pos[at3(i) + 1], pz = s.pos[at3(i) + 2];
   const double tw = a.tw;
   const double *m1 = a.m1, *m2 = a.m2;
   double db[3] = {0.0, 0.0, 0.0}, C[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
@@ -315,9 +319,9 @@ __device__ __forceinline__ void sr_aniso_kernel_of(const SrDev& s, int i, const 
   }
   const double xw[3] = {tw != 0.0 ? px + db[0] : 0.0, tw != 0.0 ? py + db[1] : 0.0, tw != 0.0 ? pz + db[2] : 0.0};
   const double lam_ = 0.9;  // akLambda
-  s.xbar[3 * i] = (float)((1 - lam_) * px + lam_ * xw[0]);
-  s.xbar[3 * i + 1] = (float)((1 - lam_) * py + lam_ * xw[1]);
-  s.xbar[3 * i + 2] = (float)((1 - lam_) * pz + lam_ * xw[2]);
+  s.xbar[at3(i)] = (float)((1 - lam_) * px + lam_ * xw[0]);
+  s.xbar[at3(i) + 1] = (float)((1 - lam_) * py + lam_ * xw[1]);
+  s.xbar[at3(i) + 2] = (float)((1 - lam_) * pz + lam_ * xw[2]);
   double lam[3], V[3][3];
   sr_sym_eig(C, lam, V);
   double sg[3] = {lam[0], lam[1], lam[2]};
@@ -333,7 +337,7 @@ __device__ __forceinline__ void sr_aniso_kernel_of(const SrDev& s, int i, const 
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const double m = V[a_][0] * V[b][0] / sg[0] + V[a_][1] * V[b][1] / sg[1] + V[a_][2] * V[b][2] / sg[2];
-      s.G[9 * i + 3 * a_ + b] = (float)(tw != 0.0 ? m / (double)s.sr : (a_ == b ? 1.0 : 0.0));
+      s.G[3 * at3(i) + 3 * a_ + b] = (float)(tw != 0.0 ? m / (double)s.sr : (a_ == b ? 1.0 : 0.0));
     }
 }
 
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(SR_PRE_WARPS * 32) k_sr_aniso_pre(SrDev s, int
   for (int k = w; k < per && base + k < s.n; k += SR_PRE_WARPS) {
     const int i = base + k;
     if (i == 0) continue;  // the reference's loop starts at 1 (srtool.py:1013)
-    const float px = s.pos[3 * i], py = s.pos[3 * i + 1], pz = s.pos[3 * i + 2];
+    const float px = s.pos[at3(i)], py = s.pos[at3(i) + 1], pz = s.pos[at3(i) + 2];
     int cx, cy, cz;
     s.g.voxel_of(px, py, pz, cx, cy, cz);
     const float rr = 2.f * s.sr;  // isoweight radius
@@ -459,7 +463,7 @@ __global__ void __launch_bounds__(SR_SPLAT_WARPS * 32) k_sr_aniso_splat(SrDev s,
     const int i = k / parts, part = k % parts;
     const SrGrid& g = s.g;
     int cx, cy, cz;
-    g.voxel_of(s.pos[3 * i], s.pos[3 * i + 1], s.pos[3 * i + 2], cx, cy, cz);
+    g.voxel_of(s.pos[at3(i)], s.pos[at3(i) + 1], s.pos[at3(i) + 2], cx, cy, cz);
     // voxels [c - off, c - off + range - 1]; their vertices one further
     const int lo[3] = {cx - s.off, cy - s.off, cz - s.off};
     const int hi[3] = {lo[0] + s.range - 1, lo[1] + s.range - 1, lo[2] + s.range - 1};
@@ -481,7 +485,7 @@ __global__ void __launch_bounds__(SR_SPLAT_WARPS * 32) k_sr_aniso_splat(SrDev s,
     }
     float Gm[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) Gm[k] = s.G[9 * i + k];
+    for (int k = 0; k < 9; ++k) Gm[k] = s.G[3 * at3(i) + k];
     const double det = (double)Gm[0] * ((double)Gm[4] * Gm[8] - (double)Gm[5] * Gm[7]) -
                        (double)Gm[1] * ((double)Gm[3] * Gm[8] - (double)Gm[5] * Gm[6]) +
                        (double)Gm[2] * ((double)Gm[3] * Gm[7] - (double)Gm[4] * Gm[6]);
@@ -497,7 +501,7 @@ __global__ void __launch_bounds__(SR_SPLAT_WARPS * 32) k_sr_aniso_splat(SrDev s,
     Gi[2][0] = ((double)Gm[3] * Gm[7] - (double)Gm[4] * Gm[6]) / det;
     Gi[2][1] = ((double)Gm[1] * Gm[6] - (double)Gm[0] * Gm[7]) / det;
     Gi[2][2] = ((double)Gm[0] * Gm[4] - (double)Gm[1] * Gm[3]) / det;
-    const float xb[3] = {s.xbar[3 * i], s.xbar[3 * i + 1], s.xbar[3 * i + 2]};
+    const float xb[3] = {s.xbar[at3(i)], s.xbar[at3(i) + 1], s.xbar[at3(i) + 2]};
     const double org[3] = {g.dox, g.doy, g.doz};
     int w0[3], w1[3];
     bool empty = false;
@@ -605,7 +609,7 @@ __global__ void k_sr_vel_splat(SrDev s) {
   const float coeff = s.g.vs * s.g.vs * s.g.vs;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < s.n; i += warps) {
     const SrGrid& g = s.g;
-    const float px = s.pos[3 * i], py = s.pos[3 * i + 1], pz = s.pos[3 * i + 2];
+    const float px = s.pos[at3(i)], py = s.pos[at3(i) + 1], pz = s.pos[at3(i) + 2];
     int cx, cy, cz;
     g.voxel_of(px, py, pz, cx, cy, cz);
     const int lo[3] = {cx - s.off, cy - s.off, cz - s.off};
@@ -622,7 +626,7 @@ __global__ void k_sr_vel_splat(SrDev s) {
       empty |= w0[a] > w1[a];
     }
     if (empty) continue;
-    const float v[3] = {s.vel[3 * i], s.vel[3 * i + 1], s.vel[3 * i + 2]};
+    const float v[3] = {s.vel[at3(i)], s.vel[at3(i) + 1], s.vel[at3(i) + 2]};
     const int nxw = w1[0] - w0[0] + 1, ncol = nxw * (w1[1] - w0[1] + 1);
     const int64_t plane = (int64_t)g.nx * g.ny, cells = plane * g.nz;
     for (int col = lane; col < ncol; col += 32) {
@@ -658,7 +662,7 @@ __global__ void k_sr_vel_splat(SrDev s) {
 __global__ void k_sr_mesh_velocity(SrDev s, int nv) {
   const int64_t plane = (int64_t)s.g.nx * s.g.ny, cells = plane * s.g.nz;
   GRID_STRIDE(i, min(nv, s.max_v)) {
-    const double p[3] = {s.vert[3 * i], s.vert[3 * i + 1], s.vert[3 * i + 2]};
+    const double p[3] = {s.vert[at3(i)], s.vert[at3(i) + 1], s.vert[at3(i) + 2]};
     int x0, y0, z0;
     s.g.voxel_of((float)p[0], (float)p[1], (float)p[2], x0, y0, z0);
     const double xd = (p[0] - (x0 * s.g.dvs + s.g.dox)) / s.g.dvs, yd = (p[1] - (y0 * s.g.dvs + s.g.doy)) / s.g.dvs,
@@ -673,7 +677,7 @@ __global__ void k_sr_mesh_velocity(SrDev s, int nv) {
           const int64_t c = s.g.idx(x, y, z);
           for (int k = 0; k < 3; ++k) acc[k] += wgt * ((double)(long long)s.vfix[k * cells + c] / SR_FIX);
         }
-    for (int k = 0; k < 3; ++k) s.mvel[3 * i + k] = (float)acc[k];
+    for (int k = 0; k < 3; ++k) s.mvel[at3(i) + k] = (float)acc[k];
   }
 }
 
@@ -1135,10 +1139,10 @@ __global__ void k_sr_mc(SrDev s, int32_t cells, int pass) {
 // ---- 7. vertex normals (process_normal) ----------------------------------------------
 __global__ void k_sr_normals(SrDev s, int nv) {
   GRID_STRIDE(i, min(nv, s.max_v)) {
-    const double p[3] = {s.vert[3 * i], s.vert[3 * i + 1], s.vert[3 * i + 2]};
+    const double p[3] = {s.vert[at3(i)], s.vert[at3(i) + 1], s.vert[at3(i) + 2]};
     double n[3];
     sr_normal_at(s, p, n);
-    s.nrm[3 * i] = (float)n[0]; s.nrm[3 * i + 1] = (float)n[1]; s.nrm[3 * i + 2] = (float)n[2];
+    s.nrm[at3(i)] = (float)n[0]; s.nrm[at3(i) + 1] = (float)n[1]; s.nrm[at3(i) + 2] = (float)n[2];
   }
 }
 

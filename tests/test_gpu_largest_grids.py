@@ -39,6 +39,35 @@ def test_surface_of_the_largest_grid(cuda_lib, dims):
         assert np.array_equal(a, b)
 
 
+def test_surface_of_the_most_particles(cuda_lib):
+    """238,712,400 particles, whose 9 words of the anisotropic kernel each pass 2^31: the last
+    particles' kernels are those of the last planes alone."""
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 90e9:
+        pytest.skip("needs 50 GB of device memory")
+    side, planes, vs = 620, 621, 0.01
+    assert 9 * side * side * planes >= 2 ** 31
+
+    def kernels(first):  # of the particles from plane `first` on
+        i = torch.arange(first * side * side, planes * side * side, dtype=torch.int32, device="cuda")
+        pos = torch.empty((len(i), 3), device="cuda")
+        for k, c in enumerate((i % side, i // side % side, i // (side * side))):
+            # on the lattice but for a tenth of a voxel, a hash of the index
+            pos[:, k] = (c.float() + 0.4 + 0.1 * ((i % 1009) * (k + 7) % 101).float() / 101) * vs
+        del i, c
+        sr = SRTool([[0.0] * 3, [side * vs, side * vs, planes * vs]], voxel_size=vs, particle_radius=0.005,
+                    max_num_vertices=1000, max_num_indices=6000, max_num_particles=len(pos))
+        sr.dual_contouring(1e9, 0.0095, len(pos), pos)  # 26 neighbours; no surface at that level
+        out = sr.stage(0, len(pos))["G"][-side * side:].clone()
+        sr.close()
+        return out
+
+    got, want = kernels(0), kernels(planes - 8)
+    torch.cuda.empty_cache()
+    assert float(want.std()) > 0
+    assert torch.allclose(got, want, rtol=1e-5, atol=1e-5 * float(want.abs().max()))
+
+
 def _dam(extra=(0, 0, 0)):
     """A dam break whose domain goes on past its box by `extra` cells of the search grid."""
     sc = S.dam_break(seed=4, n_side=(9, 7, 8), box=0.4)
