@@ -72,7 +72,6 @@ struct SceneDev {
   real cellx;                    // cell edge in x (cell / x split)
   int32_t nfx;                    // stencil half-width in x cells (nf * x split)
   real h, k_w, k2_w, k_grad, W0; // cubic spline constants
-  real k_grad_h, k_grad_h2;      // k_grad / h, k_grad / h^2
   real inv_h;
   real h2_thr;                   // smallest value whose rounded sqrt is >= h (h^2 in the FP64 build)
   real rho0, inv_rho0;
@@ -93,6 +92,7 @@ struct SceneDev {
   real cfl_factor, cfl_min_dt, cfl_max_dt, diameter;
   real V0, padding;              // volume0 and padding (rigid-body mass, ground clamp)
   int32_t n_rigid, coupling;      // rigid bodies of the scene, substeps per step
+  real k_grad_h, k_grad_h2;      // k_grad / h, k_grad / h^2 (kernel_grad; behind what every pass reads)
 };
 
 // Mutable per-scene state on the device.
@@ -439,7 +439,7 @@ __device__ __forceinline__ double acc_take(double* acc, int scene, int quantity)
 // runs `last` before it lets the others go, so that the control of a solver loop costs no
 // barrier of its own. A wait that runs out (which a resident grid cannot cause) marks the
 // barrier failed: every block then leaves the kernel, every scene of the step reports it, and
-// the next step starts with the barrier at rest (k_zero_cells).
+// the next step starts with the barrier at rest (k_step_end).
 // The counter and the generation lie in lines of their own: the polls of a thousand waiting
 // blocks would queue up before the arrivals.
 struct GridBarrier { unsigned arrived, pad0[31], gen, pad1[31]; int fail, pad2[31]; };
@@ -479,7 +479,7 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier* b, unsigned limit, uns
     }
   } else if (threadIdx.x == 0) {
     unsigned polls = 0;
-    while (limit == 0u || ld_acquire(&b->gen) == gen) {
+    while (ld_acquire(&b->gen) == gen || limit == 0u) {
       if (++polls > limit || ((polls & 1023u) == 0u && *(volatile int*)&b->fail)) {
         atomicExch(&b->fail, 1);
         sh_fail = 1;

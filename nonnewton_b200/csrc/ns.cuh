@@ -53,20 +53,9 @@ __device__ __forceinline__ void step_reset_scenes(const Dev& d) {
 }
 
 // `reset_step`: block 0 also resets the step's per-scene counters (the step's first
-// launch; nothing before the list build reads them) and, after a wait at the loops' barrier
-// that ran out, the arrivals and the sums that it left behind.
+// launch; nothing before the list build reads them).
 __global__ void k_zero_cells(Dev d, int reset_step) {
-  if (reset_step && blockIdx.x == 0) {
-    step_reset_scenes(d);
-    if (*(volatile int*)&d.bar->fail) {
-      for (int t = threadIdx.x; t < d.d_n[1] * ACC_COUNT * NN_STRIPES; t += blockDim.x) d.acc[t] = 0.0;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        d.bar->arrived = d.bar->gen = 0u;
-        d.bar->fail = 0;
-      }
-    }
-  }
+  if (reset_step && blockIdx.x == 0) step_reset_scenes(d);
   const int nc = d.d_n[2];
   FOR_CELLS(i, nc + 1) d.cell_count[i] = 0u;
 }
@@ -102,11 +91,12 @@ __global__ void k_keys(Dev d) {
 #define SCAN_TILE 16384
 #define SCAN_THREADS 1024
 #define SCAN_ROUNDS (SCAN_TILE / SCAN_THREADS / 4)
-__device__ __forceinline__ int scan_at(int t, int r) {  // this thread's 4 counts of round r
+__device__ __forceinline__ uint32_t scan_at(int t, int r) {  // this thread's 4 counts of round r
   return t * SCAN_TILE + (int)(threadIdx.x >> 5) * (SCAN_ROUNDS * 128) + r * 128 + (int)(threadIdx.x & 31) * 4;
 }
-__device__ __forceinline__ uint4 scan_load(const uint32_t* a, int i, int len) {
-  if (len - i >= 4) return *reinterpret_cast<const uint4*>(a + i);
+// (unsigned: lengths up to 2^31 - 1, to which a tile is added)
+__device__ __forceinline__ uint4 scan_load(const uint32_t* a, uint32_t i, uint32_t len) {
+  if (i + 4 <= len) return *reinterpret_cast<const uint4*>(a + i);
   return make_uint4(i < len ? a[i] : 0u, i + 1 < len ? a[i + 1] : 0u, i + 2 < len ? a[i + 2] : 0u, 0u);
 }
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
@@ -121,8 +111,8 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(Dev d) {
   __shared__ uint32_t sh[32];
-  const int len = d.d_n[2] + 1;
-  const int ntiles = (len - 1) / SCAN_TILE + 1;  // len up to 2^31 - 1: nothing is added to it
+  const uint32_t len = (uint32_t)d.d_n[2] + 1u;
+  const int ntiles = (int)((len + SCAN_TILE - 1) / SCAN_TILE);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     uint32_t s = 0;
@@ -148,8 +138,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(Dev d) {
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(Dev d) {
   static_assert(SCAN_THREADS == 1024, "32 warps, one lane each");
   __shared__ uint32_t sh[32], sh_part[32];
-  const int len = d.d_n[2] + 1;
-  const int ntiles = (len - 1) / SCAN_TILE + 1;
+  const uint32_t len = (uint32_t)d.d_n[2] + 1u;
+  const int ntiles = (int)((len + SCAN_TILE - 1) / SCAN_TILE);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint32_t before = 0;  // sum of tile_sums[0 .. done)
   int done = 0;
@@ -178,13 +168,13 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(Dev d) {
     done = t;
 #pragma unroll
     for (int r = 0; r < SCAN_ROUNDS; ++r) {
-      const int i = scan_at(t, r);
+      const uint32_t i = scan_at(t, r);
       uint4 o;
       o.x = before + base + ex[r];
       o.y = o.x + v[r].x;
       o.z = o.y + v[r].y;
       o.w = o.z + v[r].z;
-      if (len - i >= 4) {
+      if (i + 4 <= len) {
         *reinterpret_cast<uint4*>(d.cell_count + i) = o;
       } else {
         if (i < len) d.cell_count[i] = o.x;

@@ -191,7 +191,7 @@ class Engine:
             num[bound:] = 0
             lists[bound:] = -1
         self._rc(self.L.nn_get_neighbors(self.h, _ptr(num), _ptr(lists), int(width)))
-        return num[:n], lists[:n]
+        return (num, lists) if rows == n else (num[:n], lists[:n])
 
     def set_neighbor_cap(self, max_neighbors: int):
         """Re-size the neighbour lists (see nn_set_neighbor_cap); clears overflow statuses."""
