@@ -1229,12 +1229,12 @@ __global__ void NN_REGS64 k_pressure_loop(const __grid_constant__ Dev d) {
 // gradient, R_j S_j (gw V_i) (-V_j) - R_i S_i (-gw V_j) (-V_i) =
 // -V_i V_j (R_i S_i + R_j S_j) gw. On the fluid-elastic scene (64,000 elastic particles)
 // rotations 38 + stress 37 + forces 62 us became gather 3 +
-// deformation 16 + rotations 12 + stress 15 + forces 22 us.
+// deformation 18 + rotations 12 + stress 15 + forces 22 us.
 // The kernel and its gradient are those with a correctly rounded root and divisions (kernel_w,
 // kernel_grad): from rsqrt (kw_r2, kgrad_r2) the stress took 12.5 and the forces 20.2 us, but in a
 // strained block, whose terms do not cancel, the accelerations were 1.7 times as far from 64
-// bits (deformed by 10 %: 7.2e-7 against 3.7e-7 of their root mean square, the stress 3.9e-7
-// against 2.8e-7).
+// bits (deformed by 10 %: 7.2e-7 against 3.4e-7 of their root mean square, the stress 3.9e-7
+// against 2.2e-7).
 #define EL_LANES 4
 #define EL_U 2
 #define EL_BLOCK 128
@@ -1264,8 +1264,8 @@ __device__ __forceinline__ void el_walk(const Dev& d, int e, int sub, int c, Loa
   }
 }
 // Sum over the lanes of a particle (lanes p, p + 8, p + 16, p + 24 of the warp).
-template <int N>
-__device__ __forceinline__ void el_sum(real (&v)[N]) {
+template <int N, typename T>
+__device__ __forceinline__ void el_sum(T (&v)[N]) {
 #pragma unroll
   for (int o = 32 / EL_LANES; o < 32; o <<= 1)
 #pragma unroll
@@ -1274,8 +1274,10 @@ __device__ __forceinline__ void el_sum(real (&v)[N]) {
 struct ElPair { real4 x, x0; };
 struct ElForce { real4 x0; real M[9]; };
 
-// computeRotations_kernel (SPH/main.py:1249-1274): the deformation sum, into el_R (every
-// product keeps the order (x y0) w, which leaves the sum of an undeformed body symmetric)
+// computeRotations_kernel (SPH/main.py:1249-1274): the deformation sum, into el_R. In FP64: the
+// products x y0 are exact, so the sum of an undeformed body is symmetric and its rotation the
+// identity: the stress of a falling block, of 1e-4 Young's moduli, is 4.7e-7 off (root mean
+// square), where one sum in f32 left 9.0e-7 and four partial sums 1.09e-6. 16 us become 18.
 __global__ void __launch_bounds__(EL_BLOCK) k_el_deformation(Dev d, int rep) {
   const int ne = d.d_n[3];
   FOR_SPLIT(EL_LANES, e, sub, in, ne) {
@@ -1284,19 +1286,19 @@ __global__ void __launch_bounds__(EL_BLOCK) k_el_deformation(Dev d, int rep) {
     const int self = in ? e : 0;
     const real4 xi4 = d.el_x[self];
     const real3 xi = f3(xi4), x0i = f3(d.el_x0[self]);
-    real A[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double A[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     el_walk(d, e, sub, work ? d.el_cnt[e] : 0, [&](int j) { return ElPair{ldg(&d.el_x[j]), ldg(&d.el_x0[j])}; },
             [&](const ElPair& g) {
               const real3 a = f3(g.x) - xi, b = f3(g.x0) - x0i;
-              const real w = xi4.w * kernel_w(sqrt(dot3(b, b)), s);
-              A[0] += a.x * b.x * w; A[1] += a.x * b.y * w; A[2] += a.x * b.z * w;
-              A[3] += a.y * b.x * w; A[4] += a.y * b.y * w; A[5] += a.y * b.z * w;
-              A[6] += a.z * b.x * w; A[7] += a.z * b.y * w; A[8] += a.z * b.z * w;
+              const double w = xi4.w * kernel_w(sqrt(dot3(b, b)), s);
+              A[0] = fma((double)a.x * b.x, w, A[0]); A[1] = fma((double)a.x * b.y, w, A[1]); A[2] = fma((double)a.x * b.z, w, A[2]);
+              A[3] = fma((double)a.y * b.x, w, A[3]); A[4] = fma((double)a.y * b.y, w, A[4]); A[5] = fma((double)a.y * b.z, w, A[5]);
+              A[6] = fma((double)a.z * b.x, w, A[6]); A[7] = fma((double)a.z * b.y, w, A[7]); A[8] = fma((double)a.z * b.z, w, A[8]);
             });
     el_sum(A);
     if (work && sub == 0)
 #pragma unroll
-      for (int k = 0; k < 9; ++k) d.el_R[(size_t)k * d.el_stride + e] = A[k];
+      for (int k = 0; k < 9; ++k) d.el_R[(size_t)k * d.el_stride + e] = (real)A[k];
   }
 }
 // its rotation, one thread per particle (an FP64 chain)
@@ -1328,10 +1330,12 @@ __global__ void __launch_bounds__(EL_BLOCK) k_el_stress(Dev d, int rep) {
     el_walk(d, e, sub, work ? d.el_cnt[e] : 0, [&](int j) { return ElPair{ldg(&d.el_x[j]), ldg(&d.el_x0[j])}; },
             [&](const ElPair& g) {
               const real3 xji = f3(g.x) - xi, xji0 = f3(g.x0) - x0i;
-              // u_ji = R^T x_ji - x0_ji
-              real3 u = make_real3(R[0] * xji.x + R[3] * xji.y + R[6] * xji.z - xji0.x,
-                                     R[1] * xji.x + R[4] * xji.y + R[7] * xji.z - xji0.y,
-                                     R[2] * xji.x + R[5] * xji.y + R[8] * xji.z - xji0.z);
+              // u_ji = R^T x_ji - x0_ji as x_ji - x0_ji + (R - I)^T x_ji, which rounds at the size of
+              // u: at strains of 1 % the stress error is 0.7 of that of the products of R
+              const real3 dx = xji - xji0;
+              real3 u = make_real3(fma(R[6], xji.z, fma(R[3], xji.y, fma(R[0] - 1.f, xji.x, dx.x))),
+                                   fma(R[7], xji.z, fma(R[4] - 1.f, xji.y, fma(R[1], xji.x, dx.y))),
+                                   fma(R[8] - 1.f, xji.z, fma(R[5], xji.y, fma(R[2], xji.x, dx.z))));
               u = u * g.x0.w;
               const real3 gw = kernel_grad(xji0, sqrt(dot3(xji0, xji0)), s);
               G[0] -= u.x * gw.x; G[1] -= u.x * gw.y; G[2] -= u.x * gw.z;
