@@ -55,15 +55,14 @@ ALG_BYTES = {
 # loop's predicted last body) reads mass and density besides and writes acc4, srn, mu, aux2
 ALG_BYTES["density_change_np"] = ALG_BYTES["density_change"] + 4 + 4 + 16 + 4 + 4 + 8
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch on the
-# 2.4M-particle dam break, from ncu captures of the current kernels; "nonpressure" and
-# "density_change", which have no work in that step, from captures with positions and
-# velocities in separate arrays.
+# 2.4M-particle dam break, from ncu captures; "nonpressure" and "density_change", which have
+# no work in that step, from launches on their own (nn_time_kernel) after three steps.
 # list entries of the captured k_build_lists launch (an early step of the 2.4M scene); the line
 # scales that launch's traffic to the timed launch's entries, which the bytes follow
 NCU_ENTRIES_2M = 62_580_972
 NCU_TRAFFIC_2M = {"build_lists": 505586688, "density_adv": 414270976,
-                  "nonpressure": 431172096, "density_factor": 398540800,
-                  "density_change": 366368512, "divergence_update": 425979136,
+                  "nonpressure": 505473024, "density_factor": 398540800,
+                  "density_change": 394503168, "divergence_update": 425979136,
                   "pressure_update": 414269952, "cg_matvec": 431102976, "density_change_np": 464528128,
                   "cg_setup": 610421248}
 # what bounds each kernel instead of DRAM, from its ncu capture on the 2.4M scene:
@@ -71,9 +70,9 @@ NCU_TRAFFIC_2M = {"build_lists": 505586688, "density_adv": 414270976,
 LIMITER_2M = {
     "build_lists": "instruction issue: 68 % issue active, ~160 exact f32 distance tests per particle, two per packed f32x2 instruction; LSU wavefronts 60 %; DRAM 15 %",
     "density_adv": "L1 data pipe: LSU wavefronts at 78 % of peak (256-bit neighbour gathers), 47 % warps active; DRAM 23 %",
-    "nonpressure": "L1 data pipe and gather latency: LSU wavefronts 62 %, 46 % warps active; DRAM 13 %",
+    "nonpressure": "issue and gather latency: issue 68 %, LSU wavefronts 58 %, 46 % warps active at 64 registers; DRAM 16 %",
     "density_factor": "L1 data pipe: LSU wavefronts 75 %, issue 65 %, 52 % warps active; DRAM 19 %",
-    "density_change": "L1 data pipe: LSU wavefronts 85 % of peak; DRAM 18 %",
+    "density_change": "L1 data pipe: LSU wavefronts 77 % of peak, 48 % issue active, 59 % warps active; DRAM 20 %",
     "divergence_update": "gather latency and issue: LSU wavefronts 59 %, 66 % issue active, 50 % warps active; DRAM 24 %",
     "pressure_update": "L1 data pipe: LSU wavefronts 74 % of peak, 43 % issue active; DRAM 32 %",
     "cg_matvec": "L1 data pipe: LSU wavefronts 75 %, issue 63 %, 53 % warps active at 56 registers; DRAM 22 %",

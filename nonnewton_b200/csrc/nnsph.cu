@@ -137,9 +137,13 @@ struct nn_ctx {
 // thread's pass over its 26-odd neighbours is one chain of dependent loads and arithmetic,
 // 10-20 us however few particles there are; splitting it over L lanes shortens it until the
 // chip is full, and past that only costs the shuffles that fold the terms in list order.
-// Step times at 8 / 4 / 2 / 1 lanes (us): 2,197 fluid 209 / 225 / 264 / 287; 8,000 279 /
-// 284 / 322 / 368; 15,625 330 / 307 / 342 / 381; 24,389 361 / 321 / 345 / 382; 39,304
-// 486 / 427 / 389 / 433; 46,656 277 / 246 / 227 / 253; 68,921 667 / 542 / 517 / 468.
+// Step times at 8 / 4 / 2 / 1 lanes, with the loops that each brings (us): a dam break with
+// explicit viscosity, 2,197 fluid 143 / 152 / 175 / 233; 9,261 150 / 151 / 169 / 218; 10,648
+// 157 / 153 / 170 / 216; 24,389 209 / 189 / 186 / 229; 29,791 229 / 202 / 193 / 235; 54,872
+// 269 / 232 / 212 / 223; 59,319 283 / 240 / 228 / 228; 68,921 310 / 262 / 265 / 235. A settled
+// Cross pool, 2,197 166 / 169 / 199 / 258; 9,261 207 / 209 / 243 / 297; 10,648 218 / 212 / 246 /
+// 297; 27,000 324 / 277 / 277 / 325; 29,791 353 / 293 / 278 / 324; 54,872 536 / 436 / 382 /
+// 386; 59,319 561 / 468 / 420 / 394.
 // An explicit unroll (nn_set_tuning) selects the one-lane passes it names.
 static int lanes_for(const nn_ctx* c, int n_fluid) {
   if (c->unroll) return 1;
@@ -149,7 +153,9 @@ static int lanes_for(const nn_ctx* c, int n_fluid) {
 // The one-kernel loops' grids are laid out for the slots rounded up to a power of two (at most
 // the capacity): compositions of the same class share a captured step, and neither a small one
 // gets the blocks of the largest (each block more is an arrival at every barrier) nor a large one
-// those of the smallest that was captured first.
+// those of the smallest that was captured first. In a context of 300,000 slots a step of 3,933
+// takes 91 us so and 98 with the capacity's grid (137 and 152 with implicit viscosity), one of
+// 33,938 151 and 152; a change of class costs two captures and their end, 0.5 ms.
 static int log2_up(int n) {
   int b = 0;
   while (((int64_t)1 << b) < n) ++b;
@@ -433,9 +439,11 @@ static int solver_loop(nn_ctx* c, cudaStream_t s, bool check_first, Pre pre, Bod
 }
 
 // The list build: one cell row per warp while the scene does not fill the chip, else one
-// warp for all rows of its slots (rows / whole, us: 3,933 slots 9 / 36; 23,002 13 / 35;
-// 85,147 40 / 51; 135,201 46 / 44; 900,002 265 / 200; 2,400,002 694 / 470). Both write the
-// same lists.
+// warp for all rows of its slots. Rows / whole, us: 3,933 slots 12 / 35; 35,666 21 / 43; 85,147
+// 35 / 45 (settled 41 / 53); 110,621 47 / 50 (51 / 61); 125,425 50 / 53 (55 / 57); 135,201 47 /
+// 44; 148,816 55 / 55 (60 / 58); 600,002 141 / 96; 900,002 234 / 151; 2,400,002 694 / 437. The
+// steps part between 110,621 (271.6 / 270.9 us, settled 449 / 454) and 135,201 (332 / 329).
+// Both write the same lists.
 static int enq_build_lists(nn_ctx* c, cudaStream_t s, const Dev& d) {
   if (c->plan.rows) return launch_lanes(c, s, k_build_lists_rows, NSR_WARPS * 32, c->n, NSR_WARPS, d);
   return launch(c, s, k_build_lists, NS_WARPS * 32, c->n, d);
