@@ -82,7 +82,7 @@ struct Dev {
   // loop control
   int32_t* any_active;         // host-visible flag of the last check
   unsigned long long loop_handle; // cudaGraphConditionalHandle (0 when not in a graph)
-  int32_t* body_count;         // [4] executed loop bodies (div, pressure, cg, elastic)
+  int32_t* body_count;         // [4] executed loop bodies (div, pressure, cg, div with non-pressure terms)
   GridBarrier* bar;            // barrier of the one-kernel loops
   uint32_t bar_polls;          // polls of a wait at it
 };

@@ -122,8 +122,8 @@ struct nn_ctx {
   GridBarrier* d_bar = nullptr;
   uint32_t bar_polls = NN_BARRIER_POLLS;
   int64_t fixed_nodes_per_step = 0;    // kernel nodes outside loop bodies (graph mode)
-  int64_t graph_replays = 0;
-  int64_t body_nodes[3] = {3, 3, 5};   // kernels per loop body: divergence, pressure, CG
+  // kernels per loop body: divergence, pressure, CG, divergence with the non-pressure terms
+  const int64_t body_nodes[4] = {3, 3, 5, 4};
   // graphs: [parity]
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
   bool in_capture = false;
@@ -970,8 +970,9 @@ int64_t nn_launch_count(const nn_ctx* cc) {
   int32_t body[4] = {0, 0, 0, 0};
   cudaStreamSynchronize(run_stream(c));
   cudaMemcpy(body, c->d_body, sizeof(body), cudaMemcpyDeviceToHost);
-  return c->launches + c->graph_replays * c->fixed_nodes_per_step + (int64_t)body[0] * c->body_nodes[0] +
-         (int64_t)body[1] * c->body_nodes[1] + (int64_t)body[2] * c->body_nodes[2];
+  int64_t n = c->launches;
+  for (int k = 0; k < 4; ++k) n += body[k] * c->body_nodes[k];
+  return n;
 }
 
 int nn_bind_state(nn_ctx* c, const nn_state* st) {
@@ -1086,7 +1087,6 @@ int nn_set_scenes(nn_ctx* c, int32_t nscenes, const nn_scene_desc* scenes) {
   // the force pass's terms ride on the divergence loop's last density change unless a
   // scene skips the divergence solve or needs the explicit viscosity or quirk mode
   c->fold_np = c->any_fluid && all_div && (c->forces_feat & (FF_VI | FF_Q)) == 0;
-  c->body_nodes[0] = c->fold_np ? 4 : 3;  // the folded density change is a second launch per body
   if (cells >= (int64_t)0x7fffffff) return fail(c, NN_ERR_CAPACITY, "%lld grid cells exceed the 32-bit key space", (long long)cells);
   if (cells > c->max_cells) drop_graphs(c);  // the scan grids were sized for the old table
   RC(ensure_cells(c, cells));
@@ -1230,7 +1230,7 @@ int nn_step(nn_ctx* c, int32_t nsteps, uint32_t flags) {
       if (!c->exec[parity]) RC(capture_step(c, s, parity));
       CK(cudaGraphLaunch(c->exec[parity], s));
       c->cur = 1 - parity;
-      c->graph_replays++;
+      c->launches += c->fixed_nodes_per_step;  // of this graph: the next composition's has others
       c->searched = true;
     }
   }

@@ -512,7 +512,7 @@ __device__ __forceinline__ void loop_decide(const Dev& d, int any, int body) {
 #endif
 }
 __global__ void k_solver_check(Dev d, int which, int fold) {
-  loop_decide(d, solver_check_scenes(d.d_n, d.sc, d.dyn, d.acc, which, fold), which);
+  loop_decide(d, solver_check_scenes(d.d_n, d.sc, d.dyn, d.acc, which, fold), fold ? 3 : which);
 }
 
 // Per-scene loop start: which scenes iterate, counters reset.

@@ -6,6 +6,7 @@ import pytest
 import torch
 from torch.profiler import ProfilerActivity, profile
 
+from nonnewton_b200 import _abi
 from nonnewton_b200 import scene as S
 from nonnewton_b200.batch import Batch, scene_grid_cells
 
@@ -70,10 +71,10 @@ def test_rigid_scene_is_repacked_away(cuda_lib):
     _same(_steps(b), _steps(fresh))
 
 
-def _kernels(b, path):
-    """Names and grids of the kernels of a step, in time order (none without a profiler)."""
+def _kernels(b, path, run=None):
+    """Names and grids of the kernels of a step (or of `run`), in time order (none without a profiler)."""
     with profile(activities=[ProfilerActivity.CUDA]) as p:
-        b.step(1)
+        run() if run else b.step(1)
         torch.cuda.synchronize()
     p.export_chrome_trace(str(path))
     ev = [e for e in json.loads(path.read_text())["traceEvents"] if e.get("cat") == "kernel"]
@@ -107,3 +108,24 @@ def test_choices_follow_the_composition(cuda_lib, tmp_path, implicit):
         b.set([scenes[k]])
         _same(_steps(b), want[k][0])
         assert _kernels(b, tmp_path / "trace.json") == want[k][1]
+
+
+def test_launch_counts_across_compositions(cuda_lib, tmp_path):
+    """nn_launch_count over steps of several compositions and a pass of its own: the kernels that
+    a profiler sees (small scenes, whose loops are no while-nodes)."""
+    kind = dict(extra_cfg={"useNonNewtonianModel": True},
+                fluid_cfg={"nonNewtonMethod": "CROSS_", "viscosity0": 5.0, "viscosity_inf": 0.01, "consistency_index": 1.0,
+                           "power_index": 0.7, "viscosityMethod": 13})
+    scenes = [S.dam_break(seed=1, n_side=(8, 7, 6), box=0.4), S.dam_break(seed=2, n_side=(9, 8, 7), box=0.4, **kind)]
+    b = Batch(8000, 1)
+    first = b.engine.launch_count()
+    seen = in_set = 0
+    for k in (0, 1, 0, 1):
+        before = b.engine.launch_count()
+        b.set([scenes[k]])
+        in_set += b.engine.launch_count() - before
+        seen += len(_kernels(b, tmp_path / "trace.json"))
+        seen += len(_kernels(b, tmp_path / "trace.json"))
+    seen += len(_kernels(b, tmp_path / "trace.json", lambda: b.engine.run_pass(_abi.NN_PASS_SUBSTEP)))
+    if seen:  # a profiler is there
+        assert b.engine.launch_count() - first == in_set + seen
